@@ -1104,17 +1104,21 @@ def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, n_groups: in
     assert a.dim() == 2 and out.dim() == 2 and a.shape[0] == out.shape[0] and a.stride(1) == 1 and out.stride(1) == 1
     assert w.is_contiguous() and w.shape == (n_groups, n_out, k_dim) and a.dtype == w.dtype
     ll = ctypes.c_longlong
-    args = (_p(a), _p(w), _p(out), n_groups, a.shape[0], n_out, k_dim, 0, 0, ll(a.stride(0)), ll(a_goff), ll(out.stride(0)),
-            ll(c_goff), ll(n_out * k_dim), None, None, None, 0, None, 1)
+    strides = (ll(a.stride(0)), ll(a_goff), ll(out.stride(0)), ll(c_goff), ll(n_out * k_dim))
+    sizes = (_p(a), _p(w), _p(out), n_groups, a.shape[0], n_out, k_dim)
     if _grouped_mma(a, k_dim, a.stride(0), a_goff, n_out * k_dim):
-        _check(lib().st_gemm_grouped_mma(*args, int(out.dtype == torch.float32), _stream()), "gemm_heads")
+        _check(lib().st_gemm_grouped_mma(*sizes, *strides, int(out.dtype == torch.float32), _stream()), "gemm_heads")
     else:
-        _check(lib().st_gemm_grouped_plain(*args, _dt(a), int(out.dtype == torch.float32), _stream()), "gemm_heads")
+        _check(lib().st_gemm_grouped_plain(*sizes, 0, 0, *strides, None, None, None, 0, None, 1, _dt(a),
+                                           int(out.dtype == torch.float32), _stream()), "gemm_heads")
     return out
 
 
 # False: the grouped products of bfloat16 models run on the plain kernel too (measurements, tests)
 GROUPED_MMA = True
+
+
+EXPERTS_TILE = 0         # rows of an expert's matrix per tile of the tcgen05 kernel: 64, 128, 256; 0: the launcher's choice
 
 
 def _grouped_mma(a: torch.Tensor, k_dim: int, lda: int, a_goff: int, w_gstride: int) -> bool:
@@ -1202,18 +1206,24 @@ def gemm_experts(a: torch.Tensor, w: torch.Tensor, order: ExpertOrder, gather: b
                  act: str = "none") -> torch.Tensor:
     """One product per expert over the rows the order gives it: out [items, n_out] in sorted order.
     ``gather``: the rows of ``a`` are the tokens (row of item i = i // top), else ``a`` is already in sorted order.
-    w [experts, n_out (twice with ``gated``: gate rows, then up rows), k]; out = act(product), gated: act(gate) * up."""
+    w [experts, n_out (twice with ``gated``: gate rows, then up rows), k]; out = act(product), gated: act(gate) * up.
+    bfloat16 with k a multiple of 8: the tcgen05 kernel (a wait that expires inside it shows in ``kernel_status``); else
+    the plain one."""
     assert a.is_contiguous() and w.is_contiguous() and w.dim() == 3 and a.dtype == w.dtype and a.shape[1] == w.shape[2]
     n_out = w.shape[1] // 2 if gated else w.shape[1]
     out = torch.empty((order.n_items, n_out), dtype=a.dtype, device=a.device)
     ll = ctypes.c_longlong
-    args = (_p(a), _p(w), _p(out), w.shape[0], order.n_items, n_out, w.shape[2], int(gated), ACT_CODES[act], ll(a.stride(0)),
-            ll(0), ll(n_out), ll(0), ll(w.shape[1] * w.shape[2]), _p(order.offsets), _p(order.tile_group),
-            _p(order.tile_row0), order.tile_group.numel(), _p(order.sorted) if gather else None, order.top if gather else 1)
-    if _grouped_mma(a, w.shape[2], a.stride(0), 0, w.shape[1] * w.shape[2]):
-        _check(lib().st_gemm_grouped_mma(*args, 0, _stream()), "gemm_experts")
-    else:
-        _check(lib().st_gemm_grouped_plain(*args, _dt(a), 0, _stream()), "gemm_experts")
+    if GROUPED_MMA and a.dtype == torch.bfloat16 and bool(lib().st_gemm_experts_tc_applies(w.shape[0], w.shape[2])):
+        _check(lib().st_gemm_experts_tc(_p(a), ll(a.shape[0]), _p(w), _p(out), w.shape[0], order.n_items, n_out, w.shape[2],
+                                        int(gated), ACT_CODES[act], _p(order.offsets), _p(order.sorted) if gather else None,
+                                        order.top if gather else 1, EXPERTS_TILE, _p(_tc_status_word(a.device)), _stream()),
+               "gemm_experts")
+        return out
+    _check(lib().st_gemm_grouped_plain(_p(a), _p(w), _p(out), w.shape[0], order.n_items, n_out, w.shape[2], int(gated),
+                                       ACT_CODES[act], ll(a.stride(0)), ll(0), ll(n_out), ll(0),
+                                       ll(w.shape[1] * w.shape[2]), _p(order.offsets), _p(order.tile_group),
+                                       _p(order.tile_row0), order.tile_group.numel(), _p(order.sorted) if gather else None,
+                                       order.top if gather else 1, _dt(a), 0, _stream()), "gemm_experts")
     return out
 
 

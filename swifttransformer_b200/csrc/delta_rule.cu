@@ -22,26 +22,12 @@
 //
 // Since (decay S + k u^T)^T q = (decay S)^T q + u (k . q), both dot products of a token are taken from the
 // decayed state in one pass of shuffles.
-#include "common.cuh"
+#include "delta_rule.cuh"
 
 #define DR_MAX_TAPS 8
 #define DR_PREP_THREADS 256
 #define DR_EARLY_TOKENS 128   // steps of at most this many tokens let the next kernel's blocks in early
 #define DR_UNIT_PASSES 8      // a warp's lanes cover a head of up to 32 * DR_UNIT_PASSES channels
-
-struct DeltaShape {
-    int H, G, dim, vd;            // value heads, query/key heads, key size, value size
-    int q_off, k_off, v_off, b_off, a_off, g_off;   // columns of the projection
-    int rank_a, rank_g;           // 0: no low-rank pair, the projection holds the logits themselves (see below)
-    int gate_silu;                // the output gate: 0 sigmoid(z), 1 z * sigmoid(z)
-    // columns of a prepared row
-    __host__ __device__ int pq() const { return 0; }
-    __host__ __device__ int pk() const { return G * dim; }
-    __host__ __device__ int pv() const { return 2 * G * dim; }
-    __host__ __device__ int pd() const { return 2 * G * dim + H * vd; }
-    __host__ __device__ int pb() const { return 2 * G * dim + H * vd + H * dim; }
-    __host__ __device__ int row() const { return 2 * G * dim + H * vd + H * dim + H; }
-};
 
 __device__ __forceinline__ float softplusf_(float z) { return z > 20.f ? z : log1pf(expf(z)); }
 __device__ __forceinline__ float siluf_(float z) { return z / (1.f + expf(-z)); }
@@ -104,7 +90,7 @@ delta_prepare_kernel(const float* __restrict__ proj, int ld, DeltaShape sh, cons
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const float* row = proj + (size_t)t * ld;
     float* st = state + (size_t)slots[b] * keep * channels;
-    float* dst = prep + (size_t)t * sh.row();
+    float* dst = prep + (size_t)t * sh.stride;
     const int units = 2 * G + H;
     for (int u = blockIdx.y * nwarp + warp; u < units; u += nwarp * gridDim.y) {
         const bool is_v = u >= 2 * G;
@@ -224,7 +210,7 @@ delta_scan_kernel(const float* __restrict__ prep, DeltaShape sh, float* __restri
     float s[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) s[r] = (live && d0 + r < dim) ? S[(size_t)(d0 + r) * vd] : 0.f;
-    const int row_len = sh.row();
+    const int row_len = sh.stride;
     const float* p = prep + (size_t)first * row_len;
     // the padding of the staged rows (dimensions past dim, columns past vd) stays zero: nothing is copied there
     for (int i = threadIdx.x; i < DS_STAGES * DS_CHUNK * M::ROW; i += DS_THREADS) ds_smem[i] = 0.f;
@@ -382,20 +368,29 @@ ST_EXPORT int st_delta_rule_set_lanes(int lanes) {
     ds_forced_lanes = lanes;
     return 0;
 }
+// Floats of scratch with which a step of n_tokens tokens of n_seqs requests runs in chunks (0: it does not).
+ST_EXPORT long long st_delta_rule_chunk_floats(int n_tokens, int n_seqs, int H, int G, int dim, int vd) {
+    if (n_tokens <= 0 || n_seqs <= 0 || H <= 0 || G <= 0 || H % G || dim <= 0 || vd <= 0 || ds_forced_lanes) return 0;
+    DeltaShape sh = {};
+    sh.H = H; sh.G = G; sh.dim = dim; sh.vd = vd;
+    const long long more = delta_chunks_floats(n_tokens, n_seqs, sh);
+    return more ? (long long)n_tokens * ((sh.row() + 3) / 4 * 4 + (long long)H * vd) + more : 0;
+}
+// Floats of scratch for the walk.
 ST_EXPORT long long st_delta_rule_scratch_floats(int n_tokens, int H, int G, int dim, int vd) {
     return (long long)n_tokens * ((long long)2 * G * dim + (long long)H * vd + (long long)H * dim + H + (long long)H * vd);
 }
 
 // proj: float [n_tokens, ld]; w_a2 [H*dim, rank_a], w_g2 [H*vd, rank_g] in the storage type `dtype`, as is out
 // [n_tokens, H*vd]; conv_state float [slots, taps-1, 2*G*dim + H*vd]; state float [slots, H, dim, vd];
-// scratch: float, st_delta_rule_scratch_floats elements.  write_state == 0: the states are read, not moved on.
+// scratch: float, st_delta_rule_scratch_floats elements, with `chunks` 16-byte aligned and st_delta_rule_chunk_floats.  write_state == 0: the states are read, not moved on.
 ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int a_off, int g_off, int rank_a,
                             int rank_g, const float* conv_w, int taps, float* conv_state, const void* w_a2,
                             const float* a_log, const float* dt_bias, const void* w_g2, const float* norm_w, float eps,
                             float out_scale, float* state, int write_state, int single_tokens, float* scratch,
                             void* out, const int* positions, const int* seq_of_token, const int* q_start,
                             const int* slots, int n_tokens, int n_seqs, int H, int G, int dim, int vd, int dtype,
-                            void* stream, int gate_silu) {
+                            void* stream, int gate_silu, int chunks) {
     if (n_tokens <= 0 || n_seqs <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || dim <= 0 || vd <= 0 || taps < 1 || rank_a < 0 || rank_g < 0) return ST_ERR_BAD_ARG;
     if (taps > DR_MAX_TAPS || dim > 32 * DR_UNIT_PASSES || vd > 32 * DR_UNIT_PASSES) return ST_ERR_TOO_LARGE;
@@ -404,9 +399,12 @@ ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int
     sh.H = H; sh.G = G; sh.dim = dim; sh.vd = vd;
     sh.q_off = q_off; sh.k_off = q_off + G * dim; sh.v_off = q_off + 2 * G * dim;
     sh.b_off = b_off; sh.a_off = a_off; sh.g_off = g_off; sh.rank_a = rank_a; sh.rank_g = rank_g; sh.gate_silu = gate_silu;
+    sh.stride = chunks ? (sh.row() + 3) / 4 * 4 : sh.row();
+    if (chunks && delta_chunks_floats(n_tokens, n_seqs, sh) == 0) return ST_ERR_BAD_SIZE;
+    if (chunks && !aligned16(scratch)) return ST_ERR_BAD_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     float* prep = scratch;
-    float* o = scratch + (size_t)n_tokens * sh.row();
+    float* o = scratch + (size_t)n_tokens * sh.stride;
     const int move = single_tokens && write_state && taps > 1;
     int rc;
     {
@@ -424,7 +422,11 @@ ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int
                                seq_of_token, q_start, slots);
         if (rc) return rc;
     }
-    {
+    if (chunks) {
+        rc = delta_chunks_launch(prep, sh, o + (size_t)n_tokens * H * vd, state, write_state, o, positions, q_start, slots, n_tokens,
+                                 n_seqs, s);
+        if (rc) return rc;
+    } else {
 #define DS_LAUNCH(L, R)                                                                                              \
     do {                                                                                                             \
         const size_t smem = DeltaScanSmem<L, R>::BYTES;                                                              \

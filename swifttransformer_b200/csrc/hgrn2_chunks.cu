@@ -19,13 +19,7 @@
 // than about 100 tokens stay with the walk.  kv and out are bound by their instructions (half of the issue slots used,
 // two blocks of 256 threads per SM), the scan by its two trips to the second-level cache.  Against 64 bits the states
 // are off by 2.9e-7 where the walk's are by 4.0e-7 (fewer roundings in a row).
-#include "common.cuh"
-
-#define HK_C 64            // tokens of a chunk
-#define HK_H 32            // half of it
-#define HK_D 128           // the most channels and values per head
-#define HK_LD (HK_D + 4)
-#define HK_LA (HK_C + 4)
+#include "chunks.cuh"
 
 struct HgrnShape {
     int ld, q_off, f_off, v_off, n_seqs, nh, dim, vd;
@@ -34,27 +28,8 @@ struct HgrnShape {
     const int *positions, *q_start, *slots;
 };
 
-// A request's chunks have the places q_start / 64 + (its index) + 0, 1, ..: no two requests' overlap, and n / 64 + n_seqs hold
-// all.  Returns false when no chunk stands at `place`.
-__device__ __forceinline__ bool hk_find(const HgrnShape& sh, int place, int& b, int& first, int& n) {
-    int lo = 0, hi = sh.n_seqs;                           // the last request whose places begin at or before this one
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (sh.q_start[mid] / HK_C + mid <= place) lo = mid; else hi = mid;
-    }
-    b = lo;
-    const int begin = sh.q_start[b], end = sh.q_start[b + 1];
-    const int chunk = place - (begin / HK_C + b);
-    first = begin + chunk * HK_C;
-    n = min(HK_C, end - first);
-    return chunk >= 0 && n > 0 && sh.positions[begin] >= 0;      // (padding stands at position -1)
-}
-
 __device__ __forceinline__ float hk_silu(float z) { return z / (1.f + expf(-z)); }
 __device__ __forceinline__ float hk_gate(float z, float bias, float lo) { return lo + (1.f - lo) * (1.f / (1.f + expf(-(z + bias)))); }
-__device__ __forceinline__ void hk_cp16(float* dst, const float* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
-}
 
 // ---- a chunk's sum of k~ v^T [dim][vd] and its product of gates [dim] ----------------------------------------
 // 256 threads of 8 x 8 sums; lanes l and l ^ 1 share the values they read, l and l ^ 2 the keys (two cycles of shared
@@ -69,7 +44,7 @@ hgrn2_chunk_kv_kernel(const T* __restrict__ proj, const HgrnShape sh, float* __r
     const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dim = sh.dim, vd = sh.vd;
     int b, first, n;
-    if (!hk_find(sh, place, b, first, n)) return;
+    if (!hk_find(sh.q_start, sh.positions, sh.n_seqs, place, b, first, n)) return;
     {   // every thread asks for all its pieces before it works on one
         constexpr int N = HK_C * HK_D / 4 / 256;
         const int e = (tid % (HK_D / 4)) * 4, t0 = tid / (HK_D / 4);
@@ -187,9 +162,8 @@ hgrn2_chunk_scan_kernel(const HgrnShape sh, float* __restrict__ states, const fl
 // threads, values of their own memory and one block per SM it took 113 us for 2000 tokens of 16 heads).  The state's
 // rows come 16 at a time through two stages of shared memory, asked for before the gates are worked out; the values take the
 // place of the gates once those are used up.
-#define HK_SR 16
 struct HkOutSmem {
-    float Q[HK_C * HK_LD], F[HK_C * HK_LD], A[HK_C * HK_LA], S[2][HK_SR * HK_LD], total[HK_D], part[HK_C][2];
+    float Q[HK_C * HK_LD], F[HK_C * HK_LD], A[HK_C * HK_LA], S[2 * HK_SR * HK_LD], total[HK_D], part[HK_C][2];
 };
 
 template <typename T>
@@ -201,18 +175,10 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
     const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dim = sh.dim, vd = sh.vd;
     int b, first, n;
-    if (!hk_find(sh, place, b, first, n)) return;
+    if (!hk_find(sh.q_start, sh.positions, sh.n_seqs, place, b, first, n)) return;
     const float* S0 = states + ((size_t)place * sh.nh + h) * dim * vd;
-    auto copy_rows = [&](int i0) {                        // rows i0 .. i0 + 15 of the state before the chunk
-        float* dst = m.S[(i0 / HK_SR) & 1];
-        for (int i = tid; i < HK_SR * (HK_D / 4); i += 256) {
-            const int r = i / (HK_D / 4), c = (i % (HK_D / 4)) * 4;
-            if (i0 + r < dim && c < vd) hk_cp16(dst + r * HK_LD + c, S0 + (size_t)(i0 + r) * vd + c);
-        }
-        asm volatile("cp.async.commit_group;\n" ::);
-    };
-    copy_rows(0);
-    copy_rows(HK_SR);
+    hk_copy_rows(m.S, S0, 0, dim, vd);
+    hk_copy_rows(m.S, S0, HK_SR, dim, vd);
     const int e4 = (tid % (HK_D / 4)) * 4, t4 = tid / (HK_D / 4);         // a thread's pieces: four columns of every eighth row
     constexpr int N = HK_C * HK_D / 4 / 256, TSTEP = 256 / (HK_D / 4);
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -305,7 +271,9 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
     const int rl = (lane & 1) | ((lane >> 4) << 1), cl = (lane >> 1) & 7;
     if (n > HK_H) {                                       // A between the halves: 2 x 2 sums per thread
         const int t0 = HK_H + (warp >> 1) * 8 + rl, s0 = (warp & 1) * 16 + cl;
-        float a[2][2] = {};
+        float4 a[2][2];                                   // four chains per sum
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i >> 1][i & 1] = zero;
 #pragma unroll 2
         for (int e = 0; e < dim; e += 4) {
             float4 q[2], k[2];
@@ -318,12 +286,12 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
             for (int i = 0; i < 2; ++i)
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
-                    a[i][j] = fmaf(q[i].x, k[j].x, fmaf(q[i].y, k[j].y, fmaf(q[i].z, k[j].z, fmaf(q[i].w, k[j].w, a[i][j]))));
+                    a[i][j] = hk_fma4x4(q[i], k[j], a[i][j]);
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i)
 #pragma unroll
-            for (int j = 0; j < 2; ++j) m.A[(t0 + 4 * i) * HK_LA + s0 + 8 * j] = a[i][j];
+            for (int j = 0; j < 2; ++j) m.A[(t0 + 4 * i) * HK_LA + s0 + 8 * j] = (a[i][j].x + a[i][j].y) + (a[i][j].z + a[i][j].w);
     }
     __syncthreads();
     {   // the values into the gates' place, and the second half's q from the chunk's start on
@@ -349,46 +317,7 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
     float4 acc[4][2];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i][0] = acc[i][1] = zero;
-    auto add = [&](float x, float4 v, float4& a) {
-        a.x = fmaf(x, v.x, a.x); a.y = fmaf(x, v.y, a.y); a.z = fmaf(x, v.z, a.z); a.w = fmaf(x, v.w, a.w);
-    };
-    // acc += X[rows][0 .. 3] Y[0 .. 3][values]
-    auto four = [&](const float* X, int ldx, const float* Y) {
-        float4 x[4];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) x[r] = load4(X + (row0 + 4 * r) * ldx);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const float4 y0 = load4(Y + col + 32 * j), y1 = load4(Y + HK_LD + col + 32 * j);
-            const float4 y2 = load4(Y + 2 * HK_LD + col + 32 * j), y3 = load4(Y + 3 * HK_LD + col + 32 * j);
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                add(x[r].x, y0, acc[r][j]); add(x[r].y, y1, acc[r][j]); add(x[r].z, y2, acc[r][j]); add(x[r].w, y3, acc[r][j]);
-            }
-        }
-    };
-    const bool active = (warp & 1) * 64 < vd && (warp >> 1) * 16 < n;
-    for (int i0 = 0; i0 < dim; i0 += HK_SR) {
-        asm volatile("cp.async.wait_group 1;\n" ::);
-        __syncthreads();
-        const float* S = m.S[(i0 / HK_SR) & 1];
-        if (active) {
-            if (dim - i0 >= HK_SR) {
-#pragma unroll
-                for (int i = 0; i < HK_SR; i += 4) four(m.Q + i0 + i, HK_LD, S + i * HK_LD);
-            } else {
-                for (int i = 0; i < dim - i0; i += 4) four(m.Q + i0 + i, HK_LD, S + i * HK_LD);
-            }
-        }
-        __syncthreads();
-        if (i0 + 2 * HK_SR < dim) copy_rows(i0 + 2 * HK_SR);
-        else asm volatile("cp.async.commit_group;\n" ::);
-    }
-    if (active) {
-        const int s_end = ((warp >> 1) + 1) * 16;
-#pragma unroll 2
-        for (int s = 0; s < s_end; s += 4) four(m.A + s, HK_LA, m.F + s * HK_LD);
-    }
+    hk_outputs(acc, m.Q, m.A, m.F, m.S, S0, n, dim, vd, row0, col);
     // the norm over a token's values: the eight lanes of a row, then the row's two warps
     const bool has[2] = {col < vd, col + 32 < vd};
 #pragma unroll

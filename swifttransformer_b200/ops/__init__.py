@@ -44,6 +44,8 @@ def lib() -> ctypes.CDLL:
         _LIB.st_attention_decode_scratch_floats.restype = ctypes.c_longlong
         _LIB.st_latent_attention_mma_scratch.restype = ctypes.c_longlong
         _LIB.st_hgrn2_chunks_scratch.restype = ctypes.c_longlong
+        _LIB.st_delta_rule_scratch_floats.restype = ctypes.c_longlong
+        _LIB.st_delta_rule_chunk_floats.restype = ctypes.c_longlong
         _LIB.st_uniform_host.restype = ctypes.c_float
         _LIB.st_uniform_host.argtypes = [ctypes.c_longlong, ctypes.c_longlong]
     return _LIB
@@ -1469,9 +1471,17 @@ def gqa_attention_plain(q: torch.Tensor, pool: torch.Tensor, layer: int, out: to
 
 
 # ------------------------------------------------------------ the gated delta rule
+# Steps of at least so many tokens per request run in chunks side by side (at 200 the walk is ahead, 93 / 100 us; at 300 the
+# chunks, 138 / 119).
+DELTA_CHUNK_MIN_TOKENS = 256
+
+
 def delta_rule_scratch(n_tokens: int, H: int, G: int, dim: int, vd: int) -> int:
-    lib().st_delta_rule_scratch_floats.restype = ctypes.c_longlong
-    return int(lib().st_delta_rule_scratch_floats(n_tokens, H, G, dim, vd))
+    """Floats of scratch for ``delta_rule``: with them, portions of DELTA_CHUNK_MIN_TOKENS tokens and more run in chunks."""
+    walk = int(lib().st_delta_rule_scratch_floats(n_tokens, H, G, dim, vd))
+    if n_tokens < DELTA_CHUNK_MIN_TOKENS:
+        return walk
+    return max(walk, int(lib().st_delta_rule_chunk_floats(n_tokens, n_tokens // DELTA_CHUNK_MIN_TOKENS, H, G, dim, vd)))
 
 
 def delta_rule_set_lanes(lanes: int) -> None:
@@ -1493,7 +1503,9 @@ def delta_rule(proj: torch.Tensor, b_off: int, a_off: int, g_off: int, conv_w: t
     one token, moved on (else ``conv_state_update`` follows); ``state`` float32 [slots, H, dim, vd] is read and
     moved on.  out [tokens, H * vd] in the type of ``w_a2`` / ``w_g2``.  ``w_a2`` None: the projection holds one
     decay logit per head at a_off and ``dt_bias`` is [H]; ``w_g2`` None: it holds the output gate's H * vd logits
-    at g_off.  ``gate_silu``: the gate is z * sigmoid(z) instead of sigmoid(z)."""
+    at g_off.  ``gate_silu``: the gate is z * sigmoid(z) instead of sigmoid(z).  ``scratch``: ``delta_rule_scratch``
+    elements; steps of DELTA_CHUNK_MIN_TOKENS tokens per request and more (dim and vd multiples of four up to 128) run in
+    chunks of 64 tokens side by side, with less scratch token by token like the others."""
     assert proj.dtype == torch.float32 and proj.is_contiguous() and out.is_contiguous()
     assert out.shape == (proj.shape[0], H * vd) and all(w is None or w.dtype == out.dtype for w in (w_a2, w_g2))
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (H, dim, vd)
@@ -1504,13 +1516,17 @@ def delta_rule(proj: torch.Tensor, b_off: int, a_off: int, g_off: int, conv_w: t
     assert w_a2 is None or (w_a2.is_contiguous() and w_a2.shape[0] == H * dim)
     assert w_g2 is None or (w_g2.is_contiguous() and w_g2.shape[0] == H * vd)
     assert dt_bias.numel() == (H * dim if w_a2 is not None else H)
-    assert scratch.dtype == torch.float32 and scratch.numel() >= delta_rule_scratch(proj.shape[0], H, G, dim, vd)
+    n = proj.shape[0]
+    assert scratch.dtype == torch.float32
+    assert scratch.numel() >= int(lib().st_delta_rule_scratch_floats(n, H, G, dim, vd))
+    chunks = (n >= DELTA_CHUNK_MIN_TOKENS * n_seqs and scratch.data_ptr() % 16 == 0
+              and 0 < int(lib().st_delta_rule_chunk_floats(n, n_seqs, H, G, dim, vd)) <= scratch.numel())
     _check(lib().st_delta_rule(_p(proj), proj.shape[1], 0, b_off, a_off, g_off,
                                w_a2.shape[1] if w_a2 is not None else 0, w_g2.shape[1] if w_g2 is not None else 0,
                                _p(conv_w), taps, _p(conv_state), _p(w_a2), _p(a_log), _p(dt_bias), _p(w_g2),
                                _p(norm_w), _f(eps), _f(out_scale), _p(state), int(write_state), int(single_tokens),
                                _p(scratch), _p(out), _p(positions), _p(seq_of_token), _p(q_start), _p(slots),
-                               proj.shape[0], n_seqs, H, G, dim, vd, _dt(out), _stream(), int(gate_silu)), "delta_rule")
+                               proj.shape[0], n_seqs, H, G, dim, vd, _dt(out), _stream(), int(gate_silu), int(chunks)), "delta_rule")
     return out
 
 

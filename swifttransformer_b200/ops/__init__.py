@@ -1067,6 +1067,14 @@ def latent_attention_mma_applies(q_lat: torch.Tensor, kr: int, rot: int) -> bool
     return q_lat.is_cuda and q_lat.dtype == torch.bfloat16 and bool(lib().st_latent_attention_mma_applies(kr, rot))
 
 
+def latent_attention_tc_applies(q_lat: torch.Tensor, pool: torch.Tensor, layer: int, kr: int, rot: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel takes these sizes: bfloat16, kr and rot multiples of 64, kr <= 512, kr + rot <= 576, pages of
+    8, 16, 32 or 64 positions, 16-byte aligned tensors."""
+    return (q_lat.is_cuda and q_lat.dtype == torch.bfloat16 and pool.stride(0) % 8 == 0 and (layer * pool.stride(1)) % 8 == 0
+            and q_lat.data_ptr() % 16 == 0 and pool.data_ptr() % 16 == 0
+            and bool(lib().st_latent_attention_tc_applies(kr, rot, page_size)))
+
+
 def latent_attention(q_lat: torch.Tensor, pool: torch.Tensor, layer: int, out: torch.Tensor, positions: torch.Tensor,
                      seq_of_token: torch.Tensor, slots: torch.Tensor, block_table: torch.Tensor, nh: int, kr: int,
                      rot: int, page_size: int, scale: float, sink: Optional[torch.Tensor] = None,
@@ -1074,8 +1082,9 @@ def latent_attention(q_lat: torch.Tensor, pool: torch.Tensor, layer: int, out: t
                      q_start: Optional[torch.Tensor] = None, start_pos: Optional[torch.Tensor] = None, n_seqs: int = 0,
                      lens=None, start=None, scratch=None, n_splits: Optional[int] = None,
                      window: int = 0) -> torch.Tensor:
-    """Latent attention of the step's queries (see ``latent_attention_plain`` for the arguments).  kernel: "mma" = the
-    tensor-core kernel over tiles of 64 (token, head) rows (bfloat16; it needs the step's requests: ``q_start``
+    """Latent attention of the step's queries (see ``latent_attention_plain`` for the arguments).  kernel: "tc" = the
+    tcgen05 kernel over tiles of 128 (token, head) rows (``latent_attention_tc_applies``; prompt portions), "mma" = the
+    tensor-core kernel over tiles of 64 (token, head) rows (bfloat16; both need the step's requests: ``q_start``
     [n_seqs + 1], ``start_pos`` [n_seqs] on the device, or ``lens`` / ``start`` as host arrays), "plain" = the float
     kernel with one block per (token, head), "auto" = the first that applies.  Steps whose tiles do not fill the device
     (single tokens, short portions) have their key ranges cut into ``n_splits`` parts (None: chosen from the step's
@@ -1083,12 +1092,23 @@ def latent_attention(q_lat: torch.Tensor, pool: torch.Tensor, layer: int, out: t
     elements for them (None: allocated here)."""
     if kernel == "auto":
         kernel = "mma" if latent_attention_mma_applies(q_lat, kr, rot) else "plain"
+        if n_splits is None and q_start is not None and latent_attention_tc_applies(q_lat, pool, layer, kr, rot, page_size):
+            # Prompt portions: where the mma.sync kernel would not cut the key ranges and the tcgen05 kernel's blocks (128 rows by
+            # 256 value columns) fill half of the SMs.  16 heads, 512 + 64, us (mma.sync): 2 x 1000 tokens 183 (268), 300 tokens
+            # (76 blocks) 41 (54), 450 tokens behind 1200 (114) 128 (192); 450 behind 1200 with 8 heads (58) 131 (119).
+            n = q_lat.shape[0]
+            if (2 * int(lib().st_latent_attention_tc_blocks(n, nh, kr)) >= sm_count(q_lat.device)
+                    and int(lib().st_latent_attention_mma_splits(n, n_seqs, nh, window)) == 1):
+                kernel = "tc"
     if kernel == "plain":
         return latent_attention_plain(q_lat, pool, layer, out, positions, seq_of_token, slots, block_table, nh, kr, rot,
                                       page_size, scale, sink, gates, status, window=window)
-    if kernel != "mma":
+    if kernel not in ("tc", "mma"):
         raise KernelError(f"latent_attention: no kernel named {kernel!r}")
-    if not latent_attention_mma_applies(q_lat, kr, rot):
+    if kernel == "tc" and not latent_attention_tc_applies(q_lat, pool, layer, kr, rot, page_size):
+        raise KernelError("latent_attention: the tcgen05 kernel takes bfloat16, kr and rot in blocks of 64, at most 512 and 576 in all, "
+                          "pages of 8 to 64 positions")
+    if kernel == "mma" and not latent_attention_mma_applies(q_lat, kr, rot):
         raise KernelError("latent_attention: the tensor-core kernel takes bfloat16, kr % 16 == 0, kr <= 512, (kr + rot) % 8 == 0")
     if q_start is None:
         import numpy as np
@@ -1101,6 +1121,14 @@ def latent_attention(q_lat: torch.Tensor, pool: torch.Tensor, layer: int, out: t
     if gates is not None:
         assert gates.dtype == q_lat.dtype and gates.stride(1) == 1 and gates.shape == (q_lat.shape[0], nh)
     n = q_lat.shape[0]
+    if kernel == "tc":
+        st = status if status is not None else _tc_status_word(q_lat.device)
+        _check(lib().st_latent_attention_tc(_p(q_lat), _p(pool), ctypes.c_longlong(pool.shape[0]), stride, offset, _p(out),
+                                            _p(positions), _p(q_start), _p(start_pos), _p(slots), _p(block_table),
+                                            block_table.shape[1], n, n_seqs, nh, kr, rot, page_size, _p(sink), _p(gates),
+                                            gates.stride(0) if gates is not None else 0, _f(scale), _p(st), _stream(), window),
+               "latent_attention_tc")
+        return out
     if n_splits is None:
         n_splits = int(lib().st_latent_attention_mma_splits(n, n_seqs, nh, window))
     partial = None

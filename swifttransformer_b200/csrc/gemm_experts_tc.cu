@@ -31,7 +31,6 @@
 #include "tma_host.h"
 
 #define GE_THREADS 192          // and 128 more where rows are gathered
-// stages of gathered rows under way per thread, beside the one just asked for: two less than the ring has
 #define GE_RING_BYTES (200 * 1024)
 #define GE_STAGES(BN) (GE_RING_BYTES / (GE_BM * 128 + (BN) * 128) > GE_MAX_STAGES ? GE_MAX_STAGES : GE_RING_BYTES / (GE_BM * 128 + (BN) * 128))
 #define GE_BM 128
@@ -62,6 +61,23 @@ __device__ __forceinline__ bool ge_wait(uint32_t mbar, uint32_t parity, volatile
 __device__ __forceinline__ void ge_arrive(uint32_t mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory");
 }
+// 8 consecutive float columns of this thread's lane of tensor memory, as tc_ld32
+__device__ __forceinline__ void ge_ld8(uint32_t taddr, float* v) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(v);
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr) : "memory");
+}
+__device__ __forceinline__ void ge_act8(float* v, int act) {
+    if (act == 4) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = apply_act(v[j], 4);
+    } else if (act) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = apply_act(v[j], act);
+    }
+}
+
 struct ExpertsTile {
     int expert, row0, rows, n0;
 };
@@ -94,7 +110,7 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
     __shared__ int s_dead, s_issued;
     __shared__ int s_before[GE_MAX_EXPERTS + 1];
     constexpr uint32_t A_BYTES = GE_BM * 128, W_BYTES = BN * 128, STAGE = A_BYTES + W_BYTES;
-    constexpr int TMEM_COLS = 2 * BN, stages = GE_STAGES(BN), LAG = stages - 2;
+    constexpr int TMEM_COLS = 2 * BN, stages = GE_STAGES(BN);
     const uint32_t base = (tc_smem(ge_raw) + 1023u) & ~1023u;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     volatile int* dead = &s_dead;
@@ -169,7 +185,7 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
         // ---- gathered rows of a: a thread copies one 16-byte piece of every sixteenth row of the tile
         const int t128 = tid - GE_THREADS, piece = t128 & 7, r_first = t128 >> 3;
         const uint32_t at = (uint32_t)(r_first * 128 + ((piece ^ (r_first & 7)) << 4));      // rows 16 apart: the same swizzle
-        int s = 0, turn = 0, it = 0, s_arrive = 0;
+        int s = 0, turn = 0;
         bool ok = true;
         for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x) {
             const ExpertsTile t = ge_tile(tile, n_tiles_n, bn_out, s_before, sh);
@@ -187,22 +203,12 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
 #pragma unroll
                 for (int i = 0; i < GE_BM / 16; ++i)
                     if (r_first + 16 * i < t.rows) tc_cp16(dst + i * 2048, in_k ? src[i] + k * GE_BK : a, in_k);
-                tc_cp_commit();
-                if (++it > LAG) {
-                    tc_cp_wait<LAG>();
-                    tc_fence_async_smem();
-                    ge_arrive(tc_smem(&s_full[s_arrive]));
-                    if (++s_arrive == stages) s_arrive = 0;
-                }
+                // the thread's arrival when its copies have landed; the products' thread makes them visible to the tensor cores
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(tc_smem(&s_full[s])) : "memory");
                 if (++s == stages) { s = 0; ++turn; }
             }
         }
-        tc_cp_wait<0>();
-        tc_fence_async_smem();
-        for (int i = min(it, LAG); i > 0; --i) {
-            ge_arrive(tc_smem(&s_full[s_arrive]));
-            if (++s_arrive == stages) s_arrive = 0;
-        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
     } else if (warp == 5 && lane == 0) {
         // ---- products
         const uint32_t idesc = tc_idesc(GE_BM, BN, 0, 0);
@@ -213,6 +219,7 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
             tc_fence_after_sync();
             for (int k = 0; k < n_k; ++k) {
                 if (!ge_wait(tc_smem(&s_full[s]), turn & 1, dead)) break;
+                if (GATHER) tc_fence_async_smem();
                 tc_fence_after_sync();
                 const uint64_t da = tc_desc(base + s * STAGE, 16, 1024), dw = tc_desc(base + s * STAGE + A_BYTES, 16, 1024);
 #pragma unroll
@@ -236,39 +243,36 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
             if (warp * 32 < t.rows) {
                 bf16* dst = c + (size_t)(t.row0 + r) * sh.ldc + t.n0;
                 const bool live = r < t.rows;
-                for (int c0 = 0; c0 < bn_out; c0 += 32) {
+                // eight columns at a time and not unrolled: the activations' code is long, and a launch of few rows runs it
+                // once (unrolled over 32 columns it took 11 us of a decode step's 30)
+#pragma unroll 1
+                for (int c0 = 0; c0 < bn_out; c0 += 8) {
                     if (t.n0 + c0 >= sh.n_out) break;
-                    float v[32];
-                    tc_ld32(t_row + c0, v);
+                    float v[8], u[8];
+                    ge_ld8(t_row + c0, v);
+                    if (sh.gated) ge_ld8(t_row + BN / 2 + c0, u);
+                    tc_ld_wait();
                     if (sh.gated) {
-                        float u[32];
-                        tc_ld32(t_row + BN / 2 + c0, u);
-                        tc_ld_wait();
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
-                            v[j] = apply_act(to_f32(from_f32<bf16>(v[j])), sh.act) * to_f32(from_f32<bf16>(u[j]));
-                    } else {
-                        tc_ld_wait();
-                        if (sh.act) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = apply_act(v[j], sh.act);
-                        }
+                        for (int j = 0; j < 8; ++j) v[j] = to_f32(from_f32<bf16>(v[j]));
                     }
-                    if (live && sh.vec && t.n0 + c0 + 32 <= sh.n_out) {
+                    ge_act8(v, sh.act);
+                    if (sh.gated) {
 #pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            uint4 p;
-                            uint32_t* w4 = reinterpret_cast<uint32_t*>(&p);
+                        for (int j = 0; j < 8; ++j) v[j] *= to_f32(from_f32<bf16>(u[j]));
+                    }
+                    if (live && sh.vec && t.n0 + c0 + 8 <= sh.n_out) {
+                        uint4 p;
+                        uint32_t* w4 = reinterpret_cast<uint32_t*>(&p);
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) {
-                                const __nv_bfloat162 b = __floats2bfloat162_rn(v[j + 2 * e], v[j + 2 * e + 1]);
-                                w4[e] = *reinterpret_cast<const uint32_t*>(&b);
-                            }
-                            *reinterpret_cast<uint4*>(dst + c0 + j) = p;
+                        for (int e = 0; e < 4; ++e) {
+                            const __nv_bfloat162 b = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+                            w4[e] = *reinterpret_cast<const uint32_t*>(&b);
                         }
+                        *reinterpret_cast<uint4*>(dst + c0) = p;
                     } else if (live) {
 #pragma unroll
-                        for (int j = 0; j < 32; ++j)
+                        for (int j = 0; j < 8; ++j)
                             if (t.n0 + c0 + j < sh.n_out) dst[c0 + j] = from_f32<bf16>(v[j]);
                     }
                     __syncwarp();                         // the next tcgen05.ld is the whole warp's

@@ -90,6 +90,7 @@ def _p(t: Optional[torch.Tensor]):
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_current_device = getattr(torch._C, "_cuda_getDevice", torch.cuda.current_device)
 
 
 def _stream():
@@ -97,7 +98,7 @@ def _stream():
     costs ~15 us of host time per call (a fifth of the host's time for a step of eager launches); the raw
     query behind it is used where this torch has it."""
     if _raw_stream is not None:
-        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
+        return ctypes.c_void_p(_raw_stream(_current_device()))
     return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
@@ -307,7 +308,7 @@ def gemm_skinny(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] =
     assert w.is_contiguous()
     n, k = a.shape
     m = w.shape[0]
-    out = torch.empty((n, m), dtype=out_dtype, device=a.device)
+    out = a.new_empty((n, m), dtype=out_dtype)
     _check(lib().st_gemm_skinny(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act],
                                 int(out_dtype == torch.float32), _stream()), "gemm_skinny")
     return out
@@ -461,7 +462,7 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = 
     assert w.is_contiguous()
     n, k = a.shape
     m = w.shape[0]
-    out = torch.empty((n, m), dtype=out_dtype, device=a.device)
+    out = a.new_empty((n, m), dtype=out_dtype)
     _check(lib().st_gemm_plain(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], _dt(a),
                                int(out_dtype == torch.float32), _stream()), "gemm_plain")
     return out
@@ -1194,8 +1195,8 @@ def moe_choose(logits: torch.Tensor, n_experts: int, top: int, positions: Option
     """The choice of ``moe_route`` alone, from float32 router logits [tokens, >= n_experts] that a product left."""
     n = logits.shape[0]
     assert logits.dtype == torch.float32 and logits.is_contiguous() and logits.shape[1] >= n_experts
-    experts = torch.empty((n, top), dtype=torch.int32, device=logits.device)
-    weights = torch.empty((n, top), dtype=torch.float32, device=logits.device)
+    experts = logits.new_empty((n, top), dtype=torch.int32)
+    weights = logits.new_empty((n, top), dtype=torch.float32)
     _check(lib().st_moe_choose(_p(logits), logits.shape[1], n, n_experts, top,
                                *_route_rule(scores, groups, renorm, scale, correction, group_score, n_experts), _p(positions), _p(experts), _p(weights), _stream()), "moe_choose")
     return experts, weights
@@ -1215,8 +1216,8 @@ def moe_route(h: torch.Tensor, w_router: torch.Tensor, top: int, positions: Opti
     score alone."""
     n, width = h.shape
     assert h.is_contiguous() and w_router.dtype == torch.float32 and w_router.is_contiguous() and w_router.shape[1] == width
-    experts = torch.empty((n, top), dtype=torch.int32, device=h.device)
-    weights = torch.empty((n, top), dtype=torch.float32, device=h.device)
+    experts = h.new_empty((n, top), dtype=torch.int32)
+    weights = h.new_empty((n, top), dtype=torch.float32)
     gate = torch.empty((n,), dtype=torch.float32, device=h.device) if w_gate is not None else None
     if w_gate is not None:
         assert w_gate.dtype == torch.float32 and w_gate.numel() == width and w_gate.is_contiguous()
@@ -1243,9 +1244,9 @@ def moe_sort(experts: torch.Tensor, n_experts: int) -> ExpertOrder:
     n, top = experts.shape
     items, rows = n * top, grouped_tile_rows()
     cap = (items + rows - 1) // rows + n_experts
-    buf = torch.empty(n_experts + 1 + 2 * items + 2 * cap, dtype=torch.int32, device=experts.device)
-    offsets, rest = buf[:n_experts + 1], buf[n_experts + 1:]
-    sorted_items, place, tile_group, tile_row0 = rest[:items], rest[items:2 * items], rest[2 * items:2 * items + cap], rest[2 * items + cap:]
+    buf = experts.new_empty(n_experts + 1 + 2 * items + 2 * cap, dtype=torch.int32)
+    # (one split and not five slices: 16 us of host time per call were mostly theirs)
+    offsets, sorted_items, place, tile_group, tile_row0 = buf.split((n_experts + 1, items, items, cap, cap))
     _check(lib().st_moe_sort(_p(experts), items, n_experts, rows, cap, _p(offsets), _p(sorted_items), _p(place),
                              _p(tile_group), _p(tile_row0), _stream()), "moe_sort")
     return ExpertOrder(offsets, sorted_items, place, tile_group, tile_row0, items, top)
@@ -1260,7 +1261,7 @@ def gemm_experts(a: torch.Tensor, w: torch.Tensor, order: ExpertOrder, gather: b
     the plain one."""
     assert a.is_contiguous() and w.is_contiguous() and w.dim() == 3 and a.dtype == w.dtype and a.shape[1] == w.shape[2]
     n_out = w.shape[1] // 2 if gated else w.shape[1]
-    out = torch.empty((order.n_items, n_out), dtype=a.dtype, device=a.device)
+    out = a.new_empty((order.n_items, n_out))
     ll = ctypes.c_longlong
     if GROUPED_MMA and a.dtype == torch.bfloat16 and bool(lib().st_gemm_experts_tc_applies(w.shape[0], w.shape[2])):
         _check(lib().st_gemm_experts_tc(_p(a), ll(a.shape[0]), _p(w), _p(out), w.shape[0], order.n_items, n_out, w.shape[2],
@@ -1286,7 +1287,7 @@ def moe_combine(y: torch.Tensor, order: ExpertOrder, weights: torch.Tensor, shar
     n, top = weights.shape
     width = y.shape[1]
     assert y.is_contiguous() and (shared is None or (shared.is_contiguous() and shared.dtype == y.dtype))
-    out = torch.empty((n, width), dtype=out_dtype, device=y.device)
+    out = y.new_empty((n, width), dtype=out_dtype)
     if identity is not None:
         assert identity.is_contiguous() and identity.dtype == y.dtype and identity.shape == (n, width)
         assert experts.dtype == torch.int32 and experts.is_contiguous() and experts.shape == (n, top)

@@ -14,16 +14,16 @@
 // Warps: 0-3 read the accumulator (tcgen05.ld, a quarter of tensor memory each) and store; 4 copies weights, and rows of a
 // where they are neighbours, by TMA boxes of 64 k (a in boxes of 32 rows, as many as the tile has); 5 issues tcgen05.mma;
 // 6-9, where the rows are gathered, copy them by 16-byte asynchronous copies (tile::gather4 was measured at 20 cycles a row:
-// 262 us for a product of 90 GFLOP that takes 119 this way).  Copies and products meet on a ring of stages; the accumulator
+// 262 us for a product of 90 GFLOP that takes 109 this way).  Copies and products meet on a ring of stages; the accumulator
 // is double-buffered in tensor memory, so that a tile is stored under the next one's products.  Rows of a tile past its
 // expert's end hold other rows or what the shared memory held: a row of the product depends on its own row of a alone, and
 // those are not stored.
 //
 // Bound by the tensor cores for prompts and by the weights' way from memory for few rows.  Measured on one B200 (with about
 // 6 us of an empty launch between events, inputs not in cache; in brackets the mma.sync kernel with tiles of 64 x 64):
-// 4000 items, 8 experts, 2048 -> 5504: 119 us = 800 TFLOP/s (481); 2752 -> 2048: 57 us = 880 TFLOP/s (252).  300 tokens x 2,
-// 8 experts, gated 4096 -> 1024: 61 us (107).  38 items, 16 experts, 2048 -> 5504: 84 us, 361 MB = 4.6 TB/s (129).  16 items, 8
-// experts, gated 2048 -> 512: 33 us (37).
+// 4000 items, 8 experts, 2048 -> 5504: 109 us = 880 TFLOP/s (481); 2752 -> 2048: 55 us = 920 TFLOP/s (252).  300 tokens x 2,
+// 8 experts, gated 4096 -> 1024: 55 us (107).  38 items, 16 experts, 2048 -> 5504: 84 us, 361 MB = 4.6 TB/s (129).  16 items, 8
+// experts, gated 2048 -> 512: 29 us (37).
 //
 // Waits are bounded: one that expires marks the block dead, `status` gets 5, and the block waits (again with a limit) for its
 // copies under way, frees its tensor memory and leaves.
@@ -302,8 +302,9 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
 
 // The rows of w in a tile (gated tiles count their gate and up rows).  The wider, the less a is read again; a launch has at
 // least a row tile per expert that any item may go to.  Lines by measurement (us with 64 / 128 / 256 rows): the widest while
-// every SM gets a tile (4000 items, 5504 rows: 277 / 168 / 119), then 128 while half of the SMs do (600 items on 8 experts, 2048
-// gate and up rows: 68 / 61 / 84; 300 items on 16 experts, 1024: 41 / 38 / 51; 16 items on 8, 2048: 16.4 / 14.4 / 14.4), else 64.
+// every SM gets a tile (4000 items, 5504 rows: 256 / 156 / 109), then 128 while half of the SMs do (600 items on 8 experts, 2048
+// gate and up rows: 65 / 55 / 76; 300 items on 16 experts, 1024: 37 / 31 / 39; 16 items on 8, 2048: 16.4 / 14.4 / 16.4), else 64
+// (16 items on 8, 1024: 31 / 27 / 35, where the widths are as far apart as two runs of one are).
 static int ge_pick_bn(int n_items, int n_experts, int w_rows, int sms) {
     int row_tiles = (n_items + GE_BM - 1) / GE_BM;
     if (row_tiles < n_experts) row_tiles = n_items < n_experts ? n_items : n_experts;

@@ -1,7 +1,7 @@
 // Grouped-query attention for prompt portions on the warp-level tensor cores (mma.sync m16n8k16, bfloat16 in,
-// float accumulate): one block per (128 query rows of one request, query head).
+// float accumulate): one block per (64 or 128 query rows of one request, query head).
 //
-// Eight warps carry sixteen query rows each.  All read the same key tile (64 keys) and value tile from shared
+// Four or eight warps carry sixteen query rows each.  All read the same key tile (64 keys) and value tile from shared
 // memory, filled by 16-byte asynchronous copies from the pages (two stages: the next tile lands while this one
 // is multiplied).  Each warp keeps S = Q K^T, the running maximum and sum and O = P V (16 x vd) in registers.
 //
@@ -14,12 +14,24 @@
 // Sizes are template arguments rounded up (dim to 32/64/96/128, vd to 32/64/96/128/256) with the padding columns
 // zero in shared memory; dim and vd themselves must be multiples of 8 (16-byte pieces).  Scores and the softmax
 // are float; the weights' exponentials use the fast exp2.
+//
+// Bound by the latency of the chain product - softmax - product in a warp, which only other warps hide, and by the last wave
+// of blocks.  So all heads of a tile come before the next tile (the callers' lists hold the longest first, which a grid of
+// heads over tiles dealt out again for every head), a fragment of keys for two steps of 16 is one ldmatrix, and rows per block
+// follow GT_BLOCK_ROWS below.  Which rows share a block changes no number: a row's sums run over key tiles at absolute
+// positions.  2000 tokens, 16 heads on 4, dim 64, vd 128, window 512: 71.7 -> 49.2 us on one B200 (about 6 us of them an empty
+// launch between events), over all earlier keys 131 -> 100; dim 128: 84 -> 76 and 156 -> 97.
 #include "gqa_attention.cuh"
 #include "mma_sync.cuh"
 
-#define GT_ROWS 128     // query rows per block
 #define GT_KEYS 64      // keys per tile
-#define GT_THREADS 256
+// Query rows per block, from the rounded sizes.  64 rows leave room for three blocks on an SM (at most 168 registers a thread,
+// at most 53 KB of shared memory each): twelve warps instead of eight, and an evener last wave.  128 rows read a key tile half
+// as often and runs the longest rows' chain with fewer warps beside it.  us with 64 / 128 rows, 16 heads on 4, window 512 and
+// all keys, 2000 tokens: dim 64, vd 128: 49 / 66, 99 / 84 (8000 tokens: 184 / 213, 903 / 1039; 32 heads: 88 / 100, 148 / 160;
+// 4 heads: 31 / 37, 72 / 80); dim 64, vd 64: 39 / 55, 84 / 70; dim 128, vd 128: 66 / 76, 127 / 97; dim 128, vd 256: 100 / 100,
+// 141 / 131.
+#define GT_BLOCK_ROWS(DIMT, VDT) ((DIMT) <= 64 && (VDT) <= 128 ? 64 : 128)
 
 template <int DIMT, int VDT>
 struct GqaTileSmem {
@@ -31,7 +43,7 @@ struct GqaTileSmem {
 
 // keys key0 .. key0 + 63 of kv head kvh into a stage; a key the block's rows do not see (past `hi`, or between
 // the kept first keys and `lo`) is zeros and its page is not looked up
-template <int DIMT, int VDT>
+template <int DIMT, int VDT, int THREADS>
 __device__ __forceinline__ void gqa_load_kv_tile(bf16* stage, const bf16* __restrict__ pool, const DiffCache& cache,
                                                  const int* __restrict__ bt, int kvh, int key0, int lo, int hi,
                                                  int keep_first, int* __restrict__ status) {
@@ -40,8 +52,9 @@ __device__ __forceinline__ void gqa_load_kv_tile(bf16* stage, const bf16* __rest
     bf16* sv = stage + GT_KEYS * L::K_LD;
     constexpr int KC = DIMT / 8, VC = VDT / 8;      // 16-byte pieces per row
     const int dim = cache.kd, vd = cache.vd, ps = cache.page_size;
-    // four threads per key row: one look-up of the row's page, then the row's pieces in turn
-    const int row = threadIdx.x >> 2;
+    // a few threads per key row: one look-up of the row's page, then the row's pieces in turn
+    constexpr int PER_ROW = THREADS / GT_KEYS;
+    const int row = threadIdx.x / PER_ROW;
     const int key = key0 + row;
     int page = -1;
     if (key <= hi && (key >= lo || key < keep_first)) {
@@ -50,7 +63,7 @@ __device__ __forceinline__ void gqa_load_kv_tile(bf16* stage, const bf16* __rest
     }
     const bf16* krow = page >= 0 ? cache_keys(pool, cache, page, kvh, key % ps) : nullptr;
     const bf16* vrow = page >= 0 ? cache_values(pool, cache, page, kvh, key % ps) : nullptr;
-    for (int c = threadIdx.x & 3; c < KC + VC; c += 4) {
+    for (int c = threadIdx.x % PER_ROW; c < KC + VC; c += PER_ROW) {
         if (c < KC) {
             const int e = c * 8;
             bf16* dst = sk + row * L::K_LD + e;
@@ -65,8 +78,8 @@ __device__ __forceinline__ void gqa_load_kv_tile(bf16* stage, const bf16* __rest
     }
 }
 
-template <int DIMT, int VDT>
-__global__ void __launch_bounds__(GT_THREADS)
+template <int DIMT, int VDT, int ROWS>
+__global__ void __launch_bounds__(ROWS * 2, ROWS == 64 ? 3 : 1)
 gqa_attention_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pool, DiffCache cache,
                            bf16* __restrict__ out, const int* __restrict__ tiles, int parts,
                            const int* __restrict__ q_start, const int* __restrict__ start_pos,
@@ -76,17 +89,19 @@ gqa_attention_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__ 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     bf16* smem = reinterpret_cast<bf16*>(smem_raw);
     ST_PDL_TRIGGER();
-    const int tile = blockIdx.x / parts, part = blockIdx.x % parts;
-    const int req = tiles[2 * tile], off = tiles[2 * tile + 1] + part * GT_ROWS;
+    // all heads of a part of a tile, then the next; a tile's last part has its longest key ranges
+    const int h = blockIdx.x % nh, place = blockIdx.x / nh;
+    const int tile = place / parts, part = parts - 1 - place % parts;
+    const int req = tiles[2 * tile], off = tiles[2 * tile + 1] + part * ROWS;
     const int first = q_start[req], n_new = q_start[req + 1] - first;
     if (off >= n_new) return;                           // padding tile, or the part lies past the request's tokens
-    const int h = blockIdx.y, nkv = cache.nkv, vd = cache.vd, dim = cache.kd;
+    const int nkv = cache.nkv, vd = cache.vd, dim = cache.kd;
     const int kvh = h / (nh / nkv);
     const int start = start_pos[req];
     const int* bt = block_table + (size_t)slots[req] * cache.max_pages;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     const int row0 = warp * 16;
-    const int rows_here = min(GT_ROWS, n_new - off);
+    const int rows_here = min(ROWS, n_new - off);
     const int p_first = start + off, hi = p_first + rows_here - 1;
     const int lo = gqa_lo(p_first, mask);
     const bool limited = gqa_limited(mask);
@@ -136,12 +151,12 @@ gqa_attention_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__ 
     const int n_a = min((head_end + GT_KEYS - 1) / GT_KEYS, k_b);
     const int n_t = n_a + kt_last - k_b + 1;
 #define GT_TILE(i) ((i) < n_a ? (i) : k_b + (i) - n_a)
-    gqa_load_kv_tile<DIMT, VDT>(smem, pool, cache, bt, kvh, GT_TILE(0) * GT_KEYS, lo, hi, keep, status);
+    gqa_load_kv_tile<DIMT, VDT, ROWS * 2>(smem, pool, cache, bt, kvh, GT_TILE(0) * GT_KEYS, lo, hi, keep, status);
     cp_async_commit();
     for (int i = 0; i < n_t; ++i) {
         bf16* stage = smem + (i & 1) * L::STAGE;
         if (i + 1 < n_t)
-            gqa_load_kv_tile<DIMT, VDT>(smem + ((i + 1) & 1) * L::STAGE, pool, cache, bt, kvh, GT_TILE(i + 1) * GT_KEYS, lo,
+            gqa_load_kv_tile<DIMT, VDT, ROWS * 2>(smem + ((i + 1) & 1) * L::STAGE, pool, cache, bt, kvh, GT_TILE(i + 1) * GT_KEYS, lo,
                                         hi, keep, status);
         cp_async_commit();
         cp_async_wait<1>();
@@ -160,11 +175,11 @@ gqa_attention_tiles_kernel(const bf16* __restrict__ q, const bf16* __restrict__ 
 #pragma unroll
                 for (int x = 0; x < 4; ++x) s[nt][x] = 0.f;
 #pragma unroll
-                for (int ks = 0; ks < DIMT / 16; ++ks) {
-                    const bf16* kp = sk + (nt * 8 + g) * L::K_LD + ks * 16 + 2 * tq;
-                    const uint32_t b0 = *reinterpret_cast<const uint32_t*>(kp);
-                    const uint32_t b1 = *reinterpret_cast<const uint32_t*>(kp + 8);
+                for (int ks = 0; ks < DIMT / 16; ks += 2) {
+                    uint32_t b0, b1, b2, b3;        // the eight keys' fragments of two steps of 16
+                    ldmatrix_x4(b0, b1, b2, b3, sk + (nt * 8 + (lane & 7)) * L::K_LD + ks * 16 + (lane >> 3) * 8);
                     mma_bf16(s[nt], qa[ks], b0, b1);
+                    mma_bf16(s[nt], qa[ks + 1], b2, b3);
                 }
             }
             float tmax[2] = {-INFINITY, -INFINITY};
@@ -285,13 +300,16 @@ static int launch_gqa_tiles(const void* q, const void* pool, const DiffCache& c,
                             const GqaEpilogue& epi, int* status, cudaStream_t s) {
     using L = GqaTileSmem<DIMT, VDT>;
     const size_t smem = L::BYTES;
-    auto kern = gqa_attention_tiles_kernel<DIMT, VDT>;
+    constexpr int ROWS = GT_BLOCK_ROWS(DIMT, VDT);
+    auto kern = gqa_attention_tiles_kernel<DIMT, VDT, ROWS>;
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
     }
-    const int parts = (tile_rows + GT_ROWS - 1) / GT_ROWS;
-    kern<<<dim3(n_tiles * parts, nh), GT_THREADS, smem, s>>>((const bf16*)q, (const bf16*)pool, c, (bf16*)out, tiles, parts,
+    const int parts = (tile_rows + ROWS - 1) / ROWS;
+    const long long blocks = (long long)n_tiles * parts * nh;
+    if (blocks > 0x7fffffffLL) return ST_ERR_TOO_LARGE;
+    kern<<<dim3((unsigned)blocks), ROWS * 2, smem, s>>>((const bf16*)q, (const bf16*)pool, c, (bf16*)out, tiles, parts,
                                                             q_start, start_pos, slots, block_table, nh, scale, mask,
                                                             has_sink, sink, epi, status);
     return st_launch_status();

@@ -105,8 +105,8 @@ attention_plain_kernel(const T* __restrict__ q, const T* __restrict__ pool, T* _
 // and value rows come 32 at a time through three stages of shared memory filled by 16-byte asynchronous copies.  Bound by
 // shared memory (six reads of two cycles per 32 multiply-adds of a warp for the scores).
 // A run of one token: a thread per key reads its row from memory; the tile's values arrive meanwhile in shared memory.
-// Three prompts of 700 tokens in all, 32 heads of 64: 112 us; the general kernel 1089 (each of its blocks reads all its keys
-// again, the lanes of a warp in 32 different rows at once).
+// Three prompts of 700 tokens in all, 32 heads of 64: 89 us (112 with the tiles in ascending order, once per head); the general
+// kernel 1089 (each of its blocks reads all its keys again, the lanes of a warp in 32 different rows at once).
 #define AF_ROWS 32
 #define AF_SUB 32
 #define AF_STAGES 3
@@ -425,8 +425,9 @@ attention_f32_kernel(const AttentionF32 p) {
     extern __shared__ __align__(16) float smem[];
     __shared__ long long rows[2 * KT];
     __shared__ float scratch[32];
-    const int lane = threadIdx.x & 31, h = blockIdx.y, kvh = h / (p.nh / p.nkv);
-    const int first = blockIdx.x * AF_ROWS, t = first + lane;
+    // all heads of a tile of tokens before the next tile, a request's last tokens, who see the most keys, first
+    const int lane = threadIdx.x & 31, h = blockIdx.x % p.nh, kvh = h / (p.nh / p.nkv);
+    const int first = (gridDim.x / p.nh - 1 - blockIdx.x / p.nh) * AF_ROWS, t = first + lane;
     const int pos = t < p.n_tokens ? p.positions[t] : -1;
     const int seq = pos >= 0 ? p.seq_of_token[t] : -1;
     // runs: neighbouring tokens of one request at neighbouring positions (each warp finds the same ones)
@@ -455,7 +456,8 @@ static int attention_f32(const AttentionF32& p, cudaStream_t s) {
     int z = (int)((want + have - 1) / have);
     z = z > AF_ROWS ? AF_ROWS : z;
     if (z > p.n_tokens) z = p.n_tokens;
-    dim3 grid(tiles, p.nh, z);
+    if (have > 0x7fffffffLL) return ST_ERR_TOO_LARGE;
+    dim3 grid((unsigned)have, 1, z);
 #define AF_LAUNCH(NI)                                                                                                  \
     do {                                                                                                               \
         const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \

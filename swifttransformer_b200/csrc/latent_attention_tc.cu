@@ -2,7 +2,7 @@
 //
 // The mathematics is that of latent_attention_mma.cu: the rows of a query tile are (token, head) pairs of one request in the
 // order they lie in memory, all heads read the same cached rows [c | k_rot], and the values are the first kr numbers of the
-// very rows that are the keys.  A block serves 128 such rows and up to 256 of the value columns (blockIdx.y; wider latents have
+// very rows that are the keys.  A block serves 128 such rows and up to 256 of the value columns (wider latents have
 // their scores formed once per 256 columns: tensor memory has room for 256 columns of sums beside the scores).
 //
 // Shared memory holds the query tile (kb blocks of [128][64], kb = (kr + rot) / 64 <= 9) and one tile of 64 keys (kb
@@ -15,8 +15,8 @@
 //            operand of O += P V; the reference moves, and O is rescaled, only when a row's maximum has grown by 2^8
 // At the end the sink joins the denominator, the gate multiplies, and the row is stored.
 //
-// Measured on one B200, 16 heads, kr 512, rot 64, pages of 16: two prompts of 1000 tokens 175 us (mma.sync kernel 260), one of
-// 700 58 (86), 450 tokens behind 1200 120 (184).  A tile of 64 keys takes about 7300 clocks: 2000 for the key-only blocks' copies
+// Measured on one B200, 16 heads, kr 512, rot 64, pages of 16: two prompts of 1000 tokens 168 us (mma.sync kernel 251; 172
+// while the launch walked all tiles once per 256 value columns), one of 700 58 (86), 450 tokens behind 1200 120 (184).  A tile of 64 keys takes about 7300 clocks: 2000 for the key-only blocks' copies
 // (under the softmax of the tile before), 1500 more for the values', 2100 for the scores on them: a product of 64 columns
 // takes as long as one of 256, about 130 clocks per 16 dimensions, for its rows of the query tile are read each time.
 //
@@ -37,7 +37,7 @@
 
 struct LatentTc {
     int kb, vb, vb_all;                 // blocks of 64: of a row, of this launch's value columns per block, of kr
-    int max_pages, page_size, n_seqs, nh, window, gate_ld, n_tiles;
+    int max_pages, page_size, n_seqs, nh, window, gate_ld, n_tiles, parts;
     float scale_log2;
     const int *positions, *q_start, *start_pos, *slots, *block_table;
     const float* sink;
@@ -73,7 +73,8 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     ST_PDL_WAIT();
     ST_PDL_TRIGGER();
     if (tid == 0) {
-        int tile = p.n_tiles - 1 - blockIdx.x, req = -1;      // the last tiles of a request have the longest key ranges: first
+        // the last tiles of a request have the longest key ranges: first, all value columns of a tile side by side
+        int tile = p.n_tiles - 1 - blockIdx.x / p.parts, req = -1;
         for (int i = 0; i < p.n_seqs; ++i) {
             const int tiles = ((p.q_start[i + 1] - p.q_start[i]) * p.nh + LT_ROWS - 1) / LT_ROWS;
             if (tile < tiles) { req = i; break; }
@@ -108,7 +109,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     const int hi = start + last_row / p.nh + 1;               // keys lo .. hi - 1 are seen by some row of the tile
     const int lo = p.window > 0 ? max(0, start + r0 / p.nh - p.window + 1) : 0;
     const int kt0 = lo / LT_KEYS, n_kt = (hi + LT_KEYS - 1) / LT_KEYS - kt0;
-    const int v0 = blockIdx.y * p.vb, nv = min(p.vb, p.vb_all - v0);      // this block's values: blocks v0 .. v0 + nv - 1
+    const int v0 = blockIdx.x % p.parts * p.vb, nv = min(p.vb, p.vb_all - v0);      // this block's values: blocks v0 .. v0 + nv - 1
 
     if (warp >= 4 && warp < 4 + LT_COPIERS) {
         // ---- copies.  A page without a key this query tile may see may have been given back: its rows (masked later) are
@@ -333,7 +334,7 @@ ST_EXPORT int st_latent_attention_tc(const void* q_lat, const void* pool, long l
         return ST_ERR_BAD_ARG;
     const int kd = kr + rot;
     const long long tiles = ((long long)n_tokens * nh + LT_ROWS - 1) / LT_ROWS + n_seqs;
-    if (tiles > 0x7fffffffLL || (long long)n_tokens * nh > 0x7fffffffLL || n_pages > 0x7fffffffLL) return ST_ERR_TOO_LARGE;
+    if (tiles * ((kr / 64 + 3) / 4) > 0x7fffffffLL || (long long)n_tokens * nh > 0x7fffffffLL || n_pages > 0x7fffffffLL) return ST_ERR_TOO_LARGE;
     const unsigned long long qd[2] = {(unsigned long long)kd, (unsigned long long)n_tokens * nh};
     const unsigned qb[2] = {64, LT_ROWS};
     const unsigned long long kdim[3] = {(unsigned long long)kd, (unsigned long long)page_size, (unsigned long long)n_pages};
@@ -344,7 +345,7 @@ ST_EXPORT int st_latent_attention_tc(const void* q_lat, const void* pool, long l
         st_tma_encode_bf16_strided(&k_map, (const bf16*)pool + entry_offset, 3, kdim, kst, kb)) return ST_ERR_BAD_ARG;
     LatentTc p;
     p.kb = kd / 64; p.vb_all = kr / 64;
-    const int parts = (p.vb_all + 3) / 4;
+    const int parts = p.parts = (p.vb_all + 3) / 4;
     p.vb = (p.vb_all + parts - 1) / parts;
     p.max_pages = max_pages; p.page_size = page_size; p.n_seqs = n_seqs; p.nh = nh; p.window = window; p.gate_ld = gate_ld;
     p.n_tiles = (int)tiles; p.scale_log2 = scale * 1.4426950408889634f;
@@ -353,6 +354,6 @@ ST_EXPORT int st_latent_attention_tc(const void* q_lat, const void* pool, long l
     const size_t smem = (size_t)p.kb * (LT_Q_BLK + LT_K_BLK) + 1024;
     const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    return st_launch_pdl("latent_tc", latent_attention_tc_kernel, dim3((unsigned)tiles, parts), dim3(LT_THREADS), smem,
+    return st_launch_pdl("latent_tc", latent_attention_tc_kernel, dim3((unsigned)(tiles * parts)), dim3(LT_THREADS), smem,
                          (cudaStream_t)stream, q_map, k_map, (bf16*)out, p, status);
 }

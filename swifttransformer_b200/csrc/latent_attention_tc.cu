@@ -112,8 +112,8 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     const int v0 = blockIdx.x % p.parts * p.vb, nv = min(p.vb, p.vb_all - v0);      // this block's values: blocks v0 .. v0 + nv - 1
 
     if (warp >= 4 && warp < 4 + LT_COPIERS) {
-        // ---- copies.  A page without a key this query tile may see may have been given back: its rows (masked later) are
-        // filled from the tile's first live page, so that they hold finite numbers.
+        // ---- copies.  A page without a key this query tile may see may have been given back: its rows (masked, and zeroed as
+        // values) are filled from the tile's first live page.
         const int me = warp - 4, n_pg = LT_KEYS / p.page_size;
         const int* bt = p.block_table + (size_t)p.slots[b] * p.max_pages;
         const uint32_t page_bytes = (uint32_t)p.page_size * 128u;
@@ -247,6 +247,20 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
                     }
                     l_run *= corr;
                 }
+            }
+            if (k0 < lo || k0 + LT_KEYS > hi) {
+                // Rows of the tile that no row of the block sees hold what the pages hold there, behind a request's last token
+                // what an earlier owner of the page left: zeros take their place, for a weight of zero times what is not
+                // finite is not zero.  The boxes have landed (the scores are complete), and the next ones wait for O += P V.
+                lt_wait(tc_smem(&s_full[1]), i & 1, dead);
+                const int head = min(max(lo - k0, 0), LT_KEYS), tail = max(min(hi - k0, LT_KEYS), head);
+                const int n_dead = head + LT_KEYS - tail;
+                for (int c = tid; c < n_dead * nv * 8; c += LT_ROWS) {
+                    const int d = c / (nv * 8), key = d < head ? d : tail + d - head, piece = c % (nv * 8);
+                    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n"
+                                 ::"r"(sK + (v0 + piece / 8) * LT_K_BLK + key * 128 + piece % 8 * 16), "r"(0) : "memory");
+                }
+                tc_fence_async_smem();
             }
             tc_st32(t_row + 384 + 32 * (i & 1), reinterpret_cast<const float*>(w));
             l_run += ((rs[0] + rs[1]) + (rs[2] + rs[3])) + ((rs[4] + rs[5]) + (rs[6] + rs[7]));

@@ -8,15 +8,15 @@ pytestmark = pytest.mark.gpu
 
 
 def problem(runs, H, kr, rot, ps, seed, window=0, pad=0):
-    """runs: (start, tokens) per request.  Pages behind the window are taken out of the block table; rows past a request's
-    last token and spare pages hold large finite numbers."""
+    """runs: (start, tokens) per request.  Pages behind the window are taken out of the block table; spare pages and the rows
+    that no query sees (past a request's last token, behind the window) are not numbers."""
     gen = torch.Generator(device="cuda").manual_seed(seed)
     kd = kr + rot
     need = [-(-(s + n) // ps) for s, n in runs]
     order = list(range(sum(need) + 1))
     random.Random(seed).shuffle(order)
     table = torch.full((len(runs) + 1, max(need) + 1), -1, dtype=torch.int32)
-    pool = torch.full((len(order), 2, ps, kd), 300.0, dtype=torch.bfloat16, device="cuda")
+    pool = torch.full((len(order), 2, ps, kd), float("nan"), dtype=torch.bfloat16, device="cuda")
     rows, k = [], 0
     for i, (s, n) in enumerate(runs):
         r = torch.randn((s + n, kd), generator=gen, device="cuda").to(torch.bfloat16)
@@ -27,7 +27,8 @@ def problem(runs, H, kr, rot, ps, seed, window=0, pad=0):
             if not window or (j + 1) * ps > s - window + 1:
                 table[i + 1, j] = page
             part = r[j * ps:(j + 1) * ps]
-            pool[page, 1, :len(part)] = part
+            unseen = min(max(s - window + 1 - j * ps, 0), len(part)) if window else 0
+            pool[page, 1, unseen:len(part)] = part[unseen:]
     n_all = sum(n for _, n in runs)
     ints = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
     q_start = [0]

@@ -1098,7 +1098,7 @@ def latent_attention(q_lat: torch.Tensor, pool: torch.Tensor, layer: int, out: t
             # 256 value columns) fill half of the SMs.  16 heads, 512 + 64, us (mma.sync): 2 x 1000 tokens 183 (268), 300 tokens
             # (76 blocks) 41 (54), 450 tokens behind 1200 (114) 128 (192); 450 behind 1200 with 8 heads (58) 131 (119).
             n = q_lat.shape[0]
-            if (2 * int(lib().st_latent_attention_tc_blocks(n, nh, kr)) >= sm_count(q_lat.device)
+            if (out.data_ptr() % 16 == 0 and 2 * int(lib().st_latent_attention_tc_blocks(n, nh, kr)) >= sm_count(q_lat.device)
                     and int(lib().st_latent_attention_mma_splits(n, n_seqs, nh, window)) == 1):
                 kernel = "tc"
     if kernel == "plain":

@@ -112,3 +112,16 @@ def test_prompts_take_it_and_single_tokens_do_not(monkeypatch):
         auto, _ = run(q, pool, gates, sink, step, 16, 512, 64, 16, 0, "auto")
         want, _ = run(q, pool, gates, sink, step, 16, 512, 64, 16, 0, "tc" if tc else "mma")
         assert torch.equal(auto, want)
+
+
+def test_a_result_off_sixteen_bytes_is_still_taken():
+    from swifttransformer_b200 import ops
+    H, kr, rot, ps, n = 16, 512, 64, 16, 600
+    q, pool, gates, sink, _, step = problem([(0, n)], H, kr, rot, ps, 6)
+    outs = []
+    for kernel, skip in (("mma", 0), ("auto", 2)):
+        outs.append(torch.full((n * H * kr + skip,), 77.0, dtype=torch.bfloat16, device="cuda")[skip:].view(n, H * kr))
+        ops.latent_attention(q, pool, 1, outs[-1], step["positions"], step["seq"], step["slots"], step["table"], H, kr, rot, ps,
+                             (kr / 4 + rot) ** -0.5, sink, gates, kernel=kernel, q_start=step["q_start"], start_pos=step["start"],
+                             n_seqs=step["n_seqs"])
+    assert torch.equal(*outs)

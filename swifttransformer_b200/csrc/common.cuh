@@ -136,7 +136,11 @@ static inline int st_launch_status() { return (int)cudaGetLastError(); }
 // anything at all; what comes before the wait may only touch memory that no
 // kernel writes (weights).  After the wait every predecessor has finished and
 // its writes are visible.  ST_PDL_TRIGGER() lets the successor's blocks be
-// scheduled as soon as there is room.  In a kernel that is launched the plain
+// scheduled as soon as there is room.  A kernel that allocates tensor memory
+// triggers behind the allocation and a block-wide barrier: a successor's block
+// on the same multiprocessor may allocate before its own wait, and columns it
+// held while this grid still asked for some would be freed only when this grid
+// is done, which it then never is.  In a kernel that is launched the plain
 // way both are no-ops.  ST_B200_NO_PDL=1 in the environment turns the launch
 // attribute off.
 #include <stdlib.h>

@@ -133,7 +133,6 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
     ST_PDL_WAIT();
-    ST_PDL_TRIGGER();
     if (warp == 0) {
         int run = 0;
         for (int e0 = 0; e0 < sh.n_experts; e0 += 32) {
@@ -154,6 +153,7 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    ST_PDL_TRIGGER();
     const uint32_t tmem = s_tmem;
     const int bn_out = sh.gated ? BN / 2 : BN;
     const int n_tiles_n = (sh.n_out + bn_out - 1) / bn_out;

@@ -82,7 +82,6 @@ gemm_stream_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
         s_xempty[GS_MAX_X], s_accum;
     __shared__ uint32_t s_tmem;
     __shared__ int s_dead;
-    ST_PDL_TRIGGER();
     if (threadIdx.x == 0) GS_STAMP(0);
     constexpr int G = 256 / BM;                                              // blocks of 64 k per stage
     constexpr uint32_t W_TILE = BM * 128, W_BYTES = W_TILE * G;              // bytes of one weight stage
@@ -120,6 +119,7 @@ gemm_stream_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_co
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    ST_PDL_TRIGGER();
     const uint32_t tmem = s_tmem;
     if (threadIdx.x == 0) GS_STAMP(1);
 

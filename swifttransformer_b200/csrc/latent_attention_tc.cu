@@ -71,7 +71,6 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     volatile int* dead = &s_dead;
     ST_PDL_WAIT();
-    ST_PDL_TRIGGER();
     if (tid == 0) {
         // the last tiles of a request have the longest key ranges: first, all value columns of a tile side by side
         int tile = p.n_tiles - 1 - blockIdx.x / p.parts, req = -1;
@@ -103,6 +102,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
+    ST_PDL_TRIGGER();                                         // behind the allocation (blocks that have left count as well)
     const uint32_t tmem = s_tmem;                             // O at 0 (64 vb columns), S at 256 and 320, P at 384 and 416
     const int start = p.start_pos[b];
     const int last_row = min(r0 + LT_ROWS, n_rows) - 1;

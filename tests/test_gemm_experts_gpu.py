@@ -61,3 +61,23 @@ def test_a_row_does_not_depend_on_its_tile():
     whole = ops.gemm_experts(a, w, order_of([300], 1, gen)[0], gather=False)
     for n in (1, 32, 129):
         assert torch.equal(ops.gemm_experts(a[:n].contiguous(), w, order_of([n], 1, gen)[0], gather=False), whole[:n])
+
+
+def test_silu_of_every_number():
+    """Through an identity: all finite bfloat16 numbers, and rows of the tile that no expert has beside them."""
+    from swifttransformer_b200 import ops
+    a = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    a = a[torch.isfinite(a)].view(-1, 8).cuda()
+    order, _ = order_of([len(a)], 1, torch.Generator().manual_seed(0))
+    got = ops.gemm_experts(a, torch.eye(8, dtype=torch.bfloat16, device="cuda")[None].contiguous(), order, gather=False, act="silu")
+    x = a.float()
+    want = (x.double() / (1 + torch.exp(-x.double()))).to(torch.bfloat16)
+    # float arithmetic, then the rounding: at most the neighbouring bfloat16 number, or both below the normal numbers
+    step = torch.maximum(want.double().abs() * 2.0 ** -7, torch.tensor(2.0 ** -126, dtype=torch.float64, device="cuda"))
+    assert torch.all((got.double() - want.double()).abs() <= step)
+    for bad, result in ((float("inf"), float("inf")), (float("nan"), float("nan"))):
+        b = torch.zeros((3, 8), dtype=torch.bfloat16, device="cuda")
+        b[1] = bad
+        w = torch.ones((1, 8, 8), dtype=torch.bfloat16, device="cuda")
+        out = ops.gemm_experts(b, w, order_of([3], 1, torch.Generator().manual_seed(0))[0], gather=False, act="silu")
+        assert torch.all(out[::2] == 0) and torch.allclose(out[1].float(), torch.full((8,), result, device="cuda"), equal_nan=True)

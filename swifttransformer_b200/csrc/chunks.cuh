@@ -29,7 +29,7 @@ __device__ __forceinline__ void hk_cp16(float* dst, const float* src) {
 }
 
 // The outputs of a chunk before their norm: acc[r][j] += rows row0 + 4 r, values col + 32 j .. + 3 of X S + A V, by 256 threads
-// of 4 tokens x 8 values; X [HK_C][HK_LD], A [HK_C][HK_LA] (zero above its diagonal), V [HK_C][HK_LD] in shared memory, the
+// of 4 tokens x 8 values; X [HK_C][HK_LD], A [HK_C][HK_LA] (above its diagonal not read), V [HK_C][HK_LD] in shared memory, the
 // state's rows S [dim][vd] from memory 16 at a time through the two stages `ring`, the first two of which the caller has
 // asked for (hk_copy_rows) after anything else it copied.
 #define HK_SR 16
@@ -70,6 +70,31 @@ __device__ __forceinline__ void hk_sixteen(float4 (&acc)[4][2], const float* X, 
         for (int r = 0; r < 4; ++r) acc[r][j] = add4(acc[r][j], part[r]);
     }
 }
+// The same of the sixteen tokens that hold the rows themselves: row rl + 4 r adds the tokens up to itself and meets no later
+// one, whatever its values are (a weight of zero times a number that is not finite is not zero).
+__device__ __forceinline__ void hk_own_sixteen(float4 (&acc)[4][2], const float* A, const float* V, int rl) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+        float4 part[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) part[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float* y = V + 4 * i * HK_LD + 32 * j;
+            const float4 y0 = load4(y), y1 = load4(y + HK_LD), y2 = load4(y + 2 * HK_LD), y3 = load4(y + 3 * HK_LD);
+#pragma unroll
+            for (int r = i; r < 4; ++r) {
+                const float4 x = load4(A + 4 * r * HK_LA + 4 * i);
+                hk_fma4(x.x, y0, part[r]);
+                if (r > i || rl >= 1) hk_fma4(x.y, y1, part[r]);
+                if (r > i || rl >= 2) hk_fma4(x.z, y2, part[r]);
+                if (r > i || rl >= 3) hk_fma4(x.w, y3, part[r]);
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[r][j] = add4(acc[r][j], part[r]);
+    }
+}
 __device__ __forceinline__ void hk_outputs(float4 (&acc)[4][2], const float* X, const float* A, const float* V, float* ring,
                                            const float* S, int n, int dim, int vd, int row0, int col) {
     const int warp = threadIdx.x >> 5;
@@ -83,7 +108,9 @@ __device__ __forceinline__ void hk_outputs(float4 (&acc)[4][2], const float* X, 
         if (i0 + 2 * HK_SR < dim) hk_copy_rows(ring, S, i0 + 2 * HK_SR, dim, vd);
         else asm volatile("cp.async.commit_group;\n" ::);
     }
-    if (active)
-        for (int s = 0; s < ((warp >> 1) + 1) * 16; s += 16)
-            hk_sixteen(acc, A + row0 * HK_LA + s, HK_LA, V + s * HK_LD + col, 16);
+    if (active) {
+        const int s0 = (warp >> 1) * 16;                      // the sixteen tokens of the warp's own rows
+        for (int s = 0; s < s0; s += 16) hk_sixteen(acc, A + row0 * HK_LA + s, HK_LA, V + s * HK_LD + col, 16);
+        hk_own_sixteen(acc, A + row0 * HK_LA + s0, V + s0 * HK_LD + col, row0 - s0);
+    }
 }

@@ -135,3 +135,21 @@ def test_little_scratch_walks(monkeypatch):
                        st.q_start, st.slots, 1, H, G, d, dv)
         outs.append(out)
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("t0", [1, 15, 16, 31, 40, 63, 64, 100])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_broken_token_leaves_the_ones_before_it(t0, bad, monkeypatch):
+    """A value, a query, a key, a write strength or a decay that is not finite: the tokens before it, and the other heads, keep
+    their numbers."""
+    H, G, d, dv, rank, T = 2, 2, 64, 36, 0, 150
+    proj, w = inputs(T, H, G, d, dv, rank, t0, "slow")
+    C = 2 * G * d + H * dv
+    for col in (2 * G * d + 3, 5, G * d + 7, C, C + H):    # of head 0
+        outs = []
+        for x in (proj[t0, col], bad):
+            p = proj.copy()
+            p[t0, col] = x
+            state, tails = torch.zeros((2, H, d, dv), device="cuda"), torch.zeros((2, 1, C), device="cuda")
+            outs.append(step([p], [T], [0], H, G, d, dv, rank, w, tails, state, "float32", True, monkeypatch, [1])[0])
+        assert np.array_equal(outs[0][:t0], outs[1][:t0]) and np.array_equal(outs[0][:, dv:], outs[1][:, dv:])

@@ -88,3 +88,19 @@ def test_little_scratch_walks(monkeypatch):
                        st.q_start, st.slots, 1, H, d, dv, scratch=torch.zeros(T * H * dv, device="cuda"))
         outs.append(out)
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("t0", [1, 15, 16, 31, 40, 63, 64, 100])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_a_broken_token_leaves_the_ones_before_it(t0, bad, monkeypatch):
+    """A value, a query or a gate that is not finite: the tokens before it, and the other heads, keep their numbers."""
+    H, d, dv, T = 2, 64, 36, 150
+    p, f_bias, lower, norm_w = projections(T, H, d, dv, t0, "slow")
+    for col in (2 * H * d + 3, 5, H * d + 7):            # of head 0: a value, a query, a gate
+        outs = []
+        for x in (p[t0, col], bad):
+            q = p.copy()
+            q[t0, col] = x
+            state = torch.zeros((2, H, d, dv), device="cuda")
+            outs.append(scan([q], [T], [0], H, d, dv, f_bias, lower, norm_w, state, "float32", True, monkeypatch, [1])[0])
+        assert np.array_equal(outs[0][:t0], outs[1][:t0]) and np.array_equal(outs[0][:, dv:], outs[1][:, dv:])

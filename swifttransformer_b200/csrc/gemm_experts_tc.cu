@@ -321,10 +321,11 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
 // gate and up rows: 65 / 55 / 76; 300 items on 16 experts, 1024: 37 / 31 / 39; 16 items on 8, 2048: 16.4 / 14.4 / 16.4), else 64
 // (16 items on 8, 1024: 31 / 27 / 35, where the widths are as far apart as two runs of one are).
 static int ge_pick_bn(int n_items, int n_experts, int w_rows, int sms) {
+    const double hit = n_experts * (1. - exp(-(double)n_items / n_experts));      // experts that get an item, if they get them evenly
     int row_tiles = (n_items + GE_BM - 1) / GE_BM;
-    if (row_tiles < n_experts) row_tiles = n_items < n_experts ? n_items : n_experts;
+    if (row_tiles < hit) row_tiles = (int)hit;
     auto tiles = [&](int bn) { return (long long)row_tiles * ((w_rows + bn - 1) / bn); };
-    return tiles(256) >= sms ? 256 : 2 * tiles(128) >= sms ? 128 : 64;
+    return tiles(256) >= sms ? 256 : 5 * tiles(128) >= 3 * sms ? 128 : 64;
 }
 
 template <int BN, bool GATHER>

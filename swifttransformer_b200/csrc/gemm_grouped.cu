@@ -10,11 +10,12 @@
 //     given (the sorted (token, choice) items, a_row_div choices per token), else the row itself.
 // Epilogue: c = act(product), or "gated": w[g] holds 2 * n_out rows, gate rows first, and c = act(gate) * up.
 //
-// gemm_grouped_mma: the first way in bfloat16 on the warp-level tensor cores (mma.sync m16n8k16, float accumulation): tiles of
-// 64 rows x 64 outputs x 64 of k, four warps of 32 x 32 each, rows and weights streamed by 16-byte asynchronous copies in
-// three stages (two tiles of k under way per block: steps of few tokens are bound by the weights' way from memory, and what
-// a block has in flight decides the rate); k, the row strides and the group offsets must be multiples of 8 elements.  The
-// experts' products in bfloat16 are gemm_experts_tc.cu's.
+// gemm_grouped_mma: bfloat16 on the warp-level tensor cores (mma.sync m16n8k16, float accumulation): tiles of 64 rows
+// x 64 outputs x 64 of k, four warps of 32 x 32 each, rows gathered and weights streamed by 16-byte asynchronous
+// copies in three stages (two tiles of k under way per block: steps of few tokens are bound by the weights' way from
+// memory, and what a block has in flight decides the rate); k, the row strides and the group offsets must be multiples of 8 elements.
+// The experts' products in bfloat16 are gemm_experts_tc.cu's but for small matrices with few rows, where that kernel's way
+// into tensor memory and back costs more than it saves.
 // gemm_grouped_plain: float arithmetic for either storage type; every output element is one chain of fused
 // multiply-adds over k in ascending order whatever rows share its tile (the 32-bit path, and the plain twin).
 #include "common.cuh"
@@ -151,16 +152,35 @@ ST_EXPORT int st_gemm_grouped_plain(const void* a, const void* w, void* c, int n
 #define GM_LD (GM_BK + 8)
 #define GM_STAGES 3
 
-template <typename TO, int BN>
+template <typename TO, bool GATED, int BN>
 __global__ void __launch_bounds__(128)
 gemm_grouped_mma_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, TO* __restrict__ c, GroupedShape sh) {
     extern __shared__ __align__(16) unsigned char gm_smem[];
+    constexpr int WROWS = GATED ? 2 * BN : BN;
     bf16 (*sa)[GG_BM][GM_LD] = reinterpret_cast<bf16 (*)[GG_BM][GM_LD]>(gm_smem);
-    bf16 (*sw)[BN][GM_LD] = reinterpret_cast<bf16 (*)[BN][GM_LD]>(gm_smem + sizeof(bf16) * GM_STAGES * GG_BM * GM_LD);
+    bf16 (*sw)[WROWS][GM_LD] = reinterpret_cast<bf16 (*)[WROWS][GM_LD]>(gm_smem + sizeof(bf16) * GM_STAGES * GG_BM * GM_LD);
+    __shared__ int srow[GG_BM];
     ST_PDL_WAIT();
     ST_PDL_TRIGGER();
-    const int g = blockIdx.z, row0 = blockIdx.y * GG_BM, row_end = min(row0 + GG_BM, sh.n_rows);
+    int g, row0, row_end;
+    if (sh.offsets) {
+        g = __ldcg(sh.tile_group + blockIdx.y);
+        if (g < 0) return;
+        row0 = __ldcg(sh.tile_row0 + blockIdx.y);
+        row_end = min(row0 + GG_BM, __ldcg(sh.offsets + g + 1));
+    } else {
+        g = blockIdx.z;
+        row0 = blockIdx.y * GG_BM;
+        row_end = min(row0 + GG_BM, sh.n_rows);
+    }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid < GG_BM) {
+        const int r = row0 + tid;
+        int ar = -1;
+        if (r < row_end) ar = sh.a_rows ? __ldcg(sh.a_rows + r) / sh.a_row_div : r;
+        srow[tid] = ar;
+    }
+    __syncthreads();
     const int col0 = blockIdx.x * BN;
     const bf16* wg = w + (long long)g * sh.w_gstride;
     const bf16* ag = a + g * sh.a_goff;
@@ -168,23 +188,28 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, 
         // 64 rows x 8 chunks of 8 per operand
         for (int ch = tid; ch < GG_BM * 8; ch += 128) {
             const int r = ch >> 3, kc = (ch & 7) * 8;
-            const bool ok = row0 + r < row_end && k0 + kc < sh.k_dim;
-            cp_async16(&sa[stage][r][kc], ok ? ag + (long long)(row0 + r) * sh.lda + k0 + kc : a, ok);
+            const int ar = srow[r];
+            const bool ok = ar >= 0 && k0 + kc < sh.k_dim;
+            cp_async16(&sa[stage][r][kc], ok ? ag + (long long)ar * sh.lda + k0 + kc : a, ok);
         }
-        for (int ch = tid; ch < BN * 8; ch += 128) {
+        for (int ch = tid; ch < BN * 8 * (GATED ? 2 : 1); ch += 128) {
             const int r = ch >> 3, kc = (ch & 7) * 8;
-            const bool ok = col0 + r < sh.n_out && k0 + kc < sh.k_dim;
-            cp_async16(&sw[stage][r][kc], ok ? wg + (long long)(col0 + r) * sh.k_dim + k0 + kc : w, ok);
+            const int n = col0 + (r & (BN - 1)) + (r >= BN ? sh.n_out : 0);
+            const bool ok = col0 + (r & (BN - 1)) < sh.n_out && k0 + kc < sh.k_dim;
+            cp_async16(&sw[stage][r][kc], ok ? wg + (long long)n * sh.k_dim + k0 + kc : w, ok);
         }
     };
     constexpr int NJ = BN / 16;          // 8-wide output tiles of a warp (its half of the block's columns)
-    float acc[2][NJ][4];
+    float acc[2][NJ][4], acu[GATED ? 2 : 1][NJ][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
         for (int j = 0; j < NJ; ++j)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+            for (int e = 0; e < 4; ++e) {
+                acc[i][j][e] = 0.f;
+                if (GATED) acu[i][j][e] = 0.f;
+            }
     const int wm = (warp & 1) * 32, wn = (warp >> 1) * (BN / 2);
     const int a_row = (lane & 7) + ((lane >> 3) & 1) * 8, a_col = (lane >> 4) * 8;
     const int b_row = (lane & 7) + (lane >> 4) * 8, b_col = ((lane >> 3) & 1) * 8;
@@ -217,6 +242,14 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, 
                     mma_bf16(acc[i][2 * jp], af[i], b0, b1);
                     mma_bf16(acc[i][2 * jp + 1], af[i], b2, b3);
                 }
+                if (GATED) {
+                    ldmatrix_x4(b0, b1, b2, b3, &sw[stage][BN + wn + jp * 16 + b_row][kk + b_col]);
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        mma_bf16(acu[i][2 * jp], af[i], b0, b1);
+                        mma_bf16(acu[i][2 * jp + 1], af[i], b2, b3);
+                    }
+                }
             }
         }
     }
@@ -231,7 +264,8 @@ gemm_grouped_mma_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, 
                 const int n = col0 + wn + j * 8 + 2 * tq + (e & 1);
                 if (r >= row_end || n >= sh.n_out) continue;
                 float v = acc[i][j][e];
-                if (sh.act) v = apply_act(v, sh.act);
+                if (GATED) v = apply_act(to_f32(from_f32<bf16>(v)), sh.act) * to_f32(from_f32<bf16>(acu[i][j][e]));
+                else if (sh.act) v = apply_act(v, sh.act);
                 c[(long long)r * sh.ldc + g * sh.c_goff + n] = from_f32<TO>(v);
             }
 }
@@ -241,35 +275,42 @@ ST_EXPORT int st_gemm_grouped_mma_applies(int k_dim, long long lda, long long a_
 }
 
 ST_EXPORT int st_gemm_grouped_mma(const void* a, const void* w, void* c, int n_groups, int n_rows, int n_out, int k_dim,
-                                  long long lda, long long a_goff, long long ldc, long long c_goff, long long w_gstride,
-                                  int out_f32, void* stream) {
-    if (n_groups <= 0 || n_out <= 0 || n_rows <= 0) return 0;
+                                  int gated, int act, long long lda, long long a_goff, long long ldc, long long c_goff,
+                                  long long w_gstride, const int* offsets, const int* tile_group, const int* tile_row0,
+                                  int n_tiles, const int* a_rows, int a_row_div, int out_f32, void* stream) {
+    if (n_groups <= 0 || n_out <= 0) return 0;
+    if ((offsets && (!tile_group || !tile_row0 || n_tiles <= 0)) || (a_rows && a_row_div <= 0)) return ST_ERR_BAD_ARG;
+    if (!offsets && n_rows <= 0) return 0;
     if (!st_gemm_grouped_mma_applies(k_dim, lda, a_goff, w_gstride) || !aligned16(a) || !aligned16(w)) return ST_ERR_BAD_SIZE;
-    GroupedShape sh{n_rows, n_out, k_dim, 0, 0, lda, a_goff, ldc, c_goff, w_gstride, nullptr, nullptr, nullptr, nullptr, 1};
-    dim3 grid((n_out + GG_BN - 1) / GG_BN, (n_rows + GG_BM - 1) / GG_BM, n_groups);
+    GroupedShape sh{n_rows, n_out, k_dim, gated, act, lda, a_goff, ldc, c_goff, w_gstride, offsets, tile_group, tile_row0,
+                    a_rows, a_row_div};
+    dim3 grid((n_out + GG_BN - 1) / GG_BN, offsets ? n_tiles : (n_rows + GG_BM - 1) / GG_BM, offsets ? 1 : n_groups);
     if (grid.y > 65535 || grid.z > 65535) return ST_ERR_TOO_LARGE;
     // launches of few blocks (steps of few tokens, bound by the weights' way from memory) take tiles of 32 outputs:
     // twice the blocks, so that every SM pulls weights
     const bool narrow = (long long)grid.x * grid.y * grid.z < 2LL * st_sm_count();
     if (narrow) grid.x = (n_out + 31) / 32;
     cudaStream_t s = (cudaStream_t)stream;
-    auto smem_of = [](int bn) { return sizeof(bf16) * GM_STAGES * (GG_BM + bn) * GM_LD; };
+    auto smem_of = [](int bn, bool g) { return sizeof(bf16) * GM_STAGES * (GG_BM + (g ? 2 : 1) * bn) * GM_LD; };
     static bool set = false;
     if (!set) {
-#define GM_SET(TO, BN) cudaFuncSetAttribute(gemm_grouped_mma_kernel<TO, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(BN))
-        GM_SET(float, 64); GM_SET(bf16, 64); GM_SET(float, 32); GM_SET(bf16, 32);
+#define GM_SET(TO, G, BN) cudaFuncSetAttribute(gemm_grouped_mma_kernel<TO, G, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_of(BN, G))
+        GM_SET(float, true, 64); GM_SET(bf16, true, 64); GM_SET(float, false, 64); GM_SET(bf16, false, 64);
+        GM_SET(float, true, 32); GM_SET(bf16, true, 32); GM_SET(float, false, 32); GM_SET(bf16, false, 32);
 #undef GM_SET
         set = true;
     }
-#define GM_LAUNCH(TO, BN)                                                                                              \
-    return st_launch_pdl("gemm_grouped", gemm_grouped_mma_kernel<TO, BN>, grid, dim3(128), smem_of(BN), s, (const bf16*)a, \
-                         (const bf16*)w, (TO*)c, sh)
+#define GM_LAUNCH(TO, G, BN)                                                                                          \
+    return st_launch_pdl("gemm_grouped", gemm_grouped_mma_kernel<TO, G, BN>, grid, dim3(128), smem_of(BN, G), s,      \
+                         (const bf16*)a, (const bf16*)w, (TO*)c, sh)
     if (narrow) {
-        if (out_f32) GM_LAUNCH(float, 32);
-        GM_LAUNCH(bf16, 32);
+        if (gated) { if (out_f32) GM_LAUNCH(float, true, 32); GM_LAUNCH(bf16, true, 32); }
+        if (out_f32) GM_LAUNCH(float, false, 32);
+        GM_LAUNCH(bf16, false, 32);
     }
-    if (out_f32) GM_LAUNCH(float, 64);
-    GM_LAUNCH(bf16, 64);
+    if (gated) { if (out_f32) GM_LAUNCH(float, true, 64); GM_LAUNCH(bf16, true, 64); }
+    if (out_f32) GM_LAUNCH(float, false, 64);
+    GM_LAUNCH(bf16, false, 64);
 #undef GM_LAUNCH
 }
 

@@ -1154,13 +1154,12 @@ def gemm_heads(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, n_groups: in
     assert a.dim() == 2 and out.dim() == 2 and a.shape[0] == out.shape[0] and a.stride(1) == 1 and out.stride(1) == 1
     assert w.is_contiguous() and w.shape == (n_groups, n_out, k_dim) and a.dtype == w.dtype
     ll = ctypes.c_longlong
-    strides = (ll(a.stride(0)), ll(a_goff), ll(out.stride(0)), ll(c_goff), ll(n_out * k_dim))
-    sizes = (_p(a), _p(w), _p(out), n_groups, a.shape[0], n_out, k_dim)
+    args = (_p(a), _p(w), _p(out), n_groups, a.shape[0], n_out, k_dim, 0, 0, ll(a.stride(0)), ll(a_goff), ll(out.stride(0)),
+            ll(c_goff), ll(n_out * k_dim), None, None, None, 0, None, 1)
     if _grouped_mma(a, k_dim, a.stride(0), a_goff, n_out * k_dim):
-        _check(lib().st_gemm_grouped_mma(*sizes, *strides, int(out.dtype == torch.float32), _stream()), "gemm_heads")
+        _check(lib().st_gemm_grouped_mma(*args, int(out.dtype == torch.float32), _stream()), "gemm_heads")
     else:
-        _check(lib().st_gemm_grouped_plain(*sizes, 0, 0, *strides, None, None, None, 0, None, 1, _dt(a),
-                                           int(out.dtype == torch.float32), _stream()), "gemm_heads")
+        _check(lib().st_gemm_grouped_plain(*args, _dt(a), int(out.dtype == torch.float32), _stream()), "gemm_heads")
     return out
 
 
@@ -1169,6 +1168,14 @@ GROUPED_MMA = True
 
 
 EXPERTS_TILE = 0         # rows of an expert's matrix per tile of the tcgen05 kernel: 64, 128, 256; 0: the launcher's choice
+
+
+def _experts_mma(n_items: int, n_experts: int, w_rows: int, k: int) -> bool:
+    """Whether an experts' product is small enough for the mma.sync kernel: matrices of at most 65536 numbers with fewer than 64
+    items per expert.  us (tcgen05): 8 experts, gated 64 -> 64, 38 items 10.2 (11.3); 64 experts, gated 256 -> 128, 152 items 12.3
+    (16.4); 128 experts, 128 -> 256, 1024 items 12.3 (16.4).  Beyond: 8 experts, gated 256 -> 128, 600 items 15.2 (12.3); 16
+    experts, gated 512 -> 512, 152 items 17.4 (18.4), 1200 items 24.6 (18.4); 76 items, gated 1024 -> 512 25.7 (21.5)."""
+    return EXPERTS_TILE == 0 and w_rows * k <= 65536 and n_items < 64 * n_experts
 
 
 def _grouped_mma(a: torch.Tensor, k_dim: int, lda: int, a_goff: int, w_gstride: int) -> bool:
@@ -1257,23 +1264,26 @@ def gemm_experts(a: torch.Tensor, w: torch.Tensor, order: ExpertOrder, gather: b
     """One product per expert over the rows the order gives it: out [items, n_out] in sorted order.
     ``gather``: the rows of ``a`` are the tokens (row of item i = i // top), else ``a`` is already in sorted order.
     w [experts, n_out (twice with ``gated``: gate rows, then up rows), k]; out = act(product), gated: act(gate) * up.
-    bfloat16 with k a multiple of 8: the tcgen05 kernel (a wait that expires inside it shows in ``kernel_status``); else
-    the plain one."""
+    bfloat16 with k a multiple of 8: the tcgen05 kernel (a wait that expires inside it shows in ``kernel_status``), for small
+    products the mma.sync one; else the plain one."""
     assert a.is_contiguous() and w.is_contiguous() and w.dim() == 3 and a.dtype == w.dtype and a.shape[1] == w.shape[2]
     n_out = w.shape[1] // 2 if gated else w.shape[1]
     out = a.new_empty((order.n_items, n_out))
     ll = ctypes.c_longlong
-    if GROUPED_MMA and a.dtype == torch.bfloat16 and bool(lib().st_gemm_experts_tc_applies(w.shape[0], w.shape[2])):
-        _check(lib().st_gemm_experts_tc(_p(a), ll(a.shape[0]), _p(w), _p(out), w.shape[0], order.n_items, n_out, w.shape[2],
-                                        int(gated), ACT_CODES[act], _p(order.offsets), _p(order.sorted) if gather else None,
-                                        order.top if gather else 1, EXPERTS_TILE, _p(_tc_status_word(a.device)), _stream()),
-               "gemm_experts")
+    E, w_rows, k = w.shape
+    if (not _experts_mma(order.n_items, E, w_rows, k) and GROUPED_MMA and a.dtype == torch.bfloat16
+            and bool(lib().st_gemm_experts_tc_applies(E, k))):
+        _check(lib().st_gemm_experts_tc(_p(a), ll(a.shape[0]), _p(w), _p(out), E, order.n_items, n_out, k, int(gated), ACT_CODES[act],
+                                        _p(order.offsets), _p(order.sorted) if gather else None, order.top if gather else 1,
+                                        EXPERTS_TILE, _p(_tc_status_word(a.device)), _stream()), "gemm_experts")
         return out
-    _check(lib().st_gemm_grouped_plain(_p(a), _p(w), _p(out), w.shape[0], order.n_items, n_out, w.shape[2], int(gated),
-                                       ACT_CODES[act], ll(a.stride(0)), ll(0), ll(n_out), ll(0),
-                                       ll(w.shape[1] * w.shape[2]), _p(order.offsets), _p(order.tile_group),
-                                       _p(order.tile_row0), order.tile_group.numel(), _p(order.sorted) if gather else None,
-                                       order.top if gather else 1, _dt(a), 0, _stream()), "gemm_experts")
+    args = (_p(a), _p(w), _p(out), E, order.n_items, n_out, k, int(gated), ACT_CODES[act], ll(a.stride(0)), ll(0), ll(n_out), ll(0),
+            ll(w_rows * k), _p(order.offsets), _p(order.tile_group), _p(order.tile_row0), order.tile_group.numel(),
+            _p(order.sorted) if gather else None, order.top if gather else 1)
+    if _grouped_mma(a, k, a.stride(0), 0, w_rows * k):
+        _check(lib().st_gemm_grouped_mma(*args, 0, _stream()), "gemm_experts")
+    else:
+        _check(lib().st_gemm_grouped_plain(*args, _dt(a), 0, _stream()), "gemm_experts")
     return out
 
 

@@ -63,9 +63,10 @@ def test_a_row_does_not_depend_on_its_tile():
         assert torch.equal(ops.gemm_experts(a[:n].contiguous(), w, order_of([n], 1, gen)[0], gather=False), whole[:n])
 
 
-def test_silu_of_every_number():
+def test_silu_of_every_number(monkeypatch):
     """Through an identity: all finite bfloat16 numbers, and rows of the tile that no expert has beside them."""
     from swifttransformer_b200 import ops
+    monkeypatch.setattr(ops, "EXPERTS_TILE", 64)
     a = torch.arange(1 << 16, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
     a = a[torch.isfinite(a)].view(-1, 8).cuda()
     order, _ = order_of([len(a)], 1, torch.Generator().manual_seed(0))
@@ -82,3 +83,8 @@ def test_silu_of_every_number():
         w = torch.ones((1, 8, 8), dtype=torch.bfloat16, device="cuda")
         out = ops.gemm_experts(b, w, order_of([3], 1, torch.Generator().manual_seed(0))[0], gather=False, act="silu")
         assert torch.all(out[::2] == 0) and torch.allclose(out[1].float(), torch.full((8,), result, device="cuda"), equal_nan=True)
+
+
+def test_small_products_take_the_other_kernel():
+    from swifttransformer_b200 import ops
+    assert ops._experts_mma(8, 8, 256, 256) and not ops._experts_mma(8, 8, 264, 256) and not ops._experts_mma(512, 8, 256, 256)

@@ -8,20 +8,27 @@
 #define HK_LD (HK_D + 4)
 #define HK_LA (HK_C + 4)
 
-// A request's chunks have the places q_start / 64 + (its index) + 0, 1, ..: no two requests' overlap, and n / 64 + n_seqs hold
-// all.  Returns false when no chunk stands at `place`.
-__device__ __forceinline__ bool hk_find(const int* q_start, const int* positions, int n_seqs, int place, int& b, int& first, int& n) {
+// Requests with portions of at least `from` tokens run in chunks, the others walk: each by its own length, whoever shares the
+// step.  A request's chunks have the places hk_place + 0, 1, ..: no two requests' overlap (a portion of `from` tokens and more
+// moves both terms on), and hk_places hold all L = min(n_seqs, n / from) of them.
+__host__ __device__ __forceinline__ int hk_place(int begin, int b, int from) {
+    return begin / HK_C + (b < begin / from ? b : begin / from);
+}
+static inline long long hk_places(int n_tokens, int L) { return ((long long)n_tokens + HK_C - 1) / HK_C + L - 1; }
+static inline int hk_longs(int n_tokens, int n_seqs, int from) { return n_seqs < n_tokens / from ? n_seqs : n_tokens / from; }
+// The chunk at `place`: false when none stands there.
+__device__ __forceinline__ bool hk_find(const int* q_start, const int* positions, int n_seqs, int from, int place, int& b, int& first, int& n) {
     int lo = 0, hi = n_seqs;                              // the last request whose places begin at or before this one
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (q_start[mid] / HK_C + mid <= place) lo = mid; else hi = mid;
+        if (hk_place(q_start[mid], mid, from) <= place) lo = mid; else hi = mid;
     }
     b = lo;
     const int begin = q_start[b], end = q_start[b + 1];
-    const int chunk = place - (begin / HK_C + b);
+    const int chunk = place - hk_place(begin, b, from);
     first = begin + chunk * HK_C;
     n = min(HK_C, end - first);
-    return chunk >= 0 && n > 0 && positions[begin] >= 0;      // (padding stands at position -1)
+    return chunk >= 0 && n > 0 && end - begin >= from && positions[begin] >= 0;      // (padding stands at position -1)
 }
 
 __device__ __forceinline__ void hk_cp16(float* dst, const float* src) {

@@ -39,14 +39,14 @@ struct DcPrepareSmem {
 // AM holds q_t^T D(s, t) k_s at [t][s], s <= t, and k_t^T D(s, t) k_s at [s][t], s < t.
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_prepare_kernel(const float* __restrict__ prep, const DeltaShape sh, const ChunkScratch cs,
-                           const int* __restrict__ positions, const int* __restrict__ q_start, int n_seqs) {
+                           const int* __restrict__ positions, const int* __restrict__ q_start, int n_seqs, int from) {
     extern __shared__ __align__(16) unsigned char dc_raw[];
     DcPrepareSmem& m = *reinterpret_cast<DcPrepareSmem*>(dc_raw);
     ST_PDL_WAIT();
     const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dim = sh.dim, vd = sh.vd, g = h / (sh.H / sh.G);
     int b, first, n;
-    if (!hk_find(q_start, positions, n_seqs, place, b, first, n)) return;
+    if (!hk_find(q_start, positions, n_seqs, from, place, b, first, n)) return;
     const size_t unit = (size_t)place * sh.H + h;
     const float* rows = prep + (size_t)first * sh.stride;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f), one = make_float4(1.f, 1.f, 1.f, 1.f);
@@ -256,7 +256,7 @@ struct DcWalkSmem {
 template <int NC>
 __global__ void __launch_bounds__(256, 1)
 delta_chunk_walk_kernel(const DeltaShape sh, const ChunkScratch cs, float* __restrict__ state, int write_state,
-                        const int* __restrict__ positions, const int* __restrict__ q_start, const int* __restrict__ slots) {
+                        const int* __restrict__ positions, const int* __restrict__ q_start, const int* __restrict__ slots, int from) {
     using M = DcWalkSmem<NC>;
     constexpr int VS = M::VS;
     extern __shared__ __align__(16) unsigned char dc_raw[];
@@ -264,9 +264,9 @@ delta_chunk_walk_kernel(const DeltaShape sh, const ChunkScratch cs, float* __res
     ST_PDL_WAIT();
     const int b = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * VS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int begin = q_start[b], n = q_start[b + 1] - begin, dim = sh.dim, vd = sh.vd;
-    if (n <= 0 || positions[begin] < 0) return;
+    if (n < from || positions[begin] < 0) return;
     const int chunks = (n + HK_C - 1) / HK_C;
-    const size_t unit0 = (size_t)(begin / HK_C + b) * sh.H + h;      // and one place, sh.H units, further per chunk
+    const size_t unit0 = (size_t)hk_place(begin, b, from) * sh.H + h;      // and one place, sh.H units, further per chunk
     auto copy = [&](int c) {
         const float* W = cs.W + (unit0 + (size_t)c * sh.H) * HK_C * dim;
         const float* K = cs.K + (unit0 + (size_t)c * sh.H) * HK_C * dim;
@@ -402,14 +402,14 @@ struct DcOutSmem {
 
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_out_kernel(const DeltaShape sh, const ChunkScratch cs, float* __restrict__ o, const int* __restrict__ positions,
-                       const int* __restrict__ q_start, int n_seqs) {
+                       const int* __restrict__ q_start, int n_seqs, int from) {
     extern __shared__ __align__(16) unsigned char dc_raw[];
     DcOutSmem& m = *reinterpret_cast<DcOutSmem*>(dc_raw);
     ST_PDL_WAIT();
     const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dim = sh.dim, vd = sh.vd;
     int b, first, n;
-    if (!hk_find(q_start, positions, n_seqs, place, b, first, n)) return;
+    if (!hk_find(q_start, positions, n_seqs, from, place, b, first, n)) return;
     const size_t unit = (size_t)place * sh.H + h;
     for (int i = tid; i < HK_C * (HK_D / 4); i += 256) {
         const int t = i / (HK_D / 4), e = (i % (HK_D / 4)) * 4;
@@ -441,15 +441,16 @@ delta_chunk_out_kernel(const DeltaShape sh, const ChunkScratch cs, float* __rest
 
 long long delta_chunks_floats(int n_tokens, int n_seqs, const DeltaShape& sh) {
     if (sh.dim % 4 || sh.vd % 4 || sh.dim > HK_D || sh.vd > HK_D || sh.H > 65535 || n_seqs > 65535) return 0;
-    return ((long long)n_tokens / HK_C + n_seqs) * sh.H *
+    return hk_places(n_tokens, n_seqs) * sh.H *
            ((long long)HK_C * (3 * sh.dim + sh.vd) + HK_C * HK_C + sh.dim + (long long)sh.dim * sh.vd);
 }
 
 int delta_chunks_launch(const float* prep, const DeltaShape& sh, float* scratch, float* state, int write_state, float* o,
-                        const int* positions, const int* q_start, const int* slots, int n_tokens, int n_seqs, cudaStream_t s) {
-    const long long places = n_tokens / HK_C + n_seqs, units = places * sh.H;
+                        const int* positions, const int* q_start, const int* slots, int n_tokens, int n_seqs, int from, cudaStream_t s) {
+    // (as delta_chunks_floats counts for min(n_seqs, n_tokens / from) requests)
+    const long long places = hk_places(n_tokens, hk_longs(n_tokens, n_seqs, from)), units = places * sh.H;
     ChunkScratch cs;
-    float* at = scratch;                                   // as delta_chunks_floats counts
+    float* at = scratch;
     auto take = [&](long long per_unit) { float* p = at; at += units * per_unit; return p; };
     cs.W = take((long long)HK_C * sh.dim);
     cs.U = take((long long)HK_C * sh.vd);
@@ -464,15 +465,15 @@ int delta_chunks_launch(const float* prep, const DeltaShape& sh, float* scratch,
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DcOutSmem));
     if (e != cudaSuccess) return (int)e;
     int rc = st_launch_pdl("delta_chunks", delta_chunk_prepare_kernel, dim3((unsigned)places, sh.H), dim3(256), sizeof(DcPrepareSmem), s,
-                           prep, sh, cs, positions, q_start, n_seqs);
+                           prep, sh, cs, positions, q_start, n_seqs, from);
     if (rc) return rc;
     if ((long long)n_seqs * sh.H * ((sh.vd + 7) / 8) <= st_sm_count())
         rc = st_launch_pdl("delta_chunks", delta_chunk_walk_kernel<2>, dim3((sh.vd + 7) / 8, sh.H, n_seqs), dim3(256),
-                           sizeof(DcWalkSmem<2>), s, sh, cs, state, write_state, positions, q_start, slots);
+                           sizeof(DcWalkSmem<2>), s, sh, cs, state, write_state, positions, q_start, slots, from);
     else
         rc = st_launch_pdl("delta_chunks", delta_chunk_walk_kernel<4>, dim3((sh.vd + 15) / 16, sh.H, n_seqs), dim3(256),
-                           sizeof(DcWalkSmem<4>), s, sh, cs, state, write_state, positions, q_start, slots);
+                           sizeof(DcWalkSmem<4>), s, sh, cs, state, write_state, positions, q_start, slots, from);
     if (rc) return rc;
     return st_launch_pdl("delta_chunks", delta_chunk_out_kernel, dim3((unsigned)places, sh.H), dim3(256), sizeof(DcOutSmem), s, sh, cs, o,
-                         positions, q_start, n_seqs);
+                         positions, q_start, n_seqs, from);
 }

@@ -192,13 +192,13 @@ template <int L, int R>
 __global__ void __launch_bounds__(DS_THREADS)
 delta_scan_kernel(const float* __restrict__ prep, DeltaShape sh, float* __restrict__ state, int write_state,
                   float* __restrict__ o_out, const int* __restrict__ positions, const int* __restrict__ q_start,
-                  const int* __restrict__ slots) {
+                  const int* __restrict__ slots, int below) {
     using M = DeltaScanSmem<L, R>;
     extern __shared__ __align__(16) float ds_smem[];
     ST_PDL_WAIT();
     const int b = blockIdx.x, h = blockIdx.y;
     const int first = q_start[b], n = q_start[b + 1] - first;
-    if (n <= 0 || positions[first] < 0) return;            // padding of a fixed-shape step
+    if (n <= 0 || n >= below || positions[first] < 0) return;      // padding of a fixed-shape step; longer ones run in chunks
     const int H = sh.H, dim = sh.dim, vd = sh.vd;
     const int g = h / (H / sh.G);
     const int sub = threadIdx.x % L;
@@ -368,7 +368,7 @@ ST_EXPORT int st_delta_rule_set_lanes(int lanes) {
     ds_forced_lanes = lanes;
     return 0;
 }
-// Floats of scratch with which a step of n_tokens tokens of n_seqs requests runs in chunks (0: it does not).
+// Floats of scratch with which n_seqs requests of a step of n_tokens tokens run in chunks (0: they do not).
 ST_EXPORT long long st_delta_rule_chunk_floats(int n_tokens, int n_seqs, int H, int G, int dim, int vd) {
     if (n_tokens <= 0 || n_seqs <= 0 || H <= 0 || G <= 0 || H % G || dim <= 0 || vd <= 0 || ds_forced_lanes) return 0;
     DeltaShape sh = {};
@@ -383,14 +383,16 @@ ST_EXPORT long long st_delta_rule_scratch_floats(int n_tokens, int H, int G, int
 
 // proj: float [n_tokens, ld]; w_a2 [H*dim, rank_a], w_g2 [H*vd, rank_g] in the storage type `dtype`, as is out
 // [n_tokens, H*vd]; conv_state float [slots, taps-1, 2*G*dim + H*vd]; state float [slots, H, dim, vd];
-// scratch: float, st_delta_rule_scratch_floats elements, with `chunks` 16-byte aligned and st_delta_rule_chunk_floats.  write_state == 0: the states are read, not moved on.
+// scratch: float, st_delta_rule_scratch_floats elements.  write_state == 0: the states are read, not moved on.  from > 0: requests
+// of at least so many tokens run in chunks (scratch: 16-byte aligned, st_delta_rule_chunk_floats elements for min(n_seqs,
+// n_tokens / from) requests); walk == 0: there are no others.
 ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int a_off, int g_off, int rank_a,
                             int rank_g, const float* conv_w, int taps, float* conv_state, const void* w_a2,
                             const float* a_log, const float* dt_bias, const void* w_g2, const float* norm_w, float eps,
                             float out_scale, float* state, int write_state, int single_tokens, float* scratch,
                             void* out, const int* positions, const int* seq_of_token, const int* q_start,
                             const int* slots, int n_tokens, int n_seqs, int H, int G, int dim, int vd, int dtype,
-                            void* stream, int gate_silu, int chunks) {
+                            void* stream, int gate_silu, int from, int walk) {
     if (n_tokens <= 0 || n_seqs <= 0) return 0;
     if (H <= 0 || G <= 0 || H % G || dim <= 0 || vd <= 0 || taps < 1 || rank_a < 0 || rank_g < 0) return ST_ERR_BAD_ARG;
     if (taps > DR_MAX_TAPS || dim > 32 * DR_UNIT_PASSES || vd > 32 * DR_UNIT_PASSES) return ST_ERR_TOO_LARGE;
@@ -399,6 +401,9 @@ ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int
     sh.H = H; sh.G = G; sh.dim = dim; sh.vd = vd;
     sh.q_off = q_off; sh.k_off = q_off + G * dim; sh.v_off = q_off + 2 * G * dim;
     sh.b_off = b_off; sh.a_off = a_off; sh.g_off = g_off; sh.rank_a = rank_a; sh.rank_g = rank_g; sh.gate_silu = gate_silu;
+    if (from < 0 || (from == 0 && !walk)) return ST_ERR_BAD_ARG;
+    const bool chunks = from > 0 && from <= n_tokens;
+    const int below = chunks ? from : n_tokens + 1;
     sh.stride = chunks ? (sh.row() + 3) / 4 * 4 : sh.row();
     if (chunks && delta_chunks_floats(n_tokens, n_seqs, sh) == 0) return ST_ERR_BAD_SIZE;
     if (chunks && !aligned16(scratch)) return ST_ERR_BAD_ARG;
@@ -422,11 +427,7 @@ ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int
                                seq_of_token, q_start, slots);
         if (rc) return rc;
     }
-    if (chunks) {
-        rc = delta_chunks_launch(prep, sh, o + (size_t)n_tokens * H * vd, state, write_state, o, positions, q_start, slots, n_tokens,
-                                 n_seqs, s);
-        if (rc) return rc;
-    } else {
+    if (!chunks || walk) {
 #define DS_LAUNCH(L, R)                                                                                              \
     do {                                                                                                             \
         const size_t smem = DeltaScanSmem<L, R>::BYTES;                                                              \
@@ -437,7 +438,7 @@ ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int
         }                                                                                                            \
         rc = st_launch_pdl("delta_scan", delta_scan_kernel<L, R>,                                                    \
                            dim3(n_seqs, H, (vd + DS_THREADS / L - 1) / (DS_THREADS / L)), dim3(DS_THREADS), smem, s, \
-                           (const float*)prep, sh, state, write_state, o, positions, q_start, slots);                \
+                           (const float*)prep, sh, state, write_state, o, positions, q_start, slots, below);         \
     } while (0)
         // Lanes per column.  A token's step is a chain of dependent instructions, so a launch is as fast as its
         // blocks are spread: when eight lanes per column give fewer blocks than the device has multiprocessors,
@@ -461,6 +462,11 @@ ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int
             else DS_LAUNCH(16, 16);
         }
 #undef DS_LAUNCH
+        if (rc) return rc;
+    }
+    if (chunks) {
+        rc = delta_chunks_launch(prep, sh, o + (size_t)n_tokens * H * vd, state, write_state, o, positions, q_start, slots, n_tokens,
+                                 n_seqs, from, s);
         if (rc) return rc;
     }
     dim3 grid(n_tokens, H);

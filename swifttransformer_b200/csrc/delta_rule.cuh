@@ -18,8 +18,9 @@ struct DeltaShape {
     int stride;                   // floats from one prepared row to the next (at least row())
 };
 
-// Long portions in chunks (delta_chunks.cu): floats of scratch beyond the prepared rows and the outputs, 0: the sizes do not
-// fit; and the launch, between delta_prepare and delta_output.
+// Long portions in chunks (delta_chunks.cu): floats of scratch beyond the prepared rows and the outputs for n_seqs requests in
+// chunks, 0: the sizes do not fit; and the launch for the requests of at least `from` tokens, between delta_prepare and
+// delta_output.
 long long delta_chunks_floats(int n_tokens, int n_seqs, const DeltaShape& sh);
 int delta_chunks_launch(const float* prep, const DeltaShape& sh, float* scratch, float* state, int write_state, float* o,
-                        const int* positions, const int* q_start, const int* slots, int n_tokens, int n_seqs, cudaStream_t s);
+                        const int* positions, const int* q_start, const int* slots, int n_tokens, int n_seqs, int from, cudaStream_t s);

@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(128)
 hgrn2_cols_kernel(const T* __restrict__ proj, int ld, int q_off, int f_off, int v_off, const float* __restrict__ f_bias,
                   const float* __restrict__ lower, const float* __restrict__ gates, float* __restrict__ state,
                   float* __restrict__ o_raw, const int* __restrict__ positions, const int* __restrict__ q_start,
-                  const int* __restrict__ slots, int nh, int dim, int vd) {
+                  const int* __restrict__ slots, int below, int nh, int dim, int vd) {
     using L = HcLayout<R, LANES>;
     constexpr int DIMP = L::DIMP, COLS = L::COLS, CPW = L::CPW;
     constexpr int TOK_PASS = 128 / DIMP, PASSES = HG_GROUP / TOK_PASS;      // 128 threads cover 128 / DIMP tokens a pass
@@ -113,7 +113,7 @@ hgrn2_cols_kernel(const T* __restrict__ proj, int ld, int q_off, int f_off, int 
     ST_PDL_TRIGGER();
     const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * COLS;
     const int first = q_start[b], n = q_start[b + 1] - first;
-    if (n <= 0 || positions[first] < 0) return;           // padding of a fixed-shape step
+    if (n <= 0 || n >= below || positions[first] < 0) return;      // padding of a fixed-shape step; longer ones run in chunks
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int l = lane / CPW, cw = warp * CPW + lane % CPW, col = c0 + cw;
     float* st = state + ((size_t)slots[b] * nh + h) * dim * vd;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(128)
 hgrn2_wide_kernel(const T* __restrict__ proj, int ld, int q_off, int f_off, int v_off, const float* __restrict__ f_bias,
                   const float* __restrict__ lower, const float* __restrict__ gates, float* __restrict__ state,
                   float* __restrict__ o_raw, const int* __restrict__ positions, const int* __restrict__ q_start,
-                  const int* __restrict__ slots, int nh, int dim, int vd) {
+                  const int* __restrict__ slots, int below, int nh, int dim, int vd) {
     using L = HcLayout<R, 32>;
     constexpr int DIMP = L::DIMP, COLS = 4 * HW_C;           // four warps, four columns each
     constexpr int TOK_PASS = 128 / DIMP, PASSES = HG_GROUP / TOK_PASS;
@@ -238,7 +238,7 @@ hgrn2_wide_kernel(const T* __restrict__ proj, int ld, int q_off, int f_off, int 
     ST_PDL_TRIGGER();
     const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * COLS;
     const int first = q_start[b], n = q_start[b + 1] - first;
-    if (n <= 0 || positions[first] < 0) return;           // padding of a fixed-shape step
+    if (n <= 0 || n >= below || positions[first] < 0) return;      // padding of a fixed-shape step; longer ones run in chunks
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int col0 = c0 + warp * HW_C;                    // the warp's first column
     float* st = state + ((size_t)slots[b] * nh + h) * dim * vd;
@@ -373,11 +373,20 @@ hgrn2_gates_kernel(const T* __restrict__ proj, int ld, int q_off, int f_off, con
 template <typename T>
 __global__ void __launch_bounds__(256)
 hgrn2_norm_kernel(const float* __restrict__ o_raw, const float* __restrict__ norm_w, float eps, T* __restrict__ out,
-                  const int* __restrict__ positions, int n_tokens, int nh, int vd) {
+                  const int* __restrict__ positions, const int* __restrict__ q_start, int n_seqs, int below, int n_tokens, int nh,
+                  int vd) {
     ST_PDL_WAIT();
     ST_PDL_TRIGGER();
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (unit >= n_tokens * nh || positions[unit / nh] < 0) return;
+    if (below <= n_tokens) {                              // a token of a request that runs in chunks is not this kernel's
+        int lo = 0, hi = n_seqs;                          // the last request that begins at or before the token
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (q_start[mid] <= unit / nh) lo = mid; else hi = mid;
+        }
+        if (q_start[lo + 1] - q_start[lo] >= below) return;
+    }
     const float* row = o_raw + (size_t)unit * vd;
     float ss = 0.f;
     for (int j = lane; j < vd; j += 32) { const float v = __ldcg(row + j); ss = fmaf(v, v, ss); }
@@ -394,13 +403,15 @@ static size_t hgrn2_smem(int dim, int vd) {
 // state: [slots, nh, dim, vd] float; out: [tokens, nh * vd]
 // o_raw: float scratch [tokens, nh * vd] for the form with the state in registers (dim <= 128), or null for the
 // form with one block per head and the state in shared memory; gates: float scratch [tokens, 2 * nh * dim] or null:
-// with it the gates and queries are prepared by a kernel of their own (worth it for long portions)
+// with it the gates and queries are prepared by a kernel of their own (worth it for long portions); below: requests of so many
+// tokens and more are not touched (taken by the form with the state in registers); layout: of that form, 1 for few tokens per
+// request, 2 for portions, 0 by the step's average
 ST_EXPORT int st_hgrn2_scan(const void* proj, int ld, int q_off, int f_off, int v_off, const float* f_bias,
                             const float* lower, const float* norm_w, float eps, float* state, void* out, float* o_raw,
-                            float* gates, const int* positions, const int* q_start, const int* slots, int n_tokens, int n_seqs, int nh,
-                            int dim, int vd, int dtype, void* stream) {
+                            float* gates, const int* positions, const int* q_start, const int* slots, int n_tokens, int n_seqs, int below,
+                            int layout, int nh, int dim, int vd, int dtype, void* stream) {
     if (n_seqs <= 0 || n_tokens <= 0) return 0;
-    if (nh <= 0 || dim <= 0 || vd <= 0) return ST_ERR_BAD_ARG;
+    if (nh <= 0 || dim <= 0 || vd <= 0 || (below <= n_tokens && (!o_raw || dim > 128))) return ST_ERR_BAD_ARG;
     if (dtype != 0 && dtype != 1) return ST_ERR_BAD_DTYPE;
     cudaStream_t s = (cudaStream_t)stream;
     if (o_raw && dim <= 128) {
@@ -416,15 +427,15 @@ ST_EXPORT int st_hgrn2_scan(const void* proj, int ld, int q_off, int f_off, int 
     rc = st_launch_pdl("hgrn2_cols", hgrn2_cols_kernel<T, R, LANES>,                                                  \
                        dim3(n_seqs, nh, (vd + HcLayout<R, LANES>::COLS - 1) / HcLayout<R, LANES>::COLS), dim3(128), 0, s, \
                        (const T*)proj, ld, q_off, f_off, v_off, f_bias, lower, (const float*)gates, state, o_raw,     \
-                       positions, q_start, slots, nh, dim, vd)
+                       positions, q_start, slots, below, nh, dim, vd)
     // Long portions: the wide form (32 lanes per column, four columns per warp).  Steps of few tokens per request
     // are bound by reading and writing the state: eight lanes per column with many rows each, four columns side by
     // side per warp.
-    const bool long_portions = n_tokens > 4 * n_seqs;
+    const bool long_portions = layout ? layout == 2 : n_tokens > 4 * n_seqs;
 #define HW_LAUNCH(T, R)                                                                                               \
     rc = st_launch_pdl("hgrn2_wide", hgrn2_wide_kernel<T, R>, dim3(n_seqs, nh, (vd + 4 * HW_C - 1) / (4 * HW_C)), dim3(128), \
                        0, s, (const T*)proj, ld, q_off, f_off, v_off, f_bias, lower, (const float*)gates, state, o_raw, \
-                       positions, q_start, slots, nh, dim, vd)
+                       positions, q_start, slots, below, nh, dim, vd)
 #define HC_PICK(T)                                                    \
     do {                                                              \
         if (dim <= 8) HC_LAUNCH(T, 1, 8);                             \
@@ -445,9 +456,9 @@ ST_EXPORT int st_hgrn2_scan(const void* proj, int ld, int q_off, int f_off, int 
         const int units = n_tokens * nh;
         if (dtype == 0)
             return st_launch_pdl("hgrn2_norm", hgrn2_norm_kernel<float>, dim3((units + 7) / 8), dim3(256), 0, s,
-                                 (const float*)o_raw, norm_w, eps, (float*)out, positions, n_tokens, nh, vd);
+                                 (const float*)o_raw, norm_w, eps, (float*)out, positions, q_start, n_seqs, below, n_tokens, nh, vd);
         return st_launch_pdl("hgrn2_norm", hgrn2_norm_kernel<bf16>, dim3((units + 7) / 8), dim3(256), 0, s,
-                             (const float*)o_raw, norm_w, eps, (bf16*)out, positions, n_tokens, nh, vd);
+                             (const float*)o_raw, norm_w, eps, (bf16*)out, positions, q_start, n_seqs, below, n_tokens, nh, vd);
     }
     const size_t smem = hgrn2_smem(dim, vd);
     if (smem > 200 * 1024) return ST_ERR_TOO_LARGE;

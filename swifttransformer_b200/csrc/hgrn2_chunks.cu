@@ -15,14 +15,14 @@
 // chunk it is a matrix product of q and k~ decayed to the half's border.  All of it is float arithmetic.
 //
 // Measured on one B200, 2000 tokens of one request, 16 heads of 128 x 128, bfloat16 rows: 155 us (kv 40, scan 18, out 106
-// alone) against 1030 for the walk (hgrn2_wide); 1000 tokens of 8 heads 61 / 522; 2 x 66 tokens 50 / 45, so portions of fewer
-// than about 100 tokens stay with the walk.  kv and out are bound by their instructions (half of the issue slots used,
-// two blocks of 256 threads per SM), the scan by its two trips to the second-level cache.  Against 64 bits the states
+// alone) against 1030 for the walk (hgrn2_wide); 1000 tokens of 8 heads 61 / 522; 70 tokens of 16 heads 60 / 52, so portions of
+// fewer than about 100 tokens stay with the walk.  kv and out are bound by their instructions
+// (two blocks of 256 threads per SM), the scan by its two trips to the second-level cache.  Against 64 bits the states
 // are off by 2.9e-7 where the walk's are by 4.0e-7 (fewer roundings in a row).
 #include "chunks.cuh"
 
 struct HgrnShape {
-    int ld, q_off, f_off, v_off, n_seqs, nh, dim, vd;
+    int ld, q_off, f_off, v_off, n_seqs, from, nh, dim, vd;
     float eps;
     const float *f_bias, *lower, *norm_w;
     const int *positions, *q_start, *slots;
@@ -44,7 +44,7 @@ hgrn2_chunk_kv_kernel(const T* __restrict__ proj, const HgrnShape sh, float* __r
     const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dim = sh.dim, vd = sh.vd;
     int b, first, n;
-    if (!hk_find(sh.q_start, sh.positions, sh.n_seqs, place, b, first, n)) return;
+    if (!hk_find(sh.q_start, sh.positions, sh.n_seqs, sh.from, place, b, first, n)) return;
     {   // every thread asks for all its pieces before it works on one
         constexpr int N = HK_C * HK_D / 4 / 256;
         const int e = (tid % (HK_D / 4)) * 4, t0 = tid / (HK_D / 4);
@@ -124,10 +124,10 @@ hgrn2_chunk_scan_kernel(const HgrnShape sh, float* __restrict__ states, const fl
     ST_PDL_WAIT();
     const int b = blockIdx.z, h = blockIdx.y, dim = sh.dim, vd = sh.vd;
     const int begin = sh.q_start[b], n = sh.q_start[b + 1] - begin;
-    if (n <= 0 || sh.positions[begin] < 0) return;
+    if (n < sh.from || sh.positions[begin] < 0) return;
     const int e = (blockIdx.x * 128 + threadIdx.x) * 4;
     if (e < dim * vd) {
-        const int place = begin / HK_C + b, chunks = (n + HK_C - 1) / HK_C;
+        const int place = hk_place(begin, b, sh.from), chunks = (n + HK_C - 1) / HK_C;
         const size_t step = (size_t)sh.nh * dim * vd, dstep = (size_t)sh.nh * dim;
         float* at = states + (size_t)place * step + (size_t)h * dim * vd + e;
         const float* dec = decays + (size_t)place * dstep + h * dim + e / vd;
@@ -175,7 +175,7 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
     const int place = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int dim = sh.dim, vd = sh.vd;
     int b, first, n;
-    if (!hk_find(sh.q_start, sh.positions, sh.n_seqs, place, b, first, n)) return;
+    if (!hk_find(sh.q_start, sh.positions, sh.n_seqs, sh.from, place, b, first, n)) return;
     const float* S0 = states + ((size_t)place * sh.nh + h) * dim * vd;
     hk_copy_rows(m.S, S0, 0, dim, vd);
     hk_copy_rows(m.S, S0, HK_SR, dim, vd);
@@ -350,28 +350,30 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
     ST_PDL_TRIGGER();
 }
 
-// Floats of scratch a step of this shape needs, 0: the sizes do not fit (rows of whole 16-byte pieces, at most 128 channels
-// and values per head).
+// Floats of scratch for n_seqs requests in chunks in a step of n_tokens tokens, 0: the sizes do not fit (rows of whole 16-byte
+// pieces, at most 128 channels and values per head).
 ST_EXPORT long long st_hgrn2_chunks_scratch(int n_tokens, int n_seqs, int nh, int dim, int vd) {
     if (n_tokens <= 0 || n_seqs <= 0 || nh <= 0 || dim <= 0 || vd <= 0 || dim % 4 || vd % 4 || dim > HK_D || vd > HK_D) return 0;
-    return ((long long)n_tokens / HK_C + n_seqs) * nh * dim * ((long long)vd + 1);
+    return hk_places(n_tokens, n_seqs) * nh * dim * ((long long)vd + 1);
 }
 
-// Arguments as st_hgrn2_scan; scratch: float, 16-byte aligned, st_hgrn2_chunks_scratch elements.  Columns and rows of proj
-// must begin on four elements.
+// Arguments as st_hgrn2_scan, for the requests of at least `from` tokens (the others are not touched); scratch: float, 16-byte
+// aligned, st_hgrn2_chunks_scratch elements for min(n_seqs, n_tokens / from) requests.  Columns and rows of proj must begin
+// on four elements.
 ST_EXPORT int st_hgrn2_chunks(const void* proj, int ld, int q_off, int f_off, int v_off, const float* f_bias, const float* lower,
                               const float* norm_w, float eps, float* state, void* out, float* scratch, const int* positions,
-                              const int* q_start, const int* slots, int n_tokens, int n_seqs, int nh, int dim, int vd, int dtype,
-                              void* stream) {
-    if (n_seqs <= 0 || n_tokens <= 0) return 0;
+                              const int* q_start, const int* slots, int n_tokens, int n_seqs, int from, int nh, int dim, int vd,
+                              int dtype, void* stream) {
+    if (n_seqs <= 0 || n_tokens <= 0 || n_tokens < from) return 0;
+    if (from <= 0) return ST_ERR_BAD_ARG;
     if (st_hgrn2_chunks_scratch(n_tokens, n_seqs, nh, dim, vd) == 0) return ST_ERR_BAD_SIZE;
     if (dtype != 0 && dtype != 1) return ST_ERR_BAD_DTYPE;
     if (ld % 4 || q_off % 4 || f_off % 4 || v_off % 4 || !aligned16(proj) || !aligned16(out) || !aligned16(state) ||
         !aligned16(scratch) || !aligned16(f_bias) || !aligned16(lower) || !aligned16(norm_w)) return ST_ERR_BAD_ARG;
-    const long long places = n_tokens / HK_C + n_seqs;
+    const long long places = hk_places(n_tokens, hk_longs(n_tokens, n_seqs, from));
     if (nh > 65535 || n_seqs > 65535) return ST_ERR_TOO_LARGE;
     cudaStream_t s = (cudaStream_t)stream;
-    HgrnShape sh{ld, q_off, f_off, v_off, n_seqs, nh, dim, vd, eps, f_bias, lower, norm_w, positions, q_start, slots};
+    HgrnShape sh{ld, q_off, f_off, v_off, n_seqs, from, nh, dim, vd, eps, f_bias, lower, norm_w, positions, q_start, slots};
     float* states = scratch;
     float* decays = scratch + places * nh * dim * vd;
     const size_t kv_smem = sizeof(float) * 2 * HK_C * HK_LD;

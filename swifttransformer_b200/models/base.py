@@ -156,9 +156,8 @@ class CausalLM:
         plans: Dict[str, Any] = {}
         for st in self.layer_order:
             mixer = self.blocks[st.block].mixer
-            p = mixer.step_plan() if mixer is not None else None
-            if p is not None and p.name not in plans:
-                plans[p.name] = p
+            for p in mixer.step_plans() if mixer is not None else ():
+                plans.setdefault(p.name, p)
         return list(plans.values())
 
     def forward(self, ctx: Any, caches: List[Any]) -> Optional[torch.Tensor]:

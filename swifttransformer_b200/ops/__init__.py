@@ -896,8 +896,49 @@ def diff_attention_tiles(q: torch.Tensor, pool: torch.Tensor, layer: int, out: t
 
 # ------------------------------------------------------------ gated linear recurrence
 HGRN2_GATES_MIN_TOKENS = 64      # steps of more tokens prepare the recurrence's gates in a kernel of their own
-# steps of at least so many tokens per request run in chunks side by side (at 66 the walk is ahead, 45 / 50 us; at 150 the chunks, 87 / 55)
+# Portions of about so many tokens and more run in chunks side by side.  us on one B200, walk / chunks, 16 heads of 128 x 128:
+# one request of 70 tokens 52 / 60, 96 67 / 60, 128 91 / 63; 4 heads 96 52 / 58, 128 67 / 61; 16 requests of 100 tokens 271 / 183.
 HGRN2_CHUNK_MIN_TOKENS = 96
+
+def _hgrn2_chunks_from(n: int, n_seqs: int, nh: int, dim: int) -> int:
+    """The tokens from which a request of this step runs in chunks.  Alone, the chunks' three kernels must beat one chain of
+    tokens: a sixth more, half as much for few narrow heads (128 tokens of 8 heads of 64 x 64: walk 49, chunks 55; 16 heads: 61, 55).  Heads of up to 64 channels: with many requests the walk fills the device and loses less, so the line
+    rises with the step's work (16 requests of 100 tokens, 16 heads of 64 x 64: walk 99, chunks 121; 8 of 150: 146, 100; 32 of
+    100: 169, 207; 8 of 250: 187, 122)."""
+    base = HGRN2_CHUNK_MIN_TOKENS
+    if n_seqs == 1:
+        return base * 3 // 2 if dim <= 64 and nh <= 8 else base * 7 // 6
+    return int(base * min(max((40 + n * nh / 250) / 96, 1.0), 2.0)) if dim <= 64 else base
+
+
+def chunk_split(lens: Sequence[int], limit: int):
+    """How a step's requests are shared between a recurrence's two forms: (the tokens from which one runs in chunks, 0: none
+    does; what else has to walk token by token: 0 nothing, 1 few tokens each, 2 portions of some length).  Every request goes
+    by its own portion, whoever shares its step."""
+    short = [int(n) for n in lens if n < limit]
+    if len(short) == len(lens):
+        return 0, 1
+    return limit, 0 if not short else 2 if sum(short) > 4 * len(short) else 1
+
+
+def _split_of(n: int, n_seqs: int, limit: int):
+    """The same where only the step's shape is known: all or none, by the average portion."""
+    return (1, 0) if n >= limit * n_seqs else (0, 1)
+
+
+def hgrn2_split(lens: Sequence[int], n_tokens: int, n_seqs: int, nh: int, dim: int):
+    """``chunk_split`` for ``hgrn2_scan`` (n_tokens, n_seqs: of the step with its padding)."""
+    return chunk_split(lens, _hgrn2_chunks_from(n_tokens, n_seqs, nh, dim))
+
+
+def hgrn2_scratch(n_tokens: int, n_seqs: int, nh: int, dim: int, vd: int, split=None) -> int:
+    """Floats of scratch with which ``hgrn2_scan`` takes its fastest form for a step of this shape."""
+    walk = n_tokens * nh * (vd + 2 * dim)
+    start, _ = split or _split_of(n_tokens, n_seqs, _hgrn2_chunks_from(n_tokens, n_seqs, nh, dim))
+    if not start or n_tokens < start:
+        return walk
+    return max(walk, int(lib().st_hgrn2_chunks_scratch(n_tokens, min(n_seqs, n_tokens // start), nh, dim, vd)))
+
 
 def _hgrn2_chunks_apply(n: int, n_seqs: int, nh: int, dim: int, vd: int, scratch: torch.Tensor, columns, tensors) -> bool:
     """Whether the chunked form takes this step: at most 128 channels and values per head in multiples of four, columns that
@@ -910,7 +951,8 @@ def _hgrn2_chunks_apply(n: int, n_seqs: int, nh: int, dim: int, vd: int, scratch
 def hgrn2_scan(proj: torch.Tensor, q_off: int, f_off: int, v_off: int, f_bias: torch.Tensor, lower: torch.Tensor,
                norm_w: torch.Tensor, eps: float, state: torch.Tensor, out: torch.Tensor, positions: torch.Tensor,
                q_start: torch.Tensor, slots: torch.Tensor, n_seqs: int, nh: int, dim: int, vd: int,
-               scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
+               scratch: Optional[torch.Tensor] = None,
+               split=None) -> torch.Tensor:
     """The HGRN2 recurrence over each request's tokens of the step, from the fused projection (queries, gates and
     values at column offsets q_off, f_off, v_off): S <- diag(f) S + (1 - f) v^T, o = S^T silu(q), f = lower +
     (1 - lower) sigmoid(gate + f_bias); out [tokens, nh * vd] = rms(o) * norm_w per head.  ``state``: float32
@@ -918,26 +960,34 @@ def hgrn2_scan(proj: torch.Tensor, q_off: int, f_off: int, v_off: int, f_bias: t
     dim <= 128) the state is carried in registers and a head's columns are spread over blocks; without it one block
     per (request, head) keeps the state in shared memory.  With room for tokens * nh * (vd + 2 * dim) elements and
     more than HGRN2_GATES_MIN_TOKENS tokens, the gates and queries are prepared by a kernel of their own instead of
-    by every block of a head again.  Steps of HGRN2_CHUNK_MIN_TOKENS tokens per request and more, dim and vd multiples of
-    four up to 128, run in chunks of 64 tokens side by side where ``scratch`` holds a state per chunk
-    ((tokens / 64 + n_seqs) * nh * dim * (vd + 1) elements; the size above does from 128 tokens of one request on)."""
+    by every block of a head again.  Requests that bring about HGRN2_CHUNK_MIN_TOKENS tokens and more (``_hgrn2_chunks_from``),
+    dim and vd multiples of four up to 128, run in chunks of 64 tokens side by side where ``scratch`` holds a state per chunk
+    (``hgrn2_scratch`` elements do), the others token by token: ``split`` says which (``hgrn2_split``); without it all or none
+    do, by the average portion."""
     assert proj.is_contiguous() and out.is_contiguous() and out.shape == (proj.shape[0], nh * vd)
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (nh, dim, vd)
     gates = None
     if scratch is not None:
         assert scratch.dtype == torch.float32 and scratch.numel() >= out.numel()
         n = proj.shape[0]
-        if n >= HGRN2_CHUNK_MIN_TOKENS * n_seqs and _hgrn2_chunks_apply(
-                n, n_seqs, nh, dim, vd, scratch, (proj.shape[1], q_off, f_off, v_off), (proj, out, state, f_bias, lower, norm_w)):
+        start, walk = split or _split_of(n, n_seqs, _hgrn2_chunks_from(n, n_seqs, nh, dim))
+        chunks = 0 < start <= n and _hgrn2_chunks_apply(
+            n, min(n_seqs, n // start), nh, dim, vd, scratch, (proj.shape[1], q_off, f_off, v_off),
+            (proj, out, state, f_bias, lower, norm_w))
+        if n > HGRN2_GATES_MIN_TOKENS and scratch.numel() >= n * nh * (vd + 2 * dim) and not (chunks and walk == 1):
+            gates = scratch[n * nh * vd:]
+        if chunks:
+            if walk:     # the shorter ones; their sums and gates are read before the chunks' states take their place
+                _check(lib().st_hgrn2_scan(_p(proj), proj.shape[1], q_off, f_off, v_off, _p(f_bias), _p(lower), _p(norm_w),
+                                           _f(eps), _p(state), _p(out), _p(scratch), _p(gates), _p(positions), _p(q_start),
+                                           _p(slots), n, n_seqs, start, walk, nh, dim, vd, _dt(proj), _stream()), "hgrn2_scan")
             _check(lib().st_hgrn2_chunks(_p(proj), proj.shape[1], q_off, f_off, v_off, _p(f_bias), _p(lower), _p(norm_w),
                                          _f(eps), _p(state), _p(out), _p(scratch), _p(positions), _p(q_start), _p(slots),
-                                         n, n_seqs, nh, dim, vd, _dt(proj), _stream()), "hgrn2_scan")
+                                         n, n_seqs, start, nh, dim, vd, _dt(proj), _stream()), "hgrn2_scan")
             return out
-        if n > HGRN2_GATES_MIN_TOKENS and scratch.numel() >= n * nh * (vd + 2 * dim):
-            gates = scratch[n * nh * vd:]
     _check(lib().st_hgrn2_scan(_p(proj), proj.shape[1], q_off, f_off, v_off, _p(f_bias), _p(lower), _p(norm_w),
                                _f(eps), _p(state), _p(out), _p(scratch), _p(gates), _p(positions), _p(q_start), _p(slots),
-                               proj.shape[0], n_seqs, nh, dim, vd, _dt(proj), _stream()), "hgrn2_scan")
+                               proj.shape[0], n_seqs, 0x7fffffff, 0, nh, dim, vd, _dt(proj), _stream()), "hgrn2_scan")
     return out
 
 
@@ -1510,17 +1560,31 @@ def gqa_attention_plain(q: torch.Tensor, pool: torch.Tensor, layer: int, out: to
 
 
 # ------------------------------------------------------------ the gated delta rule
-# Steps of at least so many tokens per request run in chunks side by side (at 200 the walk is ahead, 93 / 100 us; at 300 the
-# chunks, 138 / 119).
+# Portions of so many tokens and more run in chunks side by side.  us on one B200, walk / chunks, 8 heads of 128 x 128: one
+# request of 200 tokens 81 / 92, 256 97 / 110, 300 116 / 95; two of 260 164 / 113, sixteen 637 / 493; 4 heads of 64 x 64: 256
+# 70 / 74, 300 79 / 74, sixteen of 260 174 / 173.
 DELTA_CHUNK_MIN_TOKENS = 256
 
 
-def delta_rule_scratch(n_tokens: int, H: int, G: int, dim: int, vd: int) -> int:
-    """Floats of scratch for ``delta_rule``: with them, portions of DELTA_CHUNK_MIN_TOKENS tokens and more run in chunks."""
+def _delta_chunks_from(n_seqs: int) -> int:
+    """The tokens from which a request of the step runs in chunks (alone an eighth more, see the figures above)."""
+    return DELTA_CHUNK_MIN_TOKENS * 9 // 8 if n_seqs == 1 else DELTA_CHUNK_MIN_TOKENS
+
+
+def delta_split(lens: Sequence[int], n_tokens: int, n_seqs: int):
+    """``chunk_split`` for ``delta_rule`` (n_tokens, n_seqs: of the step with its padding)."""
+    return chunk_split(lens, _delta_chunks_from(n_seqs))
+
+
+def delta_rule_scratch(n_tokens: int, H: int, G: int, dim: int, vd: int, n_seqs: Optional[int] = None, split=None) -> int:
+    """Floats of scratch for ``delta_rule``: with them, portions of DELTA_CHUNK_MIN_TOKENS tokens and more run in chunks
+    (n_seqs: the step's requests, None: any number; split: as ``delta_rule`` will be given it)."""
     walk = int(lib().st_delta_rule_scratch_floats(n_tokens, H, G, dim, vd))
-    if n_tokens < DELTA_CHUNK_MIN_TOKENS:
-        return walk
-    return max(walk, int(lib().st_delta_rule_chunk_floats(n_tokens, n_tokens // DELTA_CHUNK_MIN_TOKENS, H, G, dim, vd)))
+    longs = n_tokens // DELTA_CHUNK_MIN_TOKENS
+    if n_seqs is not None:
+        start, _ = split or _split_of(n_tokens, n_seqs, _delta_chunks_from(n_seqs))
+        longs = min(n_seqs, n_tokens // start) if start else 0
+    return max(walk, int(lib().st_delta_rule_chunk_floats(n_tokens, longs, H, G, dim, vd))) if longs else walk
 
 
 def delta_rule_set_lanes(lanes: int) -> None:
@@ -1534,7 +1598,7 @@ def delta_rule(proj: torch.Tensor, b_off: int, a_off: int, g_off: int, conv_w: t
                eps: float, out_scale: float, state: torch.Tensor, write_state: bool, single_tokens: bool,
                scratch: torch.Tensor, out: torch.Tensor, positions: torch.Tensor, seq_of_token: torch.Tensor,
                q_start: torch.Tensor, slots: torch.Tensor, n_seqs: int, H: int, G: int, dim: int, vd: int,
-               gate_silu: bool = False) -> torch.Tensor:
+               gate_silu: bool = False, split=None) -> torch.Tensor:
     """The gated delta rule over each request's tokens of the step, from the float32 projection ``proj`` [tokens,
     columns] = q (G * dim) | k (G * dim) | v (H * vd) from column 0, write strengths at b_off (H), the low-rank
     inputs of the decays at a_off and of the output gates at g_off.  ``conv_w`` float32 [channels, taps], the
@@ -1543,8 +1607,9 @@ def delta_rule(proj: torch.Tensor, b_off: int, a_off: int, g_off: int, conv_w: t
     moved on.  out [tokens, H * vd] in the type of ``w_a2`` / ``w_g2``.  ``w_a2`` None: the projection holds one
     decay logit per head at a_off and ``dt_bias`` is [H]; ``w_g2`` None: it holds the output gate's H * vd logits
     at g_off.  ``gate_silu``: the gate is z * sigmoid(z) instead of sigmoid(z).  ``scratch``: ``delta_rule_scratch``
-    elements; steps of DELTA_CHUNK_MIN_TOKENS tokens per request and more (dim and vd multiples of four up to 128) run in
-    chunks of 64 tokens side by side, with less scratch token by token like the others."""
+    elements; requests that bring DELTA_CHUNK_MIN_TOKENS tokens and more (dim and vd multiples of four up to 128) run in chunks
+    of 64 tokens side by side, the others, and with less scratch all, token by token: ``split`` says which (``delta_split``);
+    without it all or none do, by the average portion."""
     assert proj.dtype == torch.float32 and proj.is_contiguous() and out.is_contiguous()
     assert out.shape == (proj.shape[0], H * vd) and all(w is None or w.dtype == out.dtype for w in (w_a2, w_g2))
     assert state.dtype == torch.float32 and state.is_contiguous() and state.shape[1:] == (H, dim, vd)
@@ -1558,14 +1623,17 @@ def delta_rule(proj: torch.Tensor, b_off: int, a_off: int, g_off: int, conv_w: t
     n = proj.shape[0]
     assert scratch.dtype == torch.float32
     assert scratch.numel() >= int(lib().st_delta_rule_scratch_floats(n, H, G, dim, vd))
-    chunks = (n >= DELTA_CHUNK_MIN_TOKENS * n_seqs and scratch.data_ptr() % 16 == 0
-              and 0 < int(lib().st_delta_rule_chunk_floats(n, n_seqs, H, G, dim, vd)) <= scratch.numel())
+    start, walk = split or _split_of(n, n_seqs, _delta_chunks_from(n_seqs))
+    if not (0 < start <= n and scratch.data_ptr() % 16 == 0 and 0 < int(lib().st_delta_rule_chunk_floats(
+            n, min(n_seqs, n // start), H, G, dim, vd)) <= scratch.numel()):
+        start, walk = 0, 1
     _check(lib().st_delta_rule(_p(proj), proj.shape[1], 0, b_off, a_off, g_off,
                                w_a2.shape[1] if w_a2 is not None else 0, w_g2.shape[1] if w_g2 is not None else 0,
                                _p(conv_w), taps, _p(conv_state), _p(w_a2), _p(a_log), _p(dt_bias), _p(w_g2),
                                _p(norm_w), _f(eps), _f(out_scale), _p(state), int(write_state), int(single_tokens),
                                _p(scratch), _p(out), _p(positions), _p(seq_of_token), _p(q_start), _p(slots),
-                               proj.shape[0], n_seqs, H, G, dim, vd, _dt(out), _stream(), int(gate_silu), int(chunks)), "delta_rule")
+                               proj.shape[0], n_seqs, H, G, dim, vd, _dt(out), _stream(), int(gate_silu), start, walk),
+           "delta_rule")
     return out
 
 

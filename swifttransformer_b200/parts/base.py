@@ -178,6 +178,11 @@ class Mixer(Part):
     def step_plan(self) -> Optional[StepPlan]:
         return None
 
+    def step_plans(self) -> List[StepPlan]:
+        """All plans of the mixer (more than one where it holds other mixers)."""
+        p = self.step_plan()
+        return [] if p is None else [p]
+
     def forward(self, h: torch.Tensor, ctx: Any, cache: Any) -> Delta:
         raise NotImplementedError
 

@@ -47,8 +47,8 @@ class InputConv(Mixer):
     def cache_spec(self):
         return (StateSpec((self.taps - 1, self.width), torch.float32), self.inner.cache_spec())
 
-    def step_plan(self):
-        return self.inner.step_plan()
+    def step_plans(self):
+        return self.inner.step_plans()
 
     def forward(self, h: torch.Tensor, ctx: Any, cache: Any) -> Delta:
         tails, inner_cache = cache

@@ -29,6 +29,7 @@ import torch
 from .. import ops
 from ..weights.spec import GAIN, MATRIX, VECTOR, ParamSpec
 from .base import MIXERS, Delta, Mixer, StateSpec
+from .portions import PortionPlan
 
 
 @MIXERS.register("gated_delta_rule")
@@ -36,6 +37,8 @@ class GatedDeltaRule(Mixer):
     """names: matrices {"q","k","v","b","a1","a2","g1","g2","o"} ([out, in]; "<q|k|v>.conv" are their filters
     [channels, taps]), vectors {"A_log" [heads], "dt_bias" [heads * dim]}, and "norm" [vdim].  ``rank``: the
     low-rank pairs' inner size when weights are made at random (a checkpoint's own is taken as it is)."""
+
+    PLAN = PortionPlan("gated_delta_rule", ops.delta_split)
 
     def __init__(self, hidden: int, num_heads: int, num_qk_heads: int, dim: int, vdim: int, conv_taps: int, eps: float,
                  names: Dict[str, str], out_scale: float = 1.0, float_out: bool = False, rank: int = 16,
@@ -97,6 +100,9 @@ class GatedDeltaRule(Mixer):
         return (StateSpec((self.taps - 1, self.channels), torch.float32),
                 StateSpec((self.H, self.dim, self.vdim), torch.float32))
 
+    def step_plan(self) -> PortionPlan:
+        return self.PLAN
+
     def forward(self, h: torch.Tensor, ctx: Any, cache: Any) -> Delta:
         tails, mats = cache
         n = h.shape[0]
@@ -106,11 +112,12 @@ class GatedDeltaRule(Mixer):
         g_off = a_off + self.rank_a
         single = bool(getattr(ctx, "single_tokens", False))
         o = torch.empty((n, self.H * self.vdim), dtype=h.dtype, device=h.device)
-        scratch = ctx.scratch_f32(ops.delta_rule_scratch(n, self.H, self.G, self.dim, self.vdim))
+        split = ctx.plan(self.PLAN.name)
+        scratch = ctx.scratch_f32(ops.delta_rule_scratch(n, self.H, self.G, self.dim, self.vdim, ctx.n_seqs, split))
         ops.delta_rule(proj, b_off, a_off, g_off, self.conv_w, tails.state, self.w_a2, self.a_log, self.dt_bias,
                        self.w_g2, self.norm_w, self.eps, self.out_scale, mats.state, mats.writable, single, scratch, o,
                        ctx.positions, ctx.seq_of_token, ctx.q_start, ctx.slots, ctx.n_seqs, self.H, self.G, self.dim,
-                       self.vdim, gate_silu=self.gate_silu)
+                       self.vdim, gate_silu=self.gate_silu, split=split)
         if self.taps > 1 and tails.writable and not (single and mats.writable):
             ops.conv_state_update(proj, self.channels, tails.state, ctx.positions, ctx.q_start, ctx.slots, ctx.n_seqs)
         return Delta(ops.linear(o, self.w_o, out_dtype=torch.float32 if self.float_out else None))

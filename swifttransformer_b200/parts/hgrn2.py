@@ -19,6 +19,7 @@ import torch
 from .. import ops
 from ..weights.spec import GAIN, MATRIX, VECTOR, ParamSpec
 from .base import MIXERS, Delta, Mixer, StateSpec
+from .portions import PortionPlan
 
 
 @MIXERS.register("hgrn2")
@@ -28,6 +29,7 @@ class HGRN2(Mixer):
     def __init__(self, hidden: int, num_heads: int, dim: int, vdim: int, eps: float, names: Dict[str, str]):
         self.hidden, self.nh, self.dim, self.vdim, self.eps, self.names = hidden, num_heads, dim, vdim, float(eps), dict(names)
         self.w_qfv = self.w_o = self.f_bias = self.lower = self.norm_w = None
+        self._plan = PortionPlan(f"hgrn2_{num_heads}_{dim}", lambda lens, n, b: ops.hgrn2_split(lens, n, b, num_heads, dim))
 
     def param_specs(self) -> List[ParamSpec]:
         n, qw, vw = self.names, self.nh * self.dim, self.nh * self.vdim
@@ -45,13 +47,20 @@ class HGRN2(Mixer):
     def cache_spec(self):
         return StateSpec((self.nh, self.dim, self.vdim), torch.float32)
 
+    def step_plan(self) -> PortionPlan:
+        return self._plan
+
     def forward(self, h: torch.Tensor, ctx: Any, cache: Any) -> Delta:
         qw = self.nh * self.dim
         proj = ops.linear(h, self.w_qfv)
         o = torch.empty((h.shape[0], self.nh * self.vdim), dtype=h.dtype, device=h.device)
+        split = ctx.plan(self._plan.name)
+        scratch = None
+        if self.dim <= 128:
+            scratch = ctx.scratch_f32(ops.hgrn2_scratch(h.shape[0], ctx.n_seqs, self.nh, self.dim, self.vdim, split))
         ops.hgrn2_scan(proj, 0, qw, 2 * qw, self.f_bias, self.lower, self.norm_w, self.eps, cache.state, o,
                        ctx.positions, ctx.q_start, ctx.slots, ctx.n_seqs, self.nh, self.dim, self.vdim,
-                       scratch=ctx.scratch_f32(h.shape[0] * self.nh * (self.vdim + 2 * self.dim)) if self.dim <= 128 else None)
+                       scratch=scratch, split=split)
         return Delta(ops.linear(o, self.w_o))
 
     def param_bytes(self) -> int:

@@ -57,9 +57,8 @@ class SideBySide(Mixer):
     def cache_spec(self):
         return (self.left.cache_spec(), self.right.cache_spec())
 
-    def step_plan(self):
-        # (at most one member has a plan of its own kind; both would share it by name anyway)
-        return self.left.step_plan() or self.right.step_plan()
+    def step_plans(self):
+        return self.left.step_plans() + self.right.step_plans()
 
     def forward(self, h: torch.Tensor, ctx: Any, cache: Any) -> Delta:
         a = self.left.forward(h, ctx, cache[0])

@@ -55,9 +55,10 @@ def reference(proj, w, H, G, d, dv, rank, eps, out_scale):
 
 
 def step(projs, lens, starts, H, G, d, dv, rank, w, tails, state, dtype, chunks, monkeypatch, slots, write=True, pad=3):
-    """One step over the requests' next tokens; -> rows per request."""
+    """One step over the requests' next tokens; -> rows per request.  chunks: True all in chunks, False none, None
+    each by its own portion."""
     from swifttransformer_b200 import ops
-    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", 1 if chunks else 1 << 30)
+    monkeypatch.setattr(ops, "DELTA_CHUNK_MIN_TOKENS", {True: 1, False: 1 << 30, None: 256}[chunks])
     st = Step([(s, a, n) for s, a, n in zip(slots, starts, lens)], pad_tokens=pad, pad_requests=2)
     rows = dev(np.concatenate([p[a:a + n] for p, a, n in zip(projs, starts, lens)] + [np.full((pad, projs[0].shape[1]), 7.0)]))
     C = 2 * G * d + H * dv
@@ -66,9 +67,10 @@ def step(projs, lens, starts, H, G, d, dv, rank, w, tails, state, dtype, chunks,
     scratch = torch.full((max(need, ops.delta_rule_scratch(st.n_rows, H, G, d, dv)),), float("nan"), device="cuda")
     out = torch.full((st.n_rows, H * dv), 77.0, dtype=TD[dtype], device="cuda")
     low = lambda a: None if a is None else dev(a, TD[dtype])
+    split = ops.delta_split(lens, st.n_rows, st.n_seqs) if chunks is None else None
     ops.delta_rule(rows, C, C + H, C + H + (rank or H), dev(w["conv"]), tails, low(w["a2"]), dev(w["A_log"]), dev(w["dt_bias"]),
                    low(w["g2"]), dev(w["norm"]), 1e-5, 0.7, state, write, False, scratch, out, st.positions, st.seq, st.q_start,
-                   st.slots, st.n_seqs, H, G, d, dv)
+                   st.slots, st.n_seqs, H, G, d, dv, split=split)
     ops.conv_state_update(rows, C, tails, st.positions, st.q_start, st.slots, st.n_seqs)
     assert torch.all(out[st.n:] == 77.0)
     o, at, res = out.double().cpu().numpy(), 0, []
@@ -153,3 +155,23 @@ def test_a_broken_token_leaves_the_ones_before_it(t0, bad, monkeypatch):
             state, tails = torch.zeros((2, H, d, dv), device="cuda"), torch.zeros((2, 1, C), device="cuda")
             outs.append(step([p], [T], [0], H, G, d, dv, rank, w, tails, state, "float32", True, monkeypatch, [1])[0])
         assert np.array_equal(outs[0][:t0], outs[1][:t0]) and np.array_equal(outs[0][:, dv:], outs[1][:, dv:])
+
+
+def test_each_request_goes_by_its_own_portion(monkeypatch):
+    """Long portions beside single tokens and short ones: every request has the numbers of its own form."""
+    H, G, d, dv, rank = 2, 1, 64, 36, 0
+    lens = [1, 300, 1, 255, 256, 400, 2]
+    projs, w = [inputs(n, H, G, d, dv, rank, i, "slow")[0] for i, n in enumerate(lens)], inputs(1, H, G, d, dv, rank, 1, "slow")[1]
+    slots, outs, states, C = [3, 1, 4, 7, 5, 2, 6], [], [], 2 * G * d + H * dv
+    for chunks in (None, True, False):
+        state = torch.linspace(-1, 1, 8 * H * d * dv, device="cuda").view(8, H, d, dv).contiguous()
+        outs.append(step(projs, lens, [0] * 7, H, G, d, dv, rank, w, torch.zeros((8, 1, C), device="cuda"), state, "float32", chunks,
+                         monkeypatch, slots))
+        states.append(state)
+    for i, (n, s) in enumerate(zip(lens, slots)):
+        k = 1 if n >= 256 else 2
+        assert np.array_equal(outs[0][i], outs[k][i]) and torch.equal(states[0][s], states[k][s])
+    state = torch.linspace(-1, 1, 8 * H * d * dv, device="cuda").view(8, H, d, dv).contiguous()
+    lone = step(projs[5:6], [400], [0], H, G, d, dv, rank, w, torch.zeros((8, 1, C), device="cuda"), state, "float32", None,
+                monkeypatch, [2], pad=20)
+    assert np.array_equal(lone[0], outs[0][5]) and torch.equal(state[2], states[0][2])

@@ -21,19 +21,21 @@ def projections(T, H, d, dv, seed, gates):
 
 
 def scan(proj, lens, starts, H, d, dv, f_bias, lower, norm_w, state, dtype, chunks, monkeypatch, slots, pad=3):
-    """One step over the requests' next ``lens`` tokens from ``starts``; proj: per request.  -> rows per request."""
+    """One step over the requests' next ``lens`` tokens from ``starts``; proj: per request.  -> rows per request.
+    chunks: True all in chunks, False none, None each by its own portion."""
     from swifttransformer_b200 import ops
-    monkeypatch.setattr(ops, "HGRN2_CHUNK_MIN_TOKENS", 1 if chunks else 1 << 30)
+    monkeypatch.setattr(ops, "HGRN2_CHUNK_MIN_TOKENS", {True: 1, False: 1 << 30, None: 96}[chunks])
     st = Step([(s, a, n) for s, a, n in zip(slots, starts, lens)], pad_tokens=pad, pad_requests=2)
     rows = np.concatenate([p[a:a + n] for p, a, n in zip(proj, starts, lens)] + [np.full((pad, proj[0].shape[1]), 50.0)])
     rows = dev(rows, TD[dtype])
     out = torch.full((st.n_rows, H * dv), 77.0, dtype=TD[dtype], device="cuda")
     need = int(ops.lib().st_hgrn2_chunks_scratch(st.n_rows, st.n_seqs, H, d, dv))
     scratch = torch.full((max(need, st.n_rows * H * dv),), float("nan"), device="cuda")
+    split = ops.hgrn2_split(lens, st.n_rows, st.n_seqs, H, d) if chunks is None else None
     assert need > 0 and (not chunks or ops._hgrn2_chunks_apply(st.n_rows, st.n_seqs, H, d, dv, scratch, (rows.shape[1], 0, H * d, 2 * H * d),
                                                                (rows, out, state)))
     ops.hgrn2_scan(rows, 0, H * d, 2 * H * d, dev(f_bias), dev(lower), dev(norm_w), 1e-5, state, out, st.positions,
-                   st.q_start, st.slots, st.n_seqs, H, d, dv, scratch=scratch)
+                   st.q_start, st.slots, st.n_seqs, H, d, dv, scratch=scratch, split=split)
     assert torch.all(out[st.n:] == 77.0)
     o, at, res = out.double().cpu().numpy(), 0, []
     for n in lens:
@@ -104,3 +106,23 @@ def test_a_broken_token_leaves_the_ones_before_it(t0, bad, monkeypatch):
             state = torch.zeros((2, H, d, dv), device="cuda")
             outs.append(scan([q], [T], [0], H, d, dv, f_bias, lower, norm_w, state, "float32", True, monkeypatch, [1])[0])
         assert np.array_equal(outs[0][:t0], outs[1][:t0]) and np.array_equal(outs[0][:, dv:], outs[1][:, dv:])
+
+
+def test_each_request_goes_by_its_own_portion(monkeypatch):
+    """Long portions beside single tokens and short ones: every request has the numbers of its own form."""
+    H, d, dv = 2, 128, 36
+    lens = [1, 300, 1, 95, 96, 130, 1, 64]
+    data = [projections(n, H, d, dv, i, "slow") for i, n in enumerate(lens)]
+    proj, (f_bias, lower, norm_w) = [x[0] for x in data], data[0][1:]
+    slots, outs, states = [3, 1, 4, 8, 5, 2, 6, 7], [], []
+    for chunks in (None, True, False):
+        state = torch.linspace(-1, 1, 9 * H * d * dv, device="cuda").view(9, H, d, dv).contiguous()
+        outs.append(scan(proj, lens, [0] * 8, H, d, dv, f_bias, lower, norm_w, state, "float32", chunks, monkeypatch, slots))
+        states.append(state)
+    for i, (n, s) in enumerate(zip(lens, slots)):
+        k = 1 if n >= 96 else 2
+        assert np.array_equal(outs[0][i], outs[k][i]) and torch.equal(states[0][s], states[k][s])
+    # alone in its step, the long one has the same numbers
+    state = torch.linspace(-1, 1, 9 * H * d * dv, device="cuda").view(9, H, d, dv).contiguous()
+    lone = scan(proj[1:2], [300], [0], H, d, dv, f_bias, lower, norm_w, state, "float32", None, monkeypatch, [1], pad=20)
+    assert np.array_equal(lone[0], outs[0][1]) and torch.equal(state[1], states[0][1])

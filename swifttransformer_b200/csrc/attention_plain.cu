@@ -9,8 +9,8 @@
 // a fixed order, so the result for a position does not depend on how the
 // request was cut into steps or on what else is in the batch.
 //
-// Float storage with rows of whole 16-byte pieces goes to attention_f32_kernel (below), which gives the same bits; every
-// other size and bfloat16 storage to attention_plain_kernel.
+// Float storage with rows of whole 16-byte pieces goes to attention_f32_kernel and attention_f32_few_kernel (below), which give
+// the same bits; every other size and bfloat16 storage to attention_plain_kernel.
 //
 // Formulas: src/csrc/kernel/fused_decoding_stage_attention_mha.cu:159-252
 // (scores, softmax) and :254-318 (weighted sum of values); the prompt kernel
@@ -127,6 +127,7 @@ struct AttentionF32 {
     int n_tokens, max_pages, n_layers, layer, nh, nkv, d, page_size, window;
     float scale;
     int* status;
+    int n_seqs;
 };
 
 // the pool's row of key `key` of a request, -1: none (past the run's range, or a hole in the block table: reported)
@@ -140,12 +141,15 @@ __device__ __forceinline__ long long af_row(const AttentionF32& p, const int* bt
     return ((((long long)page * p.n_layers + p.layer) * 2) * p.nkv + kvh) * p.page_size + key % p.page_size;
 }
 
-// one token: threads are keys for the scores, dimensions for the values
+// one token: threads are keys for the scores, dimensions for the values.  A tile's values pass through GROUPS places of AF_SUB
+// rows: all of them at once (4), or two by two (2), which leaves room for more blocks on an SM
+template <int GROUPS>
 __device__ __forceinline__ void af_single(const AttentionF32& p, float* smem, long long* rows, float* scratch, int t, int h,
                                           int kvh, int pos, const int* bt) {
+    static_assert(KT / AF_SUB == 4 && (GROUPS == 2 || GROUPS == 4), "a tile is four groups of keys");
     const int d = p.d, tid = threadIdx.x;
-    float* sv = smem;                    // [KT][d] values of the tile
-    float* sq = smem + KT * d;           // [d] scaled query
+    float* sv = smem;                    // [GROUPS][AF_SUB][d] values of the tile
+    float* sq = smem + GROUPS * AF_SUB * d;     // [d] scaled query
     float* sp = sq + d;                  // [KT] weights
     const float* q = p.q + ((size_t)t * p.nh + h) * d;
     const int lo = p.window > 0 ? max(0, pos - p.window + 1) : 0, hi = pos + 1;
@@ -159,11 +163,21 @@ __device__ __forceinline__ void af_single(const AttentionF32& p, float* smem, lo
         rows[tid] = row;
         __syncthreads();                 // the rows' places; also: the tile before is done with the values' memory
         const int j_begin = max(0, lo - base), j_end = min(KT, hi - base);
-        for (int i = tid + j_begin * pieces; i < j_end * pieces; i += KT) {
-            const long long r = rows[i / pieces];
-            af_cp16(sv + i * 4, r >= 0 ? p.pool + r * d + v_off + (i % pieces) * 4 : p.pool, r >= 0);
+        auto copy = [&](float* dst, int a, int b) {      // the values of keys a .. b - 1
+            for (int i = tid + a * pieces; i < b * pieces; i += KT) {
+                const long long r = rows[i / pieces];
+                af_cp16(dst + i * 4, r >= 0 ? p.pool + r * d + v_off + (i % pieces) * 4 : p.pool, r >= 0);
+            }
+            af_commit();
+        };
+        auto group = [&](int g) { return sv + (g % GROUPS - g) * AF_SUB * d; };      // where key 0 would be
+        auto copy_group = [&](int g) { copy(group(g), max(j_begin, g * AF_SUB), min(j_end, (g + 1) * AF_SUB)); };
+        if constexpr (GROUPS == 4) {
+            copy(sv, j_begin, j_end);
+        } else {
+            copy_group(0);
+            copy_group(1);
         }
-        af_commit();
         float s = -INFINITY;
         if (row >= 0) {
             const float4* k = reinterpret_cast<const float4*>(p.pool + row * d);
@@ -182,25 +196,42 @@ __device__ __forceinline__ void af_single(const AttentionF32& p, float* smem, lo
         l = fmaf(l, corr, tile_sum);
         m = m_new;
         sp[tid] = w;
-        af_wait<0>();
-        __syncthreads();
+        auto add = [&](const float* v, int a, int b, float corr) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int e = tid + c * KT;
-            if (e < d) {
-                float a = acc[c] * corr;
-                int j = j_begin;
-                for (; j < j_end && (j & 3); ++j) a = fmaf(sp[j], sv[j * d + e], a);
+            for (int c = 0; c < 2; ++c) {
+                const int e = tid + c * KT;
+                if (e < d) {
+                    float x = acc[c] * corr;
+                    int j = a;
+                    for (; j < b && (j & 3); ++j) x = fmaf(sp[j], v[j * d + e], x);
 #pragma unroll 4
-                for (; j + 4 <= j_end; j += 4) {
-                    const float4 w4 = *reinterpret_cast<const float4*>(sp + j);
-                    a = fmaf(w4.x, sv[j * d + e], a);
-                    a = fmaf(w4.y, sv[(j + 1) * d + e], a);
-                    a = fmaf(w4.z, sv[(j + 2) * d + e], a);
-                    a = fmaf(w4.w, sv[(j + 3) * d + e], a);
+                    for (; j + 4 <= b; j += 4) {
+                        const float4 w4 = *reinterpret_cast<const float4*>(sp + j);
+                        x = fmaf(w4.x, v[j * d + e], x);
+                        x = fmaf(w4.y, v[(j + 1) * d + e], x);
+                        x = fmaf(w4.z, v[(j + 2) * d + e], x);
+                        x = fmaf(w4.w, v[(j + 3) * d + e], x);
+                    }
+                    for (; j < b; ++j) x = fmaf(sp[j], v[j * d + e], x);
+                    acc[c] = x;
                 }
-                for (; j < j_end; ++j) a = fmaf(sp[j], sv[j * d + e], a);
-                acc[c] = a;
+            }
+        };
+        if constexpr (GROUPS == 4) {
+            af_wait<0>();
+            __syncthreads();
+            add(sv, j_begin, j_end, corr);
+        } else {
+            for (int g = 0; g < 4; ++g) {
+                af_wait<1>();            // of two groups under way the first has landed
+                __syncthreads();
+                add(group(g), max(j_begin, g * AF_SUB), min(j_end, (g + 1) * AF_SUB), g == 0 ? corr : 1.f);
+                if (g < 2 && (g + 2) * AF_SUB < j_end) {
+                    __syncthreads();     // everyone is done with the group whose place is filled next
+                    copy_group(g + 2);
+                } else {
+                    af_commit();
+                }
             }
         }
     }
@@ -210,6 +241,19 @@ __device__ __forceinline__ void af_single(const AttentionF32& p, float* smem, lo
         if (e < d) p.out[((size_t)t * p.nh + h) * d + e] = acc[c] * inv;
     }
     __syncthreads();                     // shared memory is free for the next run
+}
+
+// Steps of few tokens (af_few): a block per (token, head), whatever runs there are.  At most 2 x 32 value rows in shared memory, so that
+// many blocks share an SM; a tile of 32 query rows, or a tile's values at once, leave room for two at 128 dimensions.
+__global__ void __launch_bounds__(KT, 8)
+attention_f32_few_kernel(const AttentionF32 p) {
+    extern __shared__ __align__(16) float smem[];
+    __shared__ long long rows[KT];
+    __shared__ float scratch[32];
+    const int h = blockIdx.x % p.nh, t = p.n_tokens - 1 - blockIdx.x / p.nh;
+    const int pos = p.positions[t];
+    if (pos < 0) return;
+    af_single<2>(p, smem, rows, scratch, t, h, h / (p.nh / p.nkv), pos, p.block_table + (size_t)p.slots[p.seq_of_token[t]] * p.max_pages);
 }
 
 // n tokens t0 .. t0 + n - 1 at positions pos0 .. pos0 + n - 1; NI: 64-wide blocks of dimensions
@@ -442,9 +486,22 @@ attention_f32_kernel(const AttentionF32 p) {
         if (k % gridDim.z != blockIdx.z) continue;
         const int pos0 = __shfl_sync(0xffffffffu, pos, at), s0 = __shfl_sync(0xffffffffu, seq, at);
         const int* bt = p.block_table + (size_t)p.slots[s0] * p.max_pages;
-        if (stop - at == 1) af_single(p, smem, rows, scratch, first + at, h, kvh, pos0, bt);
+        if (stop - at == 1) af_single<KT / AF_SUB>(p, smem, rows, scratch, first + at, h, kvh, pos0, bt);
         else af_tile<NI>(p, smem, rows, scratch, first + at, stop - at, h, kvh, pos0, bt);
     }
+}
+
+// Whether every token of the step is a block's of its own: (token, head) pairs per multiprocessor times tokens per request up to
+// 30000 / dimensions.  A tile reads its keys once for all its rows but takes as long for two tokens as for 32, and its shared
+// memory leaves room for four, two or one block per SM (64, 128, 256 dimensions).  us on one B200, tiles / tokens (general kernel),
+// 32 heads: 64 dimensions, one request of 16 tokens at 0 / 100 / 1000 earlier ones 20 / 10 (20), 33 / 16 (88), 199 / 84 (653);
+// 4 requests of 16 20 / 16 (27), 47 / 35, 293 / 230; 4 of 32 25 / 27 (57), 47 / 61, 285 / 385; 128 dimensions, 16 of 4 37 / 22
+// (20), 88 / 64, 698 / 473; 16 of 8 45 / 35 (35), 121 / 108, 813 / 883; one of 64 behind 1000 291 / 447; 256 dimensions, 16 heads,
+// 16 of 4 45 / 31 (27), 4 of 32 41 / 55 (102).  Steps of single tokens stay with the tiles' kernel, whose values arrive at once.
+static bool af_few(const AttentionF32& p) {
+    if (p.n_seqs <= 0 || p.n_tokens <= p.n_seqs) return false;
+    const int limit = 30000 / (p.d > 64 ? p.d : 64);
+    return (double)p.n_tokens * p.nh * p.n_tokens <= (double)limit * st_sm_count() * p.n_seqs;
 }
 
 static int attention_f32(const AttentionF32& p, cudaStream_t s) {
@@ -458,6 +515,13 @@ static int attention_f32(const AttentionF32& p, cudaStream_t s) {
     if (z > p.n_tokens) z = p.n_tokens;
     if (have > 0x7fffffffLL) return ST_ERR_TOO_LARGE;
     dim3 grid((unsigned)have, 1, z);
+    if (af_few(p)) {
+        const size_t few = sizeof(float) * (2 * AF_SUB * p.d + p.d + KT);
+        const cudaError_t e = cudaFuncSetAttribute(attention_f32_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few);
+        if (e != cudaSuccess) return (int)e;
+        attention_f32_few_kernel<<<p.n_tokens * p.nh, KT, few, s>>>(p);
+        return st_launch_status();
+    }
 #define AF_LAUNCH(NI)                                                                                                  \
     do {                                                                                                               \
         const cudaError_t e = cudaFuncSetAttribute(attention_f32_kernel<NI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
@@ -474,14 +538,14 @@ static int attention_f32(const AttentionF32& p, cudaStream_t s) {
 ST_EXPORT int st_attention_plain(const void* q, const void* pool, void* out, const int* positions,
                                  const int* seq_of_token, const int* slots, const int* block_table, int max_pages,
                                  int n_layers, int layer, int n_tokens, int nh, int nkv, int d, int page_size,
-                                 float scale, int window, int dtype, int* status, void* stream) {
+                                 float scale, int window, int dtype, int* status, void* stream, int n_seqs) {
     if (n_tokens <= 0) return 0;
     if (nh <= 0 || nkv <= 0 || nh % nkv || d <= 0 || page_size <= 0) return ST_ERR_BAD_ARG;
     if (d > 2 * KT) return ST_ERR_TOO_LARGE;
     cudaStream_t s = (cudaStream_t)stream;
     if (dtype == 0 && d % 4 == 0 && aligned16(q) && aligned16(pool) && aligned16(out) && nh <= 65535)
         return attention_f32({(const float*)q, (const float*)pool, (float*)out, positions, seq_of_token, slots, block_table,
-                              n_tokens, max_pages, n_layers, layer, nh, nkv, d, page_size, window, scale, status}, s);
+                              n_tokens, max_pages, n_layers, layer, nh, nkv, d, page_size, window, scale, status, n_seqs}, s);
     dim3 grid(n_tokens, nh);
     const size_t smem = (size_t)(d + KT) * sizeof(float);
     if (dtype == 0)

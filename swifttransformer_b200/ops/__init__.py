@@ -496,7 +496,7 @@ def attention_plain(q: torch.Tensor, pool: torch.Tensor, layer: int, out: torch.
     _, n_layers, _, nkv, page_size, d = pool.shape
     _check(lib().st_attention_plain(_p(q), _p(pool), _p(out), _p(positions), _p(seq_of_token), _p(slots),
                                     _p(block_table), block_table.shape[1], n_layers, layer, n, nh, nkv, d,
-                                    page_size, _f(scale), window, _dt(q), _p(status), _stream()), "attention_plain")
+                                    page_size, _f(scale), window, _dt(q), _p(status), _stream(), slots.numel()), "attention_plain")
     return out
 
 

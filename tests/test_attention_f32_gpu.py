@@ -49,13 +49,17 @@ def both(q, pool, layer, args, heads, window):
     return out, ref, status.tolist()
 
 
-# runs of one token, of a tile of 32 and its edges, several in a tile, starting and ending at the edges of 32 and 128 keys
+# runs of one token, of a tile of 32 and its edges, several in a tile, starting and ending at the edges of 32 and 128 keys, and
+# of a few tokens
 RUNS = [[(0, 0, 1)], [(0, 0, 300)], [(0, 127, 1), (1, 128, 1), (2, 700, 1), (3, 0, 1)], [(1, 0, 31), (0, 0, 33), (2, 95, 64)],
-        [(0, 100, 2), (1, 0, 1), (2, 126, 5), (3, 255, 30), (4, 31, 1)], [(i, 3 * i, 1) for i in range(70)], [(0, 380, 129)]]
+        [(0, 100, 2), (1, 0, 1), (2, 126, 5), (3, 255, 30), (4, 31, 1)], [(i, 3 * i, 1) for i in range(70)], [(0, 380, 129)],
+        [(0, 120, 8), (1, 124, 9), (2, 0, 8), (3, 0, 9), (4, 500, 10), (5, 0, 3)]]
 
 
+# (few heads: a block per token and head; with 256 of them most steps go by tiles of 32 rows)
 @pytest.mark.parametrize("heads,kv_heads,dim,page_size", [(2, 2, 64, 16), (4, 2, 128, 8), (3, 3, 80, 7), (2, 1, 4, 16), (1, 1, 256, 32),
-                                                          (2, 2, 132, 1), (1, 1, 20, 16)])
+                                                          (2, 2, 132, 1), (1, 1, 20, 16), (256, 2, 64, 16), (256, 2, 128, 8),
+                                                          (256, 1, 132, 7), (256, 1, 256, 32)])
 @pytest.mark.parametrize("window", [0, 50, 128, 400])
 def test_same_bits_as_the_general_kernel(heads, kv_heads, dim, page_size, window):
     for k, runs in enumerate(RUNS):

@@ -22,8 +22,8 @@
 // Bound by the tensor cores for prompts and by the weights' way from memory for few rows.  Measured on one B200 (with about
 // 6 us of an empty launch between events, inputs not in cache; in brackets the mma.sync kernel with tiles of 64 x 64):
 // 4000 items, 8 experts, 2048 -> 5504: 109 us = 880 TFLOP/s (481); 2752 -> 2048: 55 us = 920 TFLOP/s (252).  300 tokens x 2,
-// 8 experts, gated 4096 -> 1024: 55 us (107).  38 items, 16 experts, 2048 -> 5504: 84 us, 361 MB = 4.6 TB/s (129).  16 items, 8
-// experts, gated 2048 -> 512: 29 us (37).
+// 8 experts, gated 4096 -> 1024: 45 us (107).  38 items, 16 experts, 2048 -> 5504: 84 us, 361 MB = 4.6 TB/s (129).  16 items, 8
+// experts, gated 2048 -> 512: 23 us (37).
 //
 // Waits are bounded: one that expires marks the block dead, `status` gets 5, and the block waits (again with a limit) for its
 // copies under way, frees its tensor memory and leaves.
@@ -141,7 +141,9 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
                      ::"r"(tc_smem(&s_tmem)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
     }
+    __syncthreads();
     ST_PDL_WAIT();
+    ST_PDL_TRIGGER();                                         // behind the allocation
     if (warp == 0) {
         int run = 0;
         for (int e0 = 0; e0 < sh.n_experts; e0 += 32) {
@@ -162,7 +164,6 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
     tc_fence_before_sync();
     __syncthreads();
     tc_fence_after_sync();
-    ST_PDL_TRIGGER();
     const uint32_t tmem = s_tmem;
     const int bn_out = sh.gated ? BN / 2 : BN;
     const int n_tiles_n = (sh.n_out + bn_out - 1) / bn_out;
@@ -317,15 +318,15 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
 
 // The rows of w in a tile (gated tiles count their gate and up rows).  The wider, the less a is read again; a launch has at
 // least a row tile per expert that any item may go to.  Lines by measurement (us with 64 / 128 / 256 rows): the widest while
-// every SM gets a tile (4000 items, 5504 rows: 256 / 156 / 109), then 128 while half of the SMs do (600 items on 8 experts, 2048
-// gate and up rows: 65 / 55 / 76; 300 items on 16 experts, 1024: 37 / 31 / 39; 16 items on 8, 2048: 16.4 / 14.4 / 16.4), else 64
-// (16 items on 8, 1024: 31 / 27 / 35, where the widths are as far apart as two runs of one are).
+// every SM gets a tile (4000 items, 5504 rows: 254 / 152 / 102), then 128 while half of the SMs do (600 items on 8 experts, 2048
+// gate and up rows: 59 / 45 / 53; 256 items on 16 experts, 1024: 25 / 21 / 25; 16 items on 8, 2048: 16 / 14 / 18; but 16 on 16, 1024
+// of k = 512: 14.3 / 16.4 / 20.5), else 64 (16 items on 8, 1024: 23 / 25 / 29).  Over 650 products of 8 to 128 experts the choice is 2 %
+// behind the best width on average; counting only the experts that items are likely to hit, or the rounds of tiles, gained nothing.
 static int ge_pick_bn(int n_items, int n_experts, int w_rows, int sms) {
-    const double hit = n_experts * (1. - exp(-(double)n_items / n_experts));      // experts that get an item, if they get them evenly
     int row_tiles = (n_items + GE_BM - 1) / GE_BM;
-    if (row_tiles < hit) row_tiles = (int)hit;
+    if (row_tiles < n_experts) row_tiles = n_items < n_experts ? n_items : n_experts;
     auto tiles = [&](int bn) { return (long long)row_tiles * ((w_rows + bn - 1) / bn); };
-    return tiles(256) >= sms ? 256 : 5 * tiles(128) >= 3 * sms ? 128 : 64;
+    return tiles(256) >= sms ? 256 : 2 * tiles(128) >= sms ? 128 : 64;
 }
 
 template <int BN, bool GATHER>

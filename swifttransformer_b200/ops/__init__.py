@@ -1316,14 +1316,16 @@ def gemm_experts(a: torch.Tensor, w: torch.Tensor, order: ExpertOrder, gather: b
     w [experts, n_out (twice with ``gated``: gate rows, then up rows), k]; out = act(product), gated: act(gate) * up.
     bfloat16 with k a multiple of 8: the tcgen05 kernel (a wait that expires inside it shows in ``kernel_status``), for small
     products the mma.sync one; else the plain one."""
-    assert a.is_contiguous() and w.is_contiguous() and w.dim() == 3 and a.dtype == w.dtype and a.shape[1] == w.shape[2]
-    n_out = w.shape[1] // 2 if gated else w.shape[1]
+    assert a.is_contiguous() and w.is_contiguous() and w.dim() == 3 and a.dtype == w.dtype
+    E, w_rows, k = w.shape
+    n_rows, a_k = a.shape
+    assert a_k == k
+    n_out = w_rows // 2 if gated else w_rows
     out = a.new_empty((order.n_items, n_out))
     ll = ctypes.c_longlong
-    E, w_rows, k = w.shape
     if (not _experts_mma(order.n_items, E, w_rows, k) and GROUPED_MMA and a.dtype == torch.bfloat16
             and bool(lib().st_gemm_experts_tc_applies(E, k))):
-        _check(lib().st_gemm_experts_tc(_p(a), ll(a.shape[0]), _p(w), _p(out), E, order.n_items, n_out, k, int(gated), ACT_CODES[act],
+        _check(lib().st_gemm_experts_tc(_p(a), ll(n_rows), _p(w), _p(out), E, order.n_items, n_out, k, int(gated), ACT_CODES[act],
                                         _p(order.offsets), _p(order.sorted) if gather else None, order.top if gather else 1,
                                         EXPERTS_TILE, _p(_tc_status_word(a.device)), _stream()), "gemm_experts")
         return out

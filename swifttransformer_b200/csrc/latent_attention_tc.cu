@@ -15,10 +15,12 @@
 //            operand of O += P V; the reference moves, and O is rescaled, only when a row's maximum has grown by 2^8
 // At the end the sink joins the denominator, the gate multiplies, and the row is stored.
 //
-// Measured on one B200, 16 heads, kr 512, rot 64, pages of 16: two prompts of 1000 tokens 168 us (mma.sync kernel 251; 172
-// while the launch walked all tiles once per 256 value columns), one of 700 58 (86), 450 tokens behind 1200 120 (184).  A tile of 64 keys takes about 7300 clocks: 2000 for the key-only blocks' copies
-// (under the softmax of the tile before), 1500 more for the values', 2100 for the scores on them: a product of 64 columns
-// takes as long as one of 256, about 130 clocks per 16 dimensions, for its rows of the query tile are read each time.
+// Measured on one B200, 16 heads, kr 512, rot 64, pages of 16: two prompts of 1000 tokens 171 us (mma.sync kernel 251; 168
+// without the rows cleared in a block's last tile), one of 700 58 (86), 450 tokens behind 1200 120 (184).  A tile of 64 keys
+// takes about 7300 clocks (by clock stamps in a copy of the kernel, profiles/latent_attention_tc_clocks.md): 2050 for the
+// key-only blocks' copies (under the softmax of the tile before), 2900 for the values', 2150 for the scores on them, 1400 for
+// the softmax: a product of 64 columns takes as long as one of 256, about 130 clocks per 16 dimensions, for its rows of the
+// query tile are read each time.
 //
 // Waits are bounded: one that expires marks the block dead, `status` gets 6, and the block waits (again with a limit) for its
 // copies under way, frees its tensor memory and leaves.
@@ -254,11 +256,11 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __gr
                 // finite is not zero.  The boxes have landed (the scores are complete), and the next ones wait for O += P V.
                 lt_wait(tc_smem(&s_full[1]), i & 1, dead);
                 const int head = min(max(lo - k0, 0), LT_KEYS), tail = max(min(hi - k0, LT_KEYS), head);
-                const int n_dead = head + LT_KEYS - tail;
-                for (int c = tid; c < n_dead * nv * 8; c += LT_ROWS) {
-                    const int d = c / (nv * 8), key = d < head ? d : tail + d - head, piece = c % (nv * 8);
-                    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n"
-                                 ::"r"(sK + (v0 + piece / 8) * LT_K_BLK + key * 128 + piece % 8 * 16), "r"(0) : "memory");
+                if (lane < nv * 8) {                          // a lane per 16 bytes of a row's values (nv <= 4), a warp per row
+                    const uint32_t at = sK + (v0 + lane / 8) * LT_K_BLK + lane % 8 * 16;
+                    for (int key = warp; key < LT_KEYS; key += 4)
+                        if (key < head || key >= tail)
+                            asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};\n" ::"r"(at + key * 128), "r"(0) : "memory");
                 }
                 tc_fence_async_smem();
             }

@@ -12,7 +12,7 @@
 // step.  A request's chunks have the places hk_place + 0, 1, ..: no two requests' overlap (a portion of `from` tokens and more
 // moves both terms on), and hk_places hold all L = min(n_seqs, n / from) of them.
 __host__ __device__ __forceinline__ int hk_place(int begin, int b, int from) {
-    return begin / HK_C + (b < begin / from ? b : begin / from);
+    return begin / HK_C + (b == 0 ? 0 : b < begin / from ? b : begin / from);
 }
 static inline long long hk_places(int n_tokens, int L) { return ((long long)n_tokens + HK_C - 1) / HK_C + L - 1; }
 static inline int hk_longs(int n_tokens, int n_seqs, int from) { return n_seqs < n_tokens / from ? n_seqs : n_tokens / from; }

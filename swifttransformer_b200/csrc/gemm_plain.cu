@@ -226,8 +226,8 @@ static int gemm_f32_launch(const float* a, const float* w, const float* bias, fl
 // Which tile.  Measured on one B200, times with the 6 us of an empty launch between events, L2 flushed; in brackets what the
 // kernel of 64 x 64 tiles with 4 x 4 outputs per thread took, which served every size before.
 //   up to 8 rows: bound by the weights' way from memory (and below that by the chain: four clocks per multiply-add, so
-//     k = 4096 takes 8.4 us however the work is spread).  Tiles as narrow as the rows; 512 bytes to 1 KB of a row per
-//     stage and eight stages keep 32 to 80 KB per SM under way.  8 x 4096 x 4096 29.7 us, 67 MB (455); with 16 or 32
+//     k = 4096 takes 8.4 us however the work is spread).  Tiles as narrow as the rows; 256 or 512 bytes of a row per stage
+//     and eight or six stages keep 35 to 100 KB per block under way.  8 x 4096 x 4096 29.7 us, 67 MB (455); with 16 or 32
 //     outputs per block, whichever gives the SMs a block each: 1 x 2048 x 2048 14 us with 16; and where there are three
 //     halves of a block of 32 per SM two warps of 2 x 2 outputs pull more weights per instruction: 8 x 2048 x 8192 26.6 us
 //     (30.8 with four warps of 2 x 1), 8 x 2048 x 50272 106 us = 4.1 TB/s (119)

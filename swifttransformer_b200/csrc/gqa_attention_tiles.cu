@@ -30,7 +30,11 @@
 // as often and runs the longest rows' chain with fewer warps beside it.  us with 64 / 128 rows, 16 heads on 4, window 512 and
 // all keys, 2000 tokens: dim 64, vd 128: 49 / 66, 99 / 84 (8000 tokens: 184 / 213, 903 / 1039; 32 heads: 88 / 100, 148 / 160;
 // 4 heads: 31 / 37, 72 / 80); dim 64, vd 64: 39 / 55, 84 / 70; dim 128, vd 128: 66 / 76, 127 / 97; dim 128, vd 256: 100 / 100,
-// 141 / 131.
+// 141 / 131.  The line takes the better side of most of these, not of all: over all keys, 2000 tokens of 16 heads of dim 64
+// are 17 to 20 % faster with 128 rows (with more tokens, more heads or fewer 64 are ahead again), and under the window heads of
+// 128 x 128 are 15 % faster with 64; window and blocks per wave would have to be in the rule.  No size is slower than before
+// there was a choice (72 and 131 for the first, 84 and 156 for dim 128).  At 168 registers the 64-row instances spill 12 to 36
+// bytes a thread.
 #define GT_BLOCK_ROWS(DIMT, VDT) ((DIMT) <= 64 && (VDT) <= 128 ? 64 : 128)
 
 template <int DIMT, int VDT>

@@ -18,8 +18,8 @@
 // Measured on one B200, 16 heads, kr 512, rot 64, pages of 16: two prompts of 1000 tokens 171 us (mma.sync kernel 251; 168
 // without the rows cleared in a block's last tile), one of 700 58 (86), 450 tokens behind 1200 120 (184).  A tile of 64 keys
 // takes about 7300 clocks (by clock stamps in a copy of the kernel): 2050 for the key-only blocks' copies (under the softmax of
-// the tile before), 2900 for the values', 2150 for the scores on them, 1400 for the softmax: a product of 64 columns takes as long as one of 256, about 130 clocks per 16 dimensions, for its rows of the
-// query tile are read each time.
+// the tile before), 2900 for the values', 2150 for the scores on them, 1400 for the softmax: a product of 64 columns takes as
+// long as one of 256, about 130 clocks per 16 dimensions, for its rows of the query tile are read each time.
 //
 // Waits are bounded: one that expires marks the block dead, `status` gets 6, and the block waits (again with a limit) for its
 // copies under way, frees its tensor memory and leaves.

@@ -1,0 +1,62 @@
+// The 32-bit matrix product on the tensor cores, out[n, m] = act( sum_k a[n,k] * w[m,k] + bias[m] ) with float operands and
+// w stored [out, in]: what its kernels (gemm_f32_tc.cu for many rows, gemm_f32_few.cu for few) share.
+//
+// A float is the sum of three bfloat16 numbers of eight bits each: x = h + m + l, h = bf16(x), m = bf16(x - h),
+// l = bf16(x - h - m), each difference exact.  Of the nine products of two such sums six are formed,
+//   w_l a_h + w_h a_l + w_m a_m + w_m a_h + w_h a_m + w_h a_h,
+// each exact in the tensor cores' float accumulator; the three left out are at most 2^-25 of w a together.  The tensor
+// cores cut a sum off where a float addition rounds it (measured: 6e-8 of bias after four steps of 16 k, 1.2e-7 after eight), so a sum
+// stays there for one group of 64 k only, the small products first: its 24 steps end with the four of w_h a_h.  The
+// groups' sums are added up in float registers in ascending order, each addition rounded to nearest.  An output so
+// depends on its own row of a and of w alone, and its bits are the same for every number of rows, tile and kernel: all form the
+// same groups and add them in the same order (mma.sync and tcgen05.mma give the same bits for the same sixteen products; a test
+// holds the kernels to it).
+//
+// An output that comes out infinite or not a number (operands that are, sums that overflow, operands within 2^-8 of the largest
+// float) is computed again as a chain of fused multiply-adds over k, which is what such operands give in plain float.
+// Below 2^-110 in magnitude a number's last bits fall under bfloat16's smallest (2^-133).
+//
+// Error against 64 bits, relative 2-norm, normal operands: k = 512 9.6e-8, 2048 1.3e-7, 8192 2.2e-7 (a chain of fused multiply-adds
+// over k: 4.0e-7, 8.1e-7, 1.6e-6).
+#pragma once
+#include "common.cuh"
+
+#define GF_BK 64             // k of a group
+
+// what two bfloat16 numbers leave of two floats
+__device__ __forceinline__ void gf_rest(float& x0, float& x1, uint32_t packed) {
+    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tsub.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}\n"
+        : "+f"(x0), "+f"(x1) : "f"(__uint_as_float(packed << 16)), "f"(__uint_as_float(packed & 0xffff0000u)));
+}
+// two neighbours -> their three parts, packed
+__device__ __forceinline__ void gf_split(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
+    const __nv_bfloat162 hb = __floats2bfloat162_rn(x0, x1);
+    h = *reinterpret_cast<const uint32_t*>(&hb);
+    gf_rest(x0, x1, h);
+    const __nv_bfloat162 mb = __floats2bfloat162_rn(x0, x1);
+    m = *reinterpret_cast<const uint32_t*>(&mb);
+    gf_rest(x0, x1, m);
+    const __nv_bfloat162 lb = __floats2bfloat162_rn(x0, x1);
+    l = *reinterpret_cast<const uint32_t*>(&lb);
+}
+
+struct GemmF32 {
+    const float *a, *w, *bias;
+    float* out;
+    int n_rows, n_out, k_dim, act;
+};
+__device__ __noinline__ inline float gf_chain(const float* a, const float* w, int k_dim) {
+    float s = 0.f;
+    for (int k = 0; k < k_dim; ++k) s = fmaf(a[k], w[k], s);
+    return s;
+}
+// bias, activation and store of one output; a sum that is not finite gives way to the chain
+__device__ __forceinline__ void gf_store(const GemmF32& p, int row, int col, float v, float bias) {
+    if (!(fabsf(v) < INFINITY)) v = gf_chain(p.a + (size_t)row * p.k_dim, p.w + (size_t)col * p.k_dim, p.k_dim);
+    p.out[(size_t)row * p.n_out + col] = apply_act(p.bias ? v + bias : v, p.act);
+}
+
+// gemm_f32_few.cu: for up to 8 rows, or in tiles of 16
+#define GF_FEW_ROWS 8
+#define GF_FEW_MOST 32       // more rows than this it is not asked to take
+int gf_few_launch(const GemmF32& p, cudaStream_t s);

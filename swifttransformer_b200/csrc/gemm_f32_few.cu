@@ -1,0 +1,161 @@
+// The 32-bit matrix product for few rows (decode steps): see gemm_f32.cuh for the arithmetic.
+//
+// A step is bound by w's way from memory.  A tile is 16 rows of w and up to 8 or 16 of a, so that there are tiles for every SM; blocks walk through the
+// tiles, and their warps take every WARPS-th group of 64 k each.  A warp copies its groups of w and a by 16-byte asynchronous
+// copies into a ring of its own (64 KB of w under way per block, on into the next tile) and reads them back as
+// fragments of mma.sync: a lane takes the four neighbours 4 t .. 4 t + 3 of rows g and g + 8 per step of 16 k, so a step's sixteen
+// products are those of sixteen k in another order, which changes no bit.  The groups' sums meet in shared memory (two
+// rounds of them, so that one is added up while the next is written), where they are added up in ascending order.
+//
+// us on one B200 with 6 us of an empty launch between events, inputs not in cache, in brackets chains of float multiply-adds:
+// 1 x 2048 x 2048 12.3 (14.3), 8 x 4096 x 4096 24.6, 67 MB (29), 4 x 8192 x 2048 27.5 (34.8), 8 x 2048 x 50272 99, 412 MB (106);
+// 16 x 2048 x 2048 14.3 (18.4), 16 x 8192 x 2048 36 (51).
+#include "gemm_f32.cuh"
+#include "mma_sync.cuh"
+
+// NB: blocks of eight rows of a
+template <int NB>
+struct GemmFew {
+    static constexpr int WARPS = NB == 1 ? 8 : 10, STAGES = 2;
+    static constexpr int ROUND = 2 * WARPS;                  // groups whose sums are added up at a time
+    static constexpr int ROWS = 16 + 8 * NB;                 // of a stage: w's, then a's, 256 bytes each
+    static constexpr size_t SMEM = (size_t)WARPS * STAGES * ROWS * 256 + (size_t)2 * ROUND * NB * 128 * 4;
+};
+
+// 16-byte piece c of row r of a stage: odd rows turned by four pieces, so that the rows of a read's quarter hit distinct banks
+__device__ __forceinline__ int gq_at(int r, int c) { return r * 64 + ((c ^ ((r & 1) << 2)) << 2); }
+
+template <int NB>
+__global__ void __launch_bounds__(32 * GemmFew<NB>::WARPS, NB == 1 ? 2 : 1)
+gemm_f32_few_kernel(const GemmF32 p, int tiles, int row_tiles, int vec_a, int vec_w) {
+    using S = GemmFew<NB>;
+    extern __shared__ __align__(16) float gq_smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    float* ring = gq_smem + warp * S::STAGES * S::ROWS * 64;
+    float* sums = gq_smem + S::WARPS * S::STAGES * S::ROWS * 64;             // [round's parity][group][NB][row of a][row of w]
+    const int n_groups = (p.k_dim + GF_BK - 1) / GF_BK;
+    auto copy = [&](int tile, int group, int stage) {
+        const int c = lane & 15, k = group * GF_BK + 4 * c, m0 = tile / row_tiles * 16, n0 = tile % row_tiles * (8 * NB);
+        float* dst = ring + stage * S::ROWS * 64;
+#pragma unroll
+        for (int i = 0; i < S::ROWS / 2; ++i) {
+            const int r = 2 * i + (lane >> 4);
+            const bool is_w = i < 8;
+            const int row = is_w ? m0 + r : n0 + r - 16, rows = is_w ? p.n_out : p.n_rows;
+            const float* src = (is_w ? p.w : p.a) + (size_t)(row < rows ? row : 0) * p.k_dim + k;
+            float* at = dst + gq_at(r, c);
+            if (is_w ? vec_w : vec_a) {
+                const bool on = row < rows && k < p.k_dim;
+                cp_async16(at, on ? src : is_w ? p.w : p.a, on);
+            } else {
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (row < rows) {
+                    if (k < p.k_dim) v.x = __ldg(src);
+                    if (k + 1 < p.k_dim) v.y = __ldg(src + 1);
+                    if (k + 2 < p.k_dim) v.z = __ldg(src + 2);
+                    if (k + 3 < p.k_dim) v.w = __ldg(src + 3);
+                }
+                store4(at, v);
+            }
+        }
+    };
+    int next_tile = warp < n_groups ? (int)blockIdx.x : tiles, next_group = warp;          // what this warp copies next
+    auto fetch = [&](int stage) {
+        if (next_tile < tiles) {
+            copy(next_tile, next_group, stage);
+            next_group += S::WARPS;
+            if (next_group >= n_groups) { next_group = warp; next_tile += gridDim.x; }
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int s = 0; s < S::STAGES; ++s) fetch(s);
+    int stage = 0, parity = 0;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        float total[NB];                                     // outputs tid of 128, block by block of rows (the first 128 threads)
+#pragma unroll
+        for (int b = 0; b < NB; ++b) total[b] = 0.f;
+        for (int round = 0; round < n_groups; round += S::ROUND, parity ^= 1) {
+            const int end = min(n_groups, round + S::ROUND);
+            float* part = sums + parity * S::ROUND * NB * 128;
+            for (int group = round + warp; group < end; group += S::WARPS) {
+                cp_async_wait<S::STAGES - 1>();
+                __syncwarp();
+                const float* src = ring + stage * S::ROWS * 64;
+                uint32_t wh[4][4], wm[4][4], wl[4][4];       // [step of 16 k][fragment register]
+                uint32_t ah[NB][4][2], am[NB][4][2], al[NB][4][2];
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const float4 v = load4(src + gq_at(g + 8 * r, 4 * kk + t));
+                        gf_split(v.x, v.y, wh[kk][r], wm[kk][r], wl[kk][r]);
+                        gf_split(v.z, v.w, wh[kk][2 + r], wm[kk][2 + r], wl[kk][2 + r]);
+                    }
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        const float4 v = load4(src + gq_at(16 + 8 * b + g, 4 * kk + t));
+                        gf_split(v.x, v.y, ah[b][kk][0], am[b][kk][0], al[b][kk][0]);
+                        gf_split(v.z, v.w, ah[b][kk][1], am[b][kk][1], al[b][kk][1]);
+                    }
+                }
+                __syncwarp();
+                fetch(stage);                                // the stage is read: the group but one takes its place
+                float c[NB][4];
+#pragma unroll
+                for (int b = 0; b < NB; ++b) c[b][0] = c[b][1] = c[b][2] = c[b][3] = 0.f;
+#define GQ_PRODUCT(W, A)                                                                                   \
+    _Pragma("unroll") for (int kk = 0; kk < 4; ++kk)                                                       \
+        _Pragma("unroll") for (int b = 0; b < NB; ++b) mma_bf16(c[b], W[kk], A[b][kk][0], A[b][kk][1])
+                GQ_PRODUCT(wl, ah);
+                GQ_PRODUCT(wh, al);
+                GQ_PRODUCT(wm, am);
+                GQ_PRODUCT(wm, ah);
+                GQ_PRODUCT(wh, am);
+                GQ_PRODUCT(wh, ah);
+#undef GQ_PRODUCT
+#pragma unroll
+                for (int b = 0; b < NB; ++b) {
+                    float* dst = part + ((group - round) * NB + b) * 128;
+                    dst[2 * t * 16 + g] = c[b][0];
+                    dst[(2 * t + 1) * 16 + g] = c[b][1];
+                    dst[2 * t * 16 + g + 8] = c[b][2];
+                    dst[(2 * t + 1) * 16 + g + 8] = c[b][3];
+                }
+                if (++stage == S::STAGES) stage = 0;
+            }
+            __syncthreads();                                 // (a round further on the same place is written again: behind the next one)
+            if (tid < 128) {
+#pragma unroll
+                for (int b = 0; b < NB; ++b)
+#pragma unroll 16
+                    for (int i = 0; i < end - round; ++i) total[b] += part[(i * NB + b) * 128 + tid];
+            }
+        }
+        const int col = tile / row_tiles * 16 + (tid & 15), n0 = tile % row_tiles * (8 * NB);
+        if (tid < 128 && col < p.n_out) {
+            const float bias = p.bias ? __ldg(p.bias + col) : 0.f;
+#pragma unroll
+            for (int b = 0; b < NB; ++b) {
+                const int row = n0 + 8 * b + (tid >> 4);
+                if (row < p.n_rows) gf_store(p, row, col, total[b], bias);
+            }
+        }
+    }
+    cp_async_wait<0>();
+}
+
+template <int NB>
+static int gq_launch(const GemmF32& p, cudaStream_t s) {
+    using S = GemmFew<NB>;
+    const int vec_a = p.k_dim % 4 == 0 && aligned16(p.a), vec_w = p.k_dim % 4 == 0 && aligned16(p.w);
+    const cudaError_t e = cudaFuncSetAttribute(gemm_f32_few_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    const int row_tiles = (p.n_rows + 8 * NB - 1) / (8 * NB);
+    const long long all = ((long long)p.n_out + 15) / 16 * row_tiles;
+    if (all > 0x3fffffffLL) return ST_ERR_TOO_LARGE;
+    const int tiles = (int)all, most = (NB == 1 ? 2 : 1) * st_sm_count();
+    gemm_f32_few_kernel<NB><<<tiles < most ? tiles : most, 32 * S::WARPS, S::SMEM, s>>>(p, tiles, row_tiles, vec_a, vec_w);
+    return st_launch_status();
+}
+int gf_few_launch(const GemmF32& p, cudaStream_t s) { return p.n_rows <= GF_FEW_ROWS ? gq_launch<1>(p, s) : gq_launch<2>(p, s); }

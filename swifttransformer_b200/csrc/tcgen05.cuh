@@ -71,6 +71,17 @@ __device__ __forceinline__ void tc_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint
 __device__ __forceinline__ void tc_commit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
 }
+// One lane of a converged warp, the same one each time.  A warp that issues products or copies runs its loops as a whole, with the
+// waits, and only the issue stands under this: the compiler then knows that addresses and descriptors are the same in all
+// lanes and keeps them in uniform registers.  Under `lane == 0` it does not: a product of 128 x 16 x 16 from tensor memory took 46
+// clocks to issue with constant offsets, 115 with computed ones, and takes 9 this way; a copy of one box 54 and 16.
+__device__ __forceinline__ bool tc_elect() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
+// a thread's warp, known to be the same in all lanes
+__device__ __forceinline__ int tc_warp() { return __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0); }
 // bounded wait for the given phase parity; false: gave up
 __device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity) {
     for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
@@ -81,6 +92,23 @@ __device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity) {
         if (i > 64) __nanosleep(32);
     }
     return false;
+}
+// The same by a whole warp, with one answer for all its lanes, which also ends when the block has been marked dead, and marks it
+// when the limit is reached.  try_wait: the hardware holds the warp until the phase completes or a time of about a microsecond
+// is over, so that waiting warps take no issue slots from working ones.
+#define TC_TRY_LIMIT (1u << 17)       // tries: at least 0.1 s, whatever a try's time is
+__device__ __forceinline__ bool tc_wait_warp(uint32_t mbar, uint32_t parity, volatile int* dead) {
+    bool ok = false;
+    for (uint32_t i = 0; i < TC_TRY_LIMIT; ++i) {
+        uint32_t done;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+                     "selp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(done) : "r"(mbar), "r"(parity), "r"(1000u) : "memory");
+        if (done) { ok = true; break; }
+        if (*dead) break;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok) *dead = 1;
+    return ok;
 }
 // 32 consecutive float columns of this thread's TMEM lane: the load is only issued here; the values
 // may be used after tc_ld_wait() (several loads can be in flight under one wait)
@@ -138,4 +166,9 @@ __device__ __forceinline__ void tc_tma_load_2d(uint32_t dst, const void* tmap, i
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
                  "[%0], [%1, {%2, %3}], [%4];\n"
                  ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(mbar) : "memory");
+}
+__device__ __forceinline__ void tc_tma_load_4d(uint32_t dst, const void* tmap, int c0, int c1, int c2, int c3, uint32_t mbar) {
+    asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
+                 "[%0], [%1, {%2, %3, %4, %5}], [%6];\n"
+                 ::"r"(dst), "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(mbar) : "memory");
 }

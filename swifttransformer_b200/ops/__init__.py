@@ -221,7 +221,7 @@ _addmm_activation = getattr(torch, "_addmm_activation", None)    # the library p
 
 def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none",
            out_dtype: Optional[torch.dtype] = None, bias_bf16: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """act(a @ w.T + bias); w is [out, in].  float32: the plain fused-multiply-add kernel (true 32-bit).
+    """act(a @ w.T + bias); w is [out, in].  float32: ``gemm_plain`` (true 32-bit).
     bfloat16, few rows: the weight-streaming kernel.  bfloat16, more rows: the library product with float
     accumulation; bias and ReLU ride in its epilogue when ``bias_bf16`` (a lossless bfloat16 copy of
     ``bias``, see lossless_bf16) is given, else the bias/activation kernel follows."""
@@ -456,14 +456,25 @@ def qkv_linear_to_cache(h: torch.Tensor, w: torch.Tensor, bias: Optional[torch.T
 
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none",
                out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """The plain kernel for either storage type (float arithmetic, fixed summation order)."""
+    """The plain product for either storage type (fixed summation order).  float32: on the tensor cores, each operand as
+    the sum of three bfloat16 numbers, at least as close to 64 bits as a chain of float multiply-adds.  bfloat16: a
+    chain of float multiply-adds."""
     out_dtype = out_dtype or a.dtype
     a = a.contiguous()
     assert w.is_contiguous()
     n, k = a.shape
     m = w.shape[0]
     out = a.new_empty((n, m), dtype=out_dtype)
-    _check(lib().st_gemm_plain(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], _dt(a),
+    if a.dtype == torch.float32:
+        assert out_dtype == torch.float32 and w.dtype == torch.float32
+        scratch = status = None
+        if n > 8:                            # beyond that the kernel may take a's parts, [3][n][k rounded up to 64], from memory
+            scratch = a.new_empty(6 * n * ((k + 63) // 64 * 64), dtype=torch.uint8)
+            status = _tc_status_word(a.device)
+        _check(lib().st_gemm_f32(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], 0, _p(scratch), _p(status),
+                                 _stream()), "gemm_plain")
+        return out
+    _check(lib().st_gemm_plain(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act],
                                int(out_dtype == torch.float32), _stream()), "gemm_plain")
     return out
 

@@ -49,13 +49,13 @@ static inline int st_tma_encode_bf16(CUtensorMap* out, const void* base, int ran
 }
 
 // The same with the strides given: strides[i] is the distance in bytes between consecutive indices of dimension
-// i + 1 (a multiple of 16; dimensions may be listed in any order of their strides, the innermost is contiguous).
+// i + 1 (a multiple of 16; dimensions may be listed in any order of their strides, the innermost is contiguous); rank up to 4.
 static inline int st_tma_encode_bf16_strided(CUtensorMap* out, const void* base, int rank, const unsigned long long* dims,
                                              const unsigned long long* strides, const unsigned* box) {
     st_tma_encode_fn enc = st_tma_encoder();
-    if (!enc || rank < 2 || rank > 3 || box[0] != 64) return -1;
-    cuuint64_t d[3], st[2];
-    cuuint32_t b[3], elem[3] = {1, 1, 1};
+    if (!enc || rank < 2 || rank > 4 || box[0] != 64) return -1;
+    cuuint64_t d[4], st[3];
+    cuuint32_t b[4], elem[4] = {1, 1, 1, 1};
     for (int i = 0; i < rank; ++i) {
         d[i] = dims[i];
         b[i] = box[i];

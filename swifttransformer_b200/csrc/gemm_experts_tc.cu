@@ -44,20 +44,6 @@ struct ExpertsShape {
     const int* a_rows;       // null: the rows of a are in sorted order
 };
 
-__device__ __forceinline__ bool ge_wait(uint32_t mbar, uint32_t parity, volatile int* dead) {
-    for (uint32_t i = 0; i < TC_WAIT_LIMIT; ++i) {
-        uint32_t done;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.b32 %0, 1, 0, p;\n\t}\n" : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
-        if (done) return true;
-        if (i > 256) {
-            if ((i & 63) == 0 && *dead) return false;
-            __nanosleep(32);
-        }
-    }
-    *dead = 1;
-    return false;
-}
 __device__ __forceinline__ void ge_arrive(uint32_t mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar) : "memory");
 }
@@ -121,7 +107,7 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
     constexpr uint32_t A_BYTES = GE_BM * 128, W_BYTES = BN * 128, STAGE = A_BYTES + W_BYTES;
     constexpr int TMEM_COLS = 2 * BN, stages = GE_STAGES(BN);
     const uint32_t base = (tc_smem(ge_raw) + 1023u) & ~1023u;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tc_warp(), lane = tid & 31;
     volatile int* dead = &s_dead;
     if (tid == 0) {
         for (int s = 0; s < stages; ++s) {
@@ -170,27 +156,31 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
     const int n_tiles = s_before[sh.n_experts] * n_tiles_n;
     const int n_k = (sh.k_dim + GE_BK - 1) / GE_BK;
 
-    if (warp == 4 && lane == 0) {
+    if (warp == 4) {
         // ---- weights, and rows of a that are neighbours
         const int w_rows = sh.gated ? 2 * sh.n_out : sh.n_out;
         int s = 0, turn = 0, it = 0;
-        for (int tile = blockIdx.x; tile < n_tiles && !*dead; tile += gridDim.x) {
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x) {
             const ExpertsTile t = ge_tile(tile, n_tiles_n, bn_out, s_before, sh);
             const int r0 = t.expert * w_rows + t.n0;
             const int boxes = GATHER ? 0 : (t.rows + 31) / 32;
             for (int k = 0; k < n_k; ++k) {
-                if (turn > 0 && !ge_wait(tc_smem(&s_empty[s]), (turn - 1) & 1, dead)) break;
+                if (turn > 0) ok = tc_wait_warp(tc_smem(&s_empty[s]), (turn - 1) & 1, dead);
+                if (!ok) break;
                 const uint32_t full = tc_smem(&s_full[s]), dst = base + s * STAGE + A_BYTES;
-                tc_mbar_expect_tx(full, W_BYTES + (uint32_t)boxes * 4096u);
-                tc_tma_load_2d(dst, &w_map, k * GE_BK, r0, full);
-                tc_tma_load_2d(dst + W_BYTES / 2, &w_map, k * GE_BK, sh.gated ? r0 + sh.n_out : r0 + BN / 2, full);
-                for (int b = 0; b < boxes; ++b)
-                    tc_tma_load_2d(base + s * STAGE + b * 4096, &a_map, k * GE_BK, t.row0 + 32 * b, full);
+                if (tc_elect()) {
+                    tc_mbar_expect_tx(full, W_BYTES + (uint32_t)boxes * 4096u);
+                    tc_tma_load_2d(dst, &w_map, k * GE_BK, r0, full);
+                    tc_tma_load_2d(dst + W_BYTES / 2, &w_map, k * GE_BK, sh.gated ? r0 + sh.n_out : r0 + BN / 2, full);
+                    for (int b = 0; b < boxes; ++b)
+                        tc_tma_load_2d(base + s * STAGE + b * 4096, &a_map, k * GE_BK, t.row0 + 32 * b, full);
+                }
                 ++it;
                 if (++s == stages) { s = 0; ++turn; }
             }
         }
-        s_issued = it;
+        if (lane == 0) s_issued = it;
     } else if (GATHER && warp >= 6) {
         // ---- gathered rows of a: a thread copies one 16-byte piece of every sixteenth row of the tile
         const int t128 = tid - GE_THREADS, piece = t128 & 7, r_first = t128 >> 3;
@@ -206,7 +196,7 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
                 src[i] = a + (size_t)(__ldcg(sh.a_rows + row) / sh.a_row_div) * sh.k_dim + piece * 8;
             }
             for (int k = 0; k < n_k; ++k) {
-                if (turn > 0) ok = ge_wait(tc_smem(&s_empty[s]), (turn - 1) & 1, dead);
+                if (turn > 0) ok = tc_wait_warp(tc_smem(&s_empty[s]), (turn - 1) & 1, dead);
                 if (!ok) break;
                 const bool in_k = k * GE_BK + piece * 8 < sh.k_dim;
                 const uint32_t dst = base + s * STAGE + at;
@@ -219,26 +209,32 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
             }
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
-    } else if (warp == 5 && lane == 0) {
+    } else if (warp == 5) {
         // ---- products
         const uint32_t idesc = tc_idesc(GE_BM, BN, 0, 0);
         int s = 0, turn = 0, i = 0;
-        for (int tile = blockIdx.x; tile < n_tiles && !*dead; tile += gridDim.x, ++i) {
+        bool ok = true;
+        for (int tile = blockIdx.x; ok && tile < n_tiles; tile += gridDim.x, ++i) {
             const int buf = i & 1;
-            if (i >= 2 && !ge_wait(tc_smem(&s_free[buf]), ((i >> 1) - 1) & 1, dead)) break;
+            if (i >= 2) ok = tc_wait_warp(tc_smem(&s_free[buf]), ((i >> 1) - 1) & 1, dead);
+            if (!ok) break;
             tc_fence_after_sync();
             for (int k = 0; k < n_k; ++k) {
-                if (!ge_wait(tc_smem(&s_full[s]), turn & 1, dead)) break;
+                ok = tc_wait_warp(tc_smem(&s_full[s]), turn & 1, dead);
+                if (!ok) break;
                 if (GATHER) tc_fence_async_smem();
                 tc_fence_after_sync();
                 const uint64_t da = tc_desc(base + s * STAGE, 16, 1024), dw = tc_desc(base + s * STAGE + A_BYTES, 16, 1024);
+                if (tc_elect()) {
 #pragma unroll
-                for (int kk = 0; kk < GE_BK / 16; ++kk)
-                    tc_mma(tmem + buf * BN, da + ((kk * 32) >> 4), dw + ((kk * 32) >> 4), idesc, k > 0 || kk > 0);
-                tc_commit(tc_smem(&s_empty[s]));
+                    for (int kk = 0; kk < GE_BK / 16; ++kk)
+                        tc_mma(tmem + buf * BN, da + ((kk * 32) >> 4), dw + ((kk * 32) >> 4), idesc, k > 0 || kk > 0);
+                    tc_commit(tc_smem(&s_empty[s]));
+                }
+                __syncwarp();
                 if (++s == stages) { s = 0; ++turn; }
             }
-            tc_commit(tc_smem(&s_done[buf]));
+            if (tc_elect()) tc_commit(tc_smem(&s_done[buf]));
         }
     } else if (warp < 4) {
         // ---- epilogue: warp q holds rows 32 q .. 32 q + 31 of the tile, a thread its row
@@ -246,7 +242,7 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x, ++i) {
             const ExpertsTile t = ge_tile(tile, n_tiles_n, bn_out, s_before, sh);
             const int buf = i & 1;
-            if (!__all_sync(0xffffffffu, ge_wait(tc_smem(&s_done[buf]), (i >> 1) & 1, dead))) break;
+            if (!tc_wait_warp(tc_smem(&s_done[buf]), (i >> 1) & 1, dead)) break;
             tc_fence_after_sync();
             const int r = warp * 32 + lane;
             const uint32_t t_row = tmem + buf * BN + ((uint32_t)(warp * 32) << 16);

@@ -31,6 +31,29 @@ __device__ __forceinline__ bool hk_find(const int* q_start, const int* positions
     return chunk >= 0 && n > 0 && end - begin >= from && positions[begin] >= 0;      // (padding stands at position -1)
 }
 
+// 1 / d and z / d for d >= 1 to the last bit or next to it: the hardware's reciprocal (of at most 1e38: beyond, the quotient is next to
+// nothing either way) and a step of residual correction.  The compiler's own division tests every operand for its slow
+// form, and so a thread's divisions run one after the other, some 360 clocks each: 32 of them were most of a chunk's time.
+__device__ __forceinline__ float hk_inverse(float d) {
+    float r;
+    d = fminf(d, 1e38f);                                  // (a number that is none comes out as 1e-38 and makes the result none below)
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    return fmaf(r, fmaf(-d, r, 1.f), r);
+}
+__device__ __forceinline__ float hk_sigmoid(float z) {
+    const float e = expf(-z), r = hk_inverse(1.f + e);
+    return z != z ? z : r;
+}
+__device__ __forceinline__ float hk_silu(float z) {
+    const float d = fminf(1.f + expf(-z), 1e38f), r = hk_inverse(d), q = z * r, rest = fmaf(-q, d, z);
+    return rest < 0.f || rest > 0.f ? fmaf(rest, r, q) : q;          // (an infinite z has no residual)
+}
+// 1 / sqrt(x): the hardware's and a Newton step
+__device__ __forceinline__ float hk_rsqrt(float x) {
+    const float r = rsqrtf(x);
+    return x > 1e-30f && x < 1e30f ? fmaf(0.5f * r, fmaf(-x * r, r, 1.f), r) : r;
+}
+
 __device__ __forceinline__ void hk_cp16(float* dst, const float* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src));
 }

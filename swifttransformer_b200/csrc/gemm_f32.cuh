@@ -20,25 +20,9 @@
 // over k: 4.0e-7, 8.1e-7, 1.6e-6).
 #pragma once
 #include "common.cuh"
+#include "float_parts.cuh"
 
 #define GF_BK 64             // k of a group
-
-// what two bfloat16 numbers leave of two floats
-__device__ __forceinline__ void gf_rest(float& x0, float& x1, uint32_t packed) {
-    asm("{\n\t.reg .b64 a, b, d;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tsub.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}\n"
-        : "+f"(x0), "+f"(x1) : "f"(__uint_as_float(packed << 16)), "f"(__uint_as_float(packed & 0xffff0000u)));
-}
-// two neighbours -> their three parts, packed
-__device__ __forceinline__ void gf_split(float x0, float x1, uint32_t& h, uint32_t& m, uint32_t& l) {
-    const __nv_bfloat162 hb = __floats2bfloat162_rn(x0, x1);
-    h = *reinterpret_cast<const uint32_t*>(&hb);
-    gf_rest(x0, x1, h);
-    const __nv_bfloat162 mb = __floats2bfloat162_rn(x0, x1);
-    m = *reinterpret_cast<const uint32_t*>(&mb);
-    gf_rest(x0, x1, m);
-    const __nv_bfloat162 lb = __floats2bfloat162_rn(x0, x1);
-    l = *reinterpret_cast<const uint32_t*>(&lb);
-}
 
 struct GemmF32 {
     const float *a, *w, *bias;

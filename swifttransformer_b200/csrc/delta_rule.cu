@@ -22,6 +22,7 @@
 //
 // Since (decay S + k u^T)^T q = (decay S)^T q + u (k . q), both dot products of a token are taken from the
 // decayed state in one pass of shuffles.
+#include "chunks.cuh"
 #include "delta_rule.cuh"
 
 #define DR_MAX_TAPS 8
@@ -30,7 +31,6 @@
 #define DR_UNIT_PASSES 8      // a warp's lanes cover a head of up to 32 * DR_UNIT_PASSES channels
 
 __device__ __forceinline__ float softplusf_(float z) { return z > 20.f ? z : log1pf(expf(z)); }
-__device__ __forceinline__ float siluf_(float z) { return z / (1.f + expf(-z)); }
 
 // sum_r x[r] * w[r] in the order of r, the weights fetched in 16-byte pieces where the row allows it
 #define DR_RANK_SMEM 256      // low-rank inputs of up to this many numbers wait in shared memory
@@ -116,7 +116,7 @@ delta_prepare_kernel(const float* __restrict__ proj, int ld, DeltaShape sh, cons
             }
             if (move_state)
                 for (int j = 0; j < keep; ++j) st[(size_t)j * channels + c] = vv[j + 1];
-            y = siluf_(y);
+            y = hk_silu(y);
             x[r] = y;
             ss = fmaf(y, y, ss);
         }
@@ -134,7 +134,7 @@ delta_prepare_kernel(const float* __restrict__ proj, int ld, DeltaShape sh, cons
     }
     if (blockIdx.y == 0) {
         for (int h = threadIdx.x; h < H; h += blockDim.x)
-            dst[sh.pb() + h] = 1.f / (1.f + expf(-__ldcg(row + sh.b_off + h)));
+            dst[sh.pb() + h] = hk_sigmoid(__ldcg(row + sh.b_off + h));
     }
     // decays: the low-rank step size, one thread per (head, key channel)
     __shared__ float xs_a[DR_RANK_SMEM];
@@ -157,6 +157,166 @@ delta_prepare_kernel(const float* __restrict__ proj, int ld, DeltaShape sh, cons
         dst[sh.pd() + c] = expf(-expf(a_log[c / dim]) * dt);
     }
     if (!early) ST_PDL_TRIGGER();
+}
+
+// ---- delta_prepare for steps of many tokens -------------------------------------------------------------------
+// delta_prepare_kernel has every token fetch its filters, low-rank weights and past rows again, by 80 KB of code that a block runs
+// once; here a warp takes one head of q, k or v and a thread one key channel's decay through `run` tokens in a row (at most DR_RUN): filters
+// and weights stay in registers, a token's past rows are the registers of the tokens before.  Every sum is delta_prepare_kernel's in
+// the same order: a token's numbers do not depend on who shares its step.
+// us on one B200, 2000 tokens, 8 value heads and 4 key heads of 128, rank 16 (41 MB of rows): 21 where delta_prepare_kernel takes 56; with
+// runs of eight or four tokens where sixteen would leave the SMs idle 1501 tokens of 4 heads are 10 us faster, with sixteen 7 slower.
+// Bound by instructions: some 120 of each decay's, 50 of each channel's.
+#define DR_RUN 16
+#define DR_RUN_OUT 4
+#define DR_RUN_LOW 64         // low-rank inputs (or heads, without the pair) per token kept in shared memory
+#define DR_RUN_UNITS 4        // a lane's channels of a head of up to 128: lane, lane + 32, ..
+
+// sixteen low-rank weights of a row (16-byte aligned)
+__device__ __forceinline__ void dr_sixteen(const float* p, float* w) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(p) + i);
+        w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+    }
+}
+__device__ __forceinline__ void dr_sixteen(const bf16* p, float* w) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const uint4 u = __ldg(reinterpret_cast<const uint4*>(p) + i);
+        const uint32_t u4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            w[8 * i + 2 * j] = __uint_as_float(u4[j] << 16);
+            w[8 * i + 2 * j + 1] = __uint_as_float(u4[j] & 0xffff0000u);
+        }
+    }
+}
+
+// RANK: 16, 0 (no pair) or -1 (any rank up to DR_RUN_LOW)
+template <typename TW, int TAPS, int RANK>
+__global__ void __launch_bounds__(DR_PREP_THREADS)
+delta_prepare_run_kernel(const float* __restrict__ proj, int ld, DeltaShape sh, const float* __restrict__ conv_w,
+                         const float* __restrict__ state, int conv_blocks, const TW* __restrict__ w_a2,
+                         const float* __restrict__ a_log, const float* __restrict__ dt_bias, float* __restrict__ prep,
+                         const int* __restrict__ positions, const int* __restrict__ seq_of_token,
+                         const int* __restrict__ q_start, const int* __restrict__ slots, int n_tokens, int run) {
+    constexpr int KEEP = TAPS - 1;
+    __shared__ int s_place[DR_RUN], s_slot[DR_RUN];          // a token's place in its portion (-1: padding), its request's slot
+    __shared__ __align__(16) float s_low[DR_RUN][DR_RUN_LOW];
+    const int tid = threadIdx.x, lane = tid & 31, t0 = blockIdx.x * run, n_run = min(run, n_tokens - t0);
+    const int H = sh.H, G = sh.G, dim = sh.dim, vd = sh.vd;
+    ST_PDL_WAIT();
+    if ((int)blockIdx.y < conv_blocks) {
+        if (tid < n_run) {
+            const int b = seq_of_token[t0 + tid];
+            const bool on = positions[t0 + tid] >= 0;
+            s_place[tid] = on ? t0 + tid - q_start[b] : -1;
+            s_slot[tid] = on ? slots[b] : 0;
+        }
+        __syncthreads();
+        const int u = blockIdx.y * (DR_PREP_THREADS / 32) + (tid >> 5), channels = 2 * G * dim + H * vd;
+        const bool is_v = u >= 2 * G;
+        const int width = is_v ? vd : dim;
+        const int c = (is_v ? 2 * G * dim + (u - 2 * G) * vd : u * dim) + lane;
+        if (u < 2 * G + H) {
+            float w[DR_RUN_UNITS][TAPS], past[DR_RUN_UNITS][KEEP > 0 ? KEEP : 1];        // past: the rows 1 .. KEEP before the next token
+#pragma unroll
+            for (int r = 0; r < DR_RUN_UNITS; ++r)
+#pragma unroll
+                for (int j = 0; j < TAPS; ++j) w[r][j] = lane + 32 * r < width ? conv_w[(size_t)(c + 32 * r) * TAPS + j] : 0.f;
+            const float* src = proj + (size_t)t0 * ld + sh.q_off + c;
+            bool follows = false;                            // `past` belongs to the token at hand
+#pragma unroll 1
+            for (int g = 0; g < n_run; g += 4) {
+                float v[4][DR_RUN_UNITS];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+#pragma unroll
+                    for (int r = 0; r < DR_RUN_UNITS; ++r)
+                        v[k][r] = lane + 32 * r < width ? __ldcg(src + (size_t)min(g + k, n_run - 1) * ld + 32 * r) : 0.f;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const int t = g + k, place = t < n_run ? s_place[t] : -1;
+                    if (place < 0) { follows = false; continue; }
+                    if (!follows || place == 0) {
+                        const float* st = state + (size_t)s_slot[t] * KEEP * channels + c;
+#pragma unroll
+                        for (int back = 1; back <= KEEP; ++back)
+#pragma unroll
+                            for (int r = 0; r < DR_RUN_UNITS; ++r)
+                                past[r][back - 1] = lane + 32 * r >= width ? 0.f
+                                                    : back <= place ? __ldcg(src + ((long long)t - back) * ld + 32 * r)
+                                                                    : __ldcg(st + (size_t)(KEEP - (back - place)) * channels + 32 * r);
+                    }
+                    follows = true;
+                    float y[DR_RUN_UNITS], ss = 0.f;
+#pragma unroll
+                    for (int r = 0; r < DR_RUN_UNITS; ++r) {
+                        y[r] = 0.f;
+#pragma unroll
+                        for (int back = KEEP; back >= 1; --back) y[r] = fmaf(w[r][KEEP - back], past[r][back - 1], y[r]);
+                        y[r] = fmaf(w[r][KEEP], v[k][r], y[r]);
+                        y[r] = hk_silu(y[r]);
+                        if (lane + 32 * r < width) ss = fmaf(y[r], y[r], ss);
+                    }
+                    float mult = 1.f;
+                    if (!is_v) {
+                        ss = warp_sum(ss);
+                        mult = rsqrtf(ss + 1e-6f);
+                        if (u < G) mult *= rsqrtf((float)dim);
+                    }
+                    float* dst = prep + (size_t)(t0 + t) * sh.stride + c;
+#pragma unroll
+                    for (int r = 0; r < DR_RUN_UNITS; ++r) {
+                        if (lane + 32 * r < width) dst[32 * r] = y[r] * mult;
+#pragma unroll
+                        for (int back = KEEP; back >= 2; --back) past[r][back - 1] = past[r][back - 2];
+                        past[r][0] = v[k][r];
+                    }
+                }
+            }
+        }
+    } else {
+        if (tid < n_run) s_place[tid] = positions[t0 + tid];
+        const int low = RANK == 0 ? H : sh.rank_a;
+        for (int i = tid; i < n_run * DR_RUN_LOW; i += DR_PREP_THREADS) {
+            const int t = i / DR_RUN_LOW, r = i % DR_RUN_LOW;
+            if (r < low) s_low[t][r] = __ldcg(proj + (size_t)(t0 + t) * ld + sh.a_off + r);
+        }
+        __syncthreads();
+        if ((int)blockIdx.y == conv_blocks)
+            for (int i = tid; i < n_run * H; i += DR_PREP_THREADS) {
+                const int t = i / H, h = i % H;
+                if (s_place[t] >= 0)
+                    prep[(size_t)(t0 + t) * sh.stride + sh.pb() + h] = hk_sigmoid(__ldcg(proj + (size_t)(t0 + t) * ld + sh.b_off + h));
+            }
+        const int c = (blockIdx.y - conv_blocks) * DR_PREP_THREADS + tid;
+        if (c < H * dim) {
+            const int h = c / dim;
+            const float rate = expf(a_log[h]), bias = dt_bias[RANK == 0 ? h : c];
+            float w[RANK > 0 ? RANK : 1];
+            if constexpr (RANK > 0) dr_sixteen(w_a2 + (size_t)c * RANK, w);
+            float* dst = prep + (size_t)t0 * sh.stride + sh.pd() + c;
+#pragma unroll 4
+            for (int t = 0; t < n_run; ++t) {
+                float z = 0.f;
+                if constexpr (RANK > 0) {
+#pragma unroll
+                    for (int r = 0; r < RANK; r += 4) {
+                        const float4 x = load4(&s_low[t][r]);
+                        z = fmaf(x.x, w[r], z); z = fmaf(x.y, w[r + 1], z); z = fmaf(x.z, w[r + 2], z); z = fmaf(x.w, w[r + 3], z);
+                    }
+                } else if constexpr (RANK == 0) {
+                    z = s_low[t][h];
+                } else {
+                    z = lowrank_dot(s_low[t], w_a2 + (size_t)c * sh.rank_a, sh.rank_a);
+                }
+                if (s_place[t] >= 0) dst[(size_t)t * sh.stride] = expf(-rate * softplusf_(z + bias));
+            }
+        }
+    }
+    ST_PDL_TRIGGER();
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -356,8 +516,75 @@ delta_output_kernel(const float* __restrict__ o, const float* __restrict__ proj,
     for (int e = threadIdx.x; e < vd; e += blockDim.x) {
         const float z = sh.rank_g > 0 ? lowrank_dot(g1, w_g2 + (size_t)(h * vd + e) * sh.rank_g, sh.rank_g)
                                       : __ldcg(g1 + h * vd + e);
-        const float gate = (sh.gate_silu ? z : 1.f) / (1.f + expf(-z));
+        const float gate = sh.gate_silu ? hk_silu(z) : hk_sigmoid(z);
         out[((size_t)t * sh.H + h) * vd + e] = from_f32<T>(__ldcg(orow + e) * inv * norm_w[e] * gate);
+    }
+}
+
+// delta_output for steps of many tokens: a warp takes a head through DR_RUN_OUT tokens, the low-rank weights in registers; its sums are
+// delta_output_kernel's in the same order.  15 us where that takes 24 (2000 tokens, 8 heads of 128, rank 16); sixteen tokens a warp, 34
+template <typename T, int RANK>
+__global__ void __launch_bounds__(DR_PREP_THREADS)
+delta_output_run_kernel(const float* __restrict__ o, const float* __restrict__ proj, int ld, DeltaShape sh, const T* __restrict__ w_g2,
+                        const float* __restrict__ norm_w, float eps, float out_scale, T* __restrict__ out,
+                        const int* __restrict__ positions, int n_tokens) {
+    __shared__ __align__(16) float s_low[DR_RUN_OUT][DR_RUN_LOW];
+    __shared__ int s_on[DR_RUN_OUT];
+    const int tid = threadIdx.x, lane = tid & 31, t0 = blockIdx.x * DR_RUN_OUT, n_run = min(DR_RUN_OUT, n_tokens - t0);
+    const int h = blockIdx.y * (DR_PREP_THREADS / 32) + (tid >> 5), vd = sh.vd;
+    float w[DR_RUN_UNITS][RANK > 0 ? RANK : 1], nw[DR_RUN_UNITS];
+    bool on[DR_RUN_UNITS];
+#pragma unroll
+    for (int x = 0; x < DR_RUN_UNITS; ++x) {               // (weights: no kernel writes them)
+        const int e = lane + 32 * x;
+        on[x] = h < sh.H && e < vd;
+        nw[x] = on[x] ? norm_w[e] : 0.f;
+        if constexpr (RANK > 0)
+            if (on[x]) dr_sixteen(w_g2 + ((size_t)h * vd + e) * RANK, w[x]);
+    }
+    ST_PDL_WAIT();
+    ST_PDL_TRIGGER();
+    if (tid < n_run) s_on[tid] = positions[t0 + tid] >= 0;
+    if (RANK != 0)
+        for (int i = tid; i < DR_RUN_OUT * DR_RUN_LOW; i += DR_PREP_THREADS) {
+            const int t = i / DR_RUN_LOW, r = i % DR_RUN_LOW;
+            if (t < n_run && r < sh.rank_g) s_low[t][r] = __ldcg(proj + (size_t)(t0 + t) * ld + sh.g_off + r);
+        }
+    float v[DR_RUN_OUT][DR_RUN_UNITS];
+#pragma unroll
+    for (int k = 0; k < DR_RUN_OUT; ++k)
+#pragma unroll
+        for (int x = 0; x < DR_RUN_UNITS; ++x)
+            v[k][x] = on[x] ? __ldcg(o + ((size_t)(t0 + min(k, n_run - 1)) * sh.H + h) * vd + lane + 32 * x) : 0.f;
+    __syncthreads();
+    if (h >= sh.H) return;
+#pragma unroll
+    for (int k = 0; k < DR_RUN_OUT; ++k) {
+        if (k >= n_run || !s_on[k]) continue;
+        float ss = 0.f;
+#pragma unroll
+        for (int x = 0; x < DR_RUN_UNITS; ++x) ss += warp_sum(v[k][x] * v[k][x]);
+        const float inv = rsqrtf(ss / (float)vd + eps) * out_scale;
+#pragma unroll
+        for (int x = 0; x < DR_RUN_UNITS; ++x) {
+            if (!on[x]) continue;
+            const int e = lane + 32 * x;
+            float z = 0.f;
+            if constexpr (RANK > 0) {
+#pragma unroll
+                for (int r = 0; r < RANK; r += 4) {
+                    const float4 low = load4(&s_low[k][r]);
+                    z = fmaf(low.x, w[x][r], z); z = fmaf(low.y, w[x][r + 1], z);
+                    z = fmaf(low.z, w[x][r + 2], z); z = fmaf(low.w, w[x][r + 3], z);
+                }
+            } else if constexpr (RANK == 0) {
+                z = __ldcg(proj + (size_t)(t0 + k) * ld + sh.g_off + h * vd + e);
+            } else {
+                z = lowrank_dot(s_low[k], w_g2 + ((size_t)h * vd + e) * sh.rank_g, sh.rank_g);
+            }
+            const float gate = sh.gate_silu ? hk_silu(z) : hk_sigmoid(z);
+            out[((size_t)(t0 + k) * sh.H + h) * vd + e] = from_f32<T>(v[k][x] * inv * nw[x] * gate);
+        }
     }
 }
 
@@ -412,7 +639,41 @@ ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int
     float* o = scratch + (size_t)n_tokens * sh.stride;
     const int move = single_tokens && write_state && taps > 1;
     int rc;
-    {
+    // Which form of prepare and output: by runs of tokens where a step has enough of them to fill the multiprocessors, heads fit a
+    // warp's registers and the tails are not moved on here
+    const bool runs = n_tokens > DR_EARLY_TOKENS && !move && taps >= 2 && taps <= 4 && dim <= 32 * DR_RUN_UNITS && vd <= 32 * DR_RUN_UNITS &&
+                      H <= DR_RUN_LOW && rank_a <= DR_RUN_LOW && rank_g <= DR_RUN_LOW;
+    const bool sixteen_a = rank_a == 16 && aligned16(w_a2), sixteen_g = rank_g == 16 && aligned16(w_g2);
+    if (runs) {
+        const int conv_blocks = (2 * G + H + DR_PREP_THREADS / 32 - 1) / (DR_PREP_THREADS / 32);
+        // sixteen tokens a run where that still gives four blocks per SM, else eight or four
+        const int gy = conv_blocks + (H * dim + DR_PREP_THREADS - 1) / DR_PREP_THREADS;
+        int run = DR_RUN;
+        while (run > 4 && (long long)((n_tokens + run - 1) / run) * gy < 4 * st_sm_count()) run /= 2;
+        const dim3 grid((unsigned)((n_tokens + run - 1) / run), gy);
+#define DR_RUN_PREP(TW, TAPS, RANK)                                                                                   \
+    rc = st_launch_pdl("delta_prepare", delta_prepare_run_kernel<TW, TAPS, RANK>, grid, dim3(DR_PREP_THREADS), 0, s, proj, ld, sh, conv_w, \
+                       (const float*)conv_state, conv_blocks, (const TW*)w_a2, a_log, dt_bias, prep, positions, seq_of_token, q_start, \
+                       slots, n_tokens, run)
+#define DR_RUN_RANK(TW, TAPS)                                                                                         \
+    do {                                                                                                              \
+        if (sixteen_a) DR_RUN_PREP(TW, TAPS, 16);                                                                     \
+        else if (rank_a == 0) DR_RUN_PREP(TW, TAPS, 0);                                                               \
+        else DR_RUN_PREP(TW, TAPS, -1);                                                                               \
+    } while (0)
+#define DR_RUN_TAPS(TW)                                                                                               \
+    do {                                                                                                              \
+        if (taps == 4) DR_RUN_RANK(TW, 4);                                                                            \
+        else if (taps == 3) DR_RUN_RANK(TW, 3);                                                                       \
+        else DR_RUN_RANK(TW, 2);                                                                                      \
+    } while (0)
+        if (dtype == 0) DR_RUN_TAPS(float);
+        else DR_RUN_TAPS(bf16);
+#undef DR_RUN_TAPS
+#undef DR_RUN_RANK
+#undef DR_RUN_PREP
+        if (rc) return rc;
+    } else {
         const int units = 2 * G + H;
         int gy = (units + 7) / 8;
         if (gy > 16) gy = 16;
@@ -468,6 +729,22 @@ ST_EXPORT int st_delta_rule(const float* proj, int ld, int q_off, int b_off, int
         rc = delta_chunks_launch(prep, sh, o + (size_t)n_tokens * H * vd, state, write_state, o, positions, q_start, slots, n_tokens,
                                  n_seqs, from, s);
         if (rc) return rc;
+    }
+    if (runs) {
+        const dim3 grid((unsigned)((n_tokens + DR_RUN_OUT - 1) / DR_RUN_OUT), (H + DR_PREP_THREADS / 32 - 1) / (DR_PREP_THREADS / 32));
+#define DR_RUN_OUTPUT(T, RANK)                                                                                           \
+    return st_launch_pdl("delta_output", delta_output_run_kernel<T, RANK>, grid, dim3(DR_PREP_THREADS), 0, s, (const float*)o, proj, ld, sh, \
+                         (const T*)w_g2, norm_w, eps, out_scale, (T*)out, positions, n_tokens)
+#define DR_RUN_RANK(T)                                                                                                \
+    do {                                                                                                              \
+        if (sixteen_g) DR_RUN_OUTPUT(T, 16);                                                                          \
+        if (rank_g == 0) DR_RUN_OUTPUT(T, 0);                                                                            \
+        DR_RUN_OUTPUT(T, -1);                                                                                            \
+    } while (0)
+        if (dtype == 0) DR_RUN_RANK(float);
+        DR_RUN_RANK(bf16);
+#undef DR_RUN_RANK
+#undef DR_RUN_OUTPUT
     }
     dim3 grid(n_tokens, H);
     if (dtype == 0)

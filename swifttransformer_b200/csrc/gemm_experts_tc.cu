@@ -4,7 +4,7 @@
 //   c[row, n] = epilogue( sum_k a[arow, k] * w[g][n][k] )        arow = a_rows[row] / a_row_div, or the row itself
 //
 // with the epilogue of gemm_grouped.cu: act(product), or "gated": w[g] holds 2 * n_out rows, gate rows first, and
-// c = act(gate) * up, both products rounded to bfloat16 first.
+// c = act(gate) * up, both products rounded to bfloat16 first; with a limit the clamped unit of gated_clamped_act instead.
 //
 // One persistent block per SM walks through tiles of 128 rows x BN rows of w (gated: BN / 2 gate rows and the BN / 2 up rows
 // beside them, so that one accumulator holds both).  Which tiles there are follows from the offsets on the device: expert by
@@ -40,6 +40,7 @@
 
 struct ExpertsShape {
     int n_experts, n_out, k_dim, gated, act, ldc, a_row_div, vec;
+    float limit, alpha, shift;      // limit > 0: g = min(gate, limit), u = clamp(up, -limit, limit), c = g sigmoid(alpha g) (u + shift)
     const int* offsets;
     const int* a_rows;       // null: the rows of a are in sorted order
 };
@@ -63,6 +64,16 @@ __device__ __forceinline__ void ge_silu8(float* v) {
         const float d = 1.f + expf(-v[j]), sc = d > 1e30f ? 5.421010862427522e-20f : 1.f;       // (2^-64: the fast one ends at 2^126)
         const float r = __fdividef(1.f, d * sc) * sc, q = v[j] * r, rest = fmaf(-q, d, v[j]);
         v[j] = rest < 0.f || rest > 0.f ? fmaf(rest, r, q) : q;
+    }
+}
+// the clamped unit of eight gates v and ups u, the quotients as in ge_silu8
+__device__ __forceinline__ void ge_clamped8(float* v, const float* u, float limit, float alpha, float shift) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const float g = fminf(v[j], limit), up = fminf(fmaxf(u[j], -limit), limit);
+        const float d = 1.f + expf(-alpha * g), sc = d > 1e30f ? 5.421010862427522e-20f : 1.f;
+        const float r = __fdividef(1.f, d * sc) * sc, q = g * r, rest = fmaf(-q, d, g);
+        v[j] = (rest < 0.f || rest > 0.f ? fmaf(rest, r, q) : q) * (up + shift);
     }
 }
 __device__ __forceinline__ void ge_act8(float* v, int act) {
@@ -268,10 +279,17 @@ gemm_experts_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_c
 #pragma unroll
                         for (int j = 0; j < 8; ++j) v[j] = 0.f;
                     }
-                    ge_act8(v, sh.act);
                     if (sh.gated) {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) v[j] *= to_f32(from_f32<bf16>(u[j]));
+                        for (int j = 0; j < 8; ++j) u[j] = to_f32(from_f32<bf16>(u[j]));
+                    }
+                    if (sh.limit > 0.f) ge_clamped8(v, u, sh.limit, sh.alpha, sh.shift);
+                    else {
+                        ge_act8(v, sh.act);
+                        if (sh.gated) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) v[j] *= u[j];
+                        }
                     }
                     if (live && sh.vec && t.n0 + c0 + 8 <= sh.n_out) {
                         uint4 p;
@@ -343,12 +361,13 @@ ST_EXPORT int st_gemm_experts_tc_applies(int n_experts, int k_dim) {
 
 // a [a_n_rows, k_dim], w [n_experts, w_rows, k_dim] (w_rows = n_out, twice that with `gated`), c [n_items, n_out], all bfloat16
 // and contiguous; offsets [n_experts + 1]; a_rows [n_items] or null (a's rows are then the items in sorted order).
-// tile_bn: rows of w per tile (64, 128, 256), 0: chosen here.
+// tile_bn: rows of w per tile (64, 128, 256), 0: chosen here.  limit > 0 (gated): the clamped unit with alpha and shift, act is not read.
 ST_EXPORT int st_gemm_experts_tc(const void* a, long long a_n_rows, const void* w, void* c, int n_experts, int n_items, int n_out,
                                  int k_dim, int gated, int act, const int* offsets, const int* a_rows, int a_row_div, int tile_bn,
-                                 int* status, void* stream) {
+                                 int* status, void* stream, float limit, float alpha, float shift) {
     if (n_items <= 0 || n_out <= 0) return 0;
     if (!offsets || !status || (a_rows && a_row_div <= 0) || a_n_rows <= 0) return ST_ERR_BAD_ARG;
+    if (limit > 0.f && !gated) return ST_ERR_BAD_ARG;
     if (!st_gemm_experts_tc_applies(n_experts, k_dim) || !aligned16(a) || !aligned16(w)) return ST_ERR_BAD_SIZE;
     const int w_rows = gated ? 2 * n_out : n_out;
     if ((long long)n_experts * w_rows > 0x7fffffffLL || a_n_rows > 0x7fffffffLL) return ST_ERR_TOO_LARGE;
@@ -361,6 +380,7 @@ ST_EXPORT int st_gemm_experts_tc(const void* a, long long a_n_rows, const void* 
     if (st_tma_encode_bf16(&w_map, w, 2, wd, wb) || st_tma_encode_bf16(&a_map, a, 2, ad, ab)) return ST_ERR_BAD_ARG;
     ExpertsShape sh;
     sh.n_experts = n_experts; sh.n_out = n_out; sh.k_dim = k_dim; sh.gated = gated; sh.act = act; sh.ldc = n_out;
+    sh.limit = limit; sh.alpha = alpha; sh.shift = shift;
     sh.a_row_div = a_row_div; sh.vec = n_out % 8 == 0 && aligned16(c); sh.offsets = offsets; sh.a_rows = a_rows;
     const int bn_out = gated ? bn / 2 : bn;
     const long long max_tiles = ((n_items + GE_BM - 1) / GE_BM + (long long)n_experts) * ((n_out + bn_out - 1) / bn_out);

@@ -1320,25 +1320,33 @@ def moe_sort(experts: torch.Tensor, n_experts: int) -> ExpertOrder:
     return ExpertOrder(offsets, sorted_items, place, tile_group, tile_row0, items, top)
 
 
+_NO_CLAMP = [_f(0.0)] * 3
+
+
 def gemm_experts(a: torch.Tensor, w: torch.Tensor, order: ExpertOrder, gather: bool, gated: bool = False,
-                 act: str = "none") -> torch.Tensor:
+                 act: str = "none", clamp: Optional[Sequence[float]] = None) -> torch.Tensor:
     """One product per expert over the rows the order gives it: out [items, n_out] in sorted order.
     ``gather``: the rows of ``a`` are the tokens (row of item i = i // top), else ``a`` is already in sorted order.
-    w [experts, n_out (twice with ``gated``: gate rows, then up rows), k]; out = act(product), gated: act(gate) * up.
+    w [experts, n_out (twice with ``gated``: gate rows, then up rows), k]; out = act(product), gated: act(gate) * up,
+    with ``clamp`` (limit, alpha, shift) the unit of ``gated_clamped_act``.
     bfloat16 with k a multiple of 8: the tcgen05 kernel (a wait that expires inside it shows in ``kernel_status``), for small
     products the mma.sync one; else the plain one."""
     assert a.is_contiguous() and w.is_contiguous() and w.dim() == 3 and a.dtype == w.dtype
     E, w_rows, k = w.shape
     n_rows, a_k = a.shape
-    assert a_k == k
+    assert a_k == k and (clamp is None or gated)
+    tensor_cores = (not _experts_mma(order.n_items, E, w_rows, k) and GROUPED_MMA and a.dtype == torch.bfloat16
+                    and bool(lib().st_gemm_experts_tc_applies(E, k)))
+    if clamp is not None and not (tensor_cores and clamp[0] > 0):      # gate | up of every item as the product leaves them, then the unit over the rows
+        return gated_clamped_act(gemm_experts(a, w, order, gather), None, *clamp)
     n_out = w_rows // 2 if gated else w_rows
     out = a.new_empty((order.n_items, n_out))
     ll = ctypes.c_longlong
-    if (not _experts_mma(order.n_items, E, w_rows, k) and GROUPED_MMA and a.dtype == torch.bfloat16
-            and bool(lib().st_gemm_experts_tc_applies(E, k))):
+    if tensor_cores:
+        limit = _NO_CLAMP if clamp is None else [_f(x) for x in clamp]
         _check(lib().st_gemm_experts_tc(_p(a), ll(n_rows), _p(w), _p(out), E, order.n_items, n_out, k, int(gated), ACT_CODES[act],
                                         _p(order.offsets), _p(order.sorted) if gather else None, order.top if gather else 1,
-                                        EXPERTS_TILE, _p(_tc_status_word(a.device)), _stream()), "gemm_experts")
+                                        EXPERTS_TILE, _p(_tc_status_word(a.device)), _stream(), *limit), "gemm_experts")
         return out
     args = (_p(a), _p(w), _p(out), E, order.n_items, n_out, k, int(gated), ACT_CODES[act], ll(a.stride(0)), ll(0), ll(n_out), ll(0),
             ll(w_rows * k), _p(order.offsets), _p(order.tile_group), _p(order.tile_row0), order.tile_group.numel(),

@@ -106,12 +106,8 @@ class RoutedExperts(FeedForward):
         else:
             experts, weights, gate = ops.moe_route(h, self.w_router, self.top, ctx.positions, self.w_sg, **self.rule)
         order = ops.moe_sort(experts, self.n_experts)
-        if self.limit is not None:
-            # gate | up of every item as the product leaves them, then the clamped unit over the rows
-            u = ops.gated_clamped_act(ops.gemm_experts(h, self.w_gu, order, gather=True), None, self.limit, self.alpha,
-                                      self.shift)
-        else:
-            u = ops.gemm_experts(h, self.w_gu, order, gather=True, gated=self.gated, act=self.activation)
+        clamp = (self.limit, self.alpha, self.shift) if self.limit is not None else None
+        u = ops.gemm_experts(h, self.w_gu, order, gather=True, gated=self.gated, act=self.activation, clamp=clamp)
         y = ops.gemm_experts(u, self.w_down, order, gather=False)
         some = dict(experts=experts, n_real=self.n_experts, identity=h) if self.n_identity else {}
         return ops.ExpertSum(y, order, weights, **some), gate

@@ -54,6 +54,28 @@ def test_products_in_every_tile(tile, gather, gated, act, k, n_out, counts, monk
         assert torch.all((got[lo:hi] - z).abs() <= bound), (e, float(((got[lo:hi] - z).abs() - bound).max()))
 
 
+@pytest.mark.parametrize("tile", [0, 64, 128, 256])
+@pytest.mark.parametrize("clamp", [(7.0, 1.0, 1.0), (0.5, 1.702, 0.0), (1e30, 3.0, -1.0), (-1.0, 1.0, 1.0)])
+@pytest.mark.parametrize("k,n_out,counts", [(200, 200, [33, 0, 129]), (1032, 31, [1]), (64, 136, [256, 5, 2])])
+def test_the_clamped_unit_in_the_epilogue(tile, clamp, k, n_out, counts, monkeypatch):
+    """The unit over the product's rows as they are stored, up to a neighbouring quotient: one bfloat16 of the result."""
+    from swifttransformer_b200 import ops
+    monkeypatch.setattr(ops, "EXPERTS_TILE", tile)
+    gen = torch.Generator().manual_seed(k + n_out)
+    order, tokens = order_of(counts, 2, gen)
+    a = torch.randn((tokens, k), generator=gen).to(torch.bfloat16).cuda()
+    w = (torch.randn((len(counts), 2 * n_out, k), generator=gen) * 4 * k ** -0.5).to(torch.bfloat16).cuda()
+    a[0, 0], a[-1, 1] = float("inf"), float("nan")
+    got = ops.gemm_experts(a, w, order, True, gated=True, clamp=clamp)
+    want = ops.gated_clamped_act(ops.gemm_experts(a, w, order, True), None, *clamp)
+    live = int(order.offsets[-1])
+    got, want = got[:live].float(), want[:live].float()
+    assert torch.equal(got.isnan(), want.isnan())
+    same = (got == want) | want.isnan()
+    assert torch.all(same | ((got - want).abs() <= 2.0 ** -7 * want.abs())) and same.float().mean() > 0.999
+    assert ops.kernel_status(a.device) == 0
+
+
 def test_a_row_does_not_depend_on_its_tile():
     from swifttransformer_b200 import ops
     gen = torch.Generator().manual_seed(1)

@@ -15,22 +15,47 @@
 // kernels between delta_prepare and delta_output: delta_chunk_prepare forms W, U0, the decayed q and k and the matrix of
 // q^T D k of every chunk side by side; delta_chunk_walk carries the state from chunk to chunk, a block per head and 8 or 16
 // of its value columns, as two products per chunk, and leaves U and the state before every chunk; delta_chunk_out forms the
-// outputs.  All of it is float arithmetic, and every factor is a product of decays (at most 1), none a quotient.
+// outputs.  The walk's products run on the tensor cores, every float as the sum of three bfloat16 numbers (float_parts.cuh), the
+// rest is float arithmetic, and every factor is a product of decays (at most 1), none a quotient.
 //
-// Measured on one B200, the whole operation with delta_prepare (56 us) and delta_output (24): 2000 tokens of one request, 8
-// heads of 128 x 128, 283 us (prepare 55, walk 113, out 30) against 673 for the walk token by token (delta_scan 584); 16 heads
-// 496 / 892; 500 tokens of 8 heads 126 / 194; 300: 119 / 138; 200: 100 / 93, so portions of fewer than 256 tokens stay with
-// the walk.  Errors against 64 bits: outputs 2.24e-7 (walk 2.33e-7), states 3.34e-7 (3.67e-7).
+// Measured on one B200, 2000 tokens of one request, 8 heads of 128 x 128: prepare 53 us, walk 57, out 26, with delta_prepare (20)
+// and delta_output (15) 169 us.  The walk on the float unit, 256 threads that copied W and K into shared memory, took 110; with
+// the cells' parts formed in the walk itself, 256 threads, 74.  Errors against 64 bits: outputs 2.17e-7 (walk on the
+// float unit 2.18e-7, token by token 2.33e-7), states 3.10e-7 (3.11e-7).  16 heads 178 us (281).  Portions of fewer than 256 tokens stay with the walk
+// token by token.
 #include "chunks.cuh"
 #include "delta_rule.cuh"
+#include "float_parts.cuh"
+#include "mma_sync.cuh"
 
 struct ChunkScratch {
-    float *W, *U, *Q, *K, *A, *P, *S;      // per (place, head): [64][dim], [64][vd], [64][dim], [64][dim], [64][64], [dim], [dim][vd]
+    uint4 *W, *K;                          // per (place, head): cells of W and K^T, see below
+    float *Q, *A, *P, *S;                  // [64][dim], [64][64], [dim], [dim][vd]
+    float* U;                              // [token][head][vd], where the outputs will stand: U0, then U
 };
+
+// W [64][dim] and the transpose of K [64][dim] are left operands of the walk's products: cells of 16 x 16, every float as three
+// bfloat16 numbers (float_parts.cuh), in the order of mma.m16n8k16's registers: [cell][part][lane] of 16 bytes.  W's cell (token
+// block, channel block) is number token * dc_blocks + channel, K^T's (channel block, token block) channel * 4 + token.
+#define DC_CELL 96                         // of 16 bytes
+__host__ __device__ __forceinline__ int dc_blocks(int dim) { return (dim + 15) / 16; }
+__host__ __device__ __forceinline__ long long dc_cells(int dim) { return (long long)dc_blocks(dim) * (HK_C / 16) * DC_CELL; }
 
 // element (t, e) of the unpadded rows of delta_chunk_prepare: pieces of four turned by the row, so that reads of one piece of
 // eight rows hit distinct banks
 __device__ __forceinline__ int dc_at(int t, int e) { return t * HK_D + (e ^ ((t & 7) << 2)); }
+
+// a lane's part of a cell
+__device__ __forceinline__ void dc_cell(uint4* to, float2 a, float2 b, float2 c, float2 d) {
+    uint4 hi, mid, lo;
+    gf_split(a.x, a.y, hi.x, mid.x, lo.x);
+    gf_split(b.x, b.y, hi.y, mid.y, lo.y);
+    gf_split(c.x, c.y, hi.z, mid.z, lo.z);
+    gf_split(d.x, d.y, hi.w, mid.w, lo.w);
+    to[0] = hi;
+    to[32] = mid;
+    to[64] = lo;
+}
 
 struct DcPrepareSmem {
     float Q[HK_C * HK_D], K[HK_C * HK_D], F[HK_C * HK_D], AM[HK_C * HK_C], total[2][HK_D];
@@ -180,20 +205,26 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, const DeltaShape sh, 
     __syncthreads();
     {   // the decayed q and k and A leave
         float* Qd = cs.Q + unit * HK_C * dim;
-        float* Kd = cs.K + unit * HK_C * dim;
         float* A = cs.A + unit * HK_C * HK_C;
         if (e4 < dim) {
             const float4 w0 = load4(m.total[0] + e4), w1 = load4(m.total[1] + e4);
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
                 const int t = t8 + 8 * i;
-                float4 q = load4(m.Q + dc_at(t, e4)), k = load4(m.F + dc_at(t, e4));
+                float4 q = load4(m.Q + dc_at(t, e4));
                 if (i >= 4) q = make_float4(q.x * w0.x, q.y * w0.y, q.z * w0.z, q.w * w0.w);
-                else k = make_float4(k.x * w1.x, k.y * w1.y, k.z * w1.z, k.w * w1.w);
                 store4(Qd + t * dim + e4, q);
-                store4(Kd + t * dim + e4, k);
             }
             if (t8 == 0) store4(cs.P + unit * dim + e4, make_float4(w0.x * w1.x, w0.y * w1.y, w0.z * w1.z, w0.w * w1.w));
+        }
+        uint4* K = cs.K + unit * dc_cells(dim);
+#pragma unroll 2
+        for (int i = warp; i < dc_blocks(dim) * 4; i += 8) {
+            const int c = (i >> 2) * 16 + (lane >> 2), t = (i & 3) * 16 + (lane & 3) * 2;
+            const float w0 = t < HK_H ? m.total[1][c] : 1.f, w1 = t < HK_H ? m.total[1][c + 8] : 1.f;
+            dc_cell(K + i * DC_CELL + lane, make_float2(m.F[dc_at(t, c)] * w0, m.F[dc_at(t + 1, c)] * w0),
+                    make_float2(m.F[dc_at(t, c + 8)] * w1, m.F[dc_at(t + 1, c + 8)] * w1), make_float2(m.F[dc_at(t + 8, c)] * w0, m.F[dc_at(t + 9, c)] * w0),
+                    make_float2(m.F[dc_at(t + 8, c + 8)] * w1, m.F[dc_at(t + 9, c + 8)] * w1));
         }
         for (int i = tid; i < HK_C * HK_C / 4; i += 256) {
             const int t = i / (HK_C / 4), s = (i % (HK_C / 4)) * 4;
@@ -217,181 +248,326 @@ delta_chunk_prepare_kernel(const float* __restrict__ prep, const DeltaShape sh, 
         const bool for_w = tid < HK_D;
         const int c = tid & (HK_D - 1);
         if (c < (for_w ? dim : vd)) {
-            const float* right = for_w ? m.K : m.F;
+            float* right = for_w ? m.K : m.F;             // (each x takes the place of its right side)
             const float w0 = for_w ? m.total[0][c] : 1.f;
-            float* dst = for_w ? cs.W + unit * HK_C * dim + c : cs.U + unit * HK_C * vd + c;
-            const int ld = for_w ? dim : vd;
-            float y[HK_C];
+#pragma unroll 1
+            for (int t0 = 0; t0 < HK_C; t0 += 16) {
+                float y[16];
 #pragma unroll
-            for (int t = 0; t < HK_C; ++t) y[t] = 0.f;
+                for (int t = 0; t < 16; ++t) y[t] = 0.f;
+#pragma unroll 2
+                for (int s = 0; s < t0; ++s) {
+                    const float x = right[dc_at(s, c)];
 #pragma unroll
-            for (int s = 0; s < HK_C; ++s) {
-                const float x = m.Q[s] * (right[dc_at(s, c)] * (s >= HK_H ? w0 : 1.f) - y[s]);
-                dst[s * ld] = x;
-#pragma unroll
-                for (int t = s / 4 * 4; t < HK_C; t += 4) {
-                    if (t + 3 <= s) continue;
-                    const float4 w = load4(m.AM + s * HK_C + t);
-                    if (t > s) y[t] = fmaf(w.x, x, y[t]);
-                    if (t + 1 > s) y[t + 1] = fmaf(w.y, x, y[t + 1]);
-                    if (t + 2 > s) y[t + 2] = fmaf(w.z, x, y[t + 2]);
-                    y[t + 3] = fmaf(w.w, x, y[t + 3]);
+                    for (int t = 0; t < 16; t += 4) {
+                        const float4 w = load4(m.AM + s * HK_C + t0 + t);
+                        y[t] = fmaf(w.x, x, y[t]);
+                        y[t + 1] = fmaf(w.y, x, y[t + 1]);
+                        y[t + 2] = fmaf(w.z, x, y[t + 2]);
+                        y[t + 3] = fmaf(w.w, x, y[t + 3]);
+                    }
                 }
+                const float wt = t0 >= HK_H ? w0 : 1.f;
+                float z[16];
+#pragma unroll
+                for (int s = 0; s < 16; ++s) z[s] = right[dc_at(t0 + s, c)] * wt;
+#pragma unroll
+                for (int s = 0; s < 16; ++s) {
+                    const float x = m.Q[t0 + s] * (z[s] - y[s]);
+                    z[s] = x;
+#pragma unroll
+                    for (int t = s / 4 * 4; t < 16; t += 4) {
+                        if (t + 3 <= s) continue;
+                        const float4 w = load4(m.AM + (t0 + s) * HK_C + t0 + t);
+                        if (t > s) y[t] = fmaf(w.x, x, y[t]);
+                        if (t + 1 > s) y[t + 1] = fmaf(w.y, x, y[t + 1]);
+                        if (t + 2 > s) y[t + 2] = fmaf(w.z, x, y[t + 2]);
+                        y[t + 3] = fmaf(w.w, x, y[t + 3]);
+                    }
+                }
+#pragma unroll
+                for (int s = 0; s < 16; ++s) right[dc_at(t0 + s, c)] = z[s];
             }
         }
+    }
+    __syncthreads();
+    if (e4 < vd)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = t8 + 8 * i;
+            if (t < n) store4(cs.U + ((size_t)(first + t) * sh.H + h) * vd + e4, load4(m.F + dc_at(t, e4)));
+        }
+    uint4* W = cs.W + unit * dc_cells(dim);
+    const int blocks = dc_blocks(dim);
+#pragma unroll 2
+    for (int i = warp; i < blocks * 4; i += 8) {
+        const int t = i / blocks * 16 + (lane >> 2), c = i % blocks * 16 + (lane & 3) * 2;
+        auto two = [&](int t, int c) { return *reinterpret_cast<const float2*>(m.K + dc_at(t, c)); };
+        dc_cell(W + i * DC_CELL + lane, two(t, c), two(t + 8, c), two(t, c + 8), two(t + 8, c + 8));
     }
     ST_PDL_TRIGGER();
 }
 
 // ---- the state from chunk to chunk ------------------------------------------------------------------------------
-// A block carries VS = 4 NC columns of a head's state through a request's chunks: U = U0 - W S (K split over four lanes), then
-// S <- P S + K^T U (the tokens split over two).  W and K of the next chunk are copied meanwhile.  Bound by its two products'
-// reads of shared memory and two barriers per chunk.
-template <int NC>
+// A block carries 8 NT columns of a head's state through a request's chunks: U = U0 - W S, then S <- P S + K^T U, on the tensor
+// cores, every float as three bfloat16 numbers and six products of them per step of sixteen; the highest parts' products have two
+// accumulators by turns, the others three, added up in float (one accumulator for all, or one for the highest, is off by more than
+// the float unit was).  Eight warps hold W, sixteen tokens and half of the channels each, eight K^T and the state, sixteen channels
+// each.  S and U pass between them through shared memory in the order of the right operand's registers, [columns][block of
+// 16][part][lane], two barriers per chunk; while eight warps multiply the others ask for the cells of the chunk after next.
+//
+// Bound by the way of the cells into shared memory (98 KB a chunk and block, some 41 bytes a clock) and by the chain of products,
+// sums, parts and barriers.  With the cells in registers straight from memory every load held up the next product: 185 us.
+template <int NT>
 struct DcWalkSmem {
-    static constexpr int VS = 4 * NC;
-    float W[2][HK_C * HK_LD], K[2][HK_C * HK_LD], U[HK_C * VS], S[VS * 144];     // S transposed: [VS][128 + 16]
+    uint4 cells[2][16][12][32];            // [chunk & 1][warp][..][lane]: every lane copies what it reads itself
+    float2 u0[2][2][NT][128];
+    float decay[2][2][256];
+    float4 half[4][NT][32];                // W S over the second half of the channels
+    uint2 S[NT][8][3][32], U[NT][4][3][32];
 };
+__device__ __forceinline__ void dc_copy8(float2* dst, const float* src, bool on) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 8 : 0) : "memory");
+}
+__device__ __forceinline__ void dc_copy4(float* dst, const float* src, bool on) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(on ? 4 : 0) : "memory");
+}
 
-template <int NC>
-__global__ void __launch_bounds__(256, 1)
+// the 16 x 8 block x of a right operand, rows (lane >> 2) and + 8, columns 2 (lane & 3) and + 1, as parts in its registers' order
+__device__ __forceinline__ void dc_put(uint2 (*dst)[32], const float (&x)[4], int lane) {
+    const bool odd = lane & 4;
+    uint2 hi, mid, lo;
+    const float r0 = __shfl_xor_sync(0xffffffffu, odd ? x[0] : x[1], 4), r1 = __shfl_xor_sync(0xffffffffu, odd ? x[2] : x[3], 4);
+    gf_split(odd ? r0 : x[0], odd ? x[1] : r0, hi.x, mid.x, lo.x);
+    gf_split(odd ? r1 : x[2], odd ? x[3] : r1, hi.y, mid.y, lo.y);
+    const int at = ((lane & 3) * 2 + (lane >> 2 & 1)) * 4 + (lane >> 3);
+    dst[0][at] = hi;
+    dst[1][at] = mid;
+    dst[2][at] = lo;
+}
+// the six products of a cell with the parts b of a right operand, the highest parts' by turns in one accumulator or the other
+__device__ __forceinline__ void dc_products(float (&acc)[6][4], int turn, const uint4 (&a)[3], const uint2 (&b)[3]) {
+    mma_bf16(acc[4], &a[1].x, b[1].x, b[1].y);
+    mma_bf16(acc[turn & 1], &a[0].x, b[0].x, b[0].y);
+    mma_bf16(acc[2], &a[0].x, b[1].x, b[1].y);
+    mma_bf16(acc[4], &a[2].x, b[0].x, b[0].y);
+    mma_bf16(acc[3], &a[1].x, b[0].x, b[0].y);
+    mma_bf16(acc[5], &a[0].x, b[2].x, b[2].y);
+}
+__device__ __forceinline__ float dc_sum(const float (&acc)[6][4], int i) {
+    return (acc[0][i] + acc[1][i]) + ((acc[2][i] + acc[3][i]) + (acc[4][i] + acc[5][i]));
+}
+// Sums that are not finite, as chains over their n products give them: rows r and r + 8 of the cells from `cells` on, whose columns go
+// on by a cell every sixteen, with every `step`-th float from x on and from x + 1 on.  (What is no number stays none.)
+__device__ __forceinline__ float dc_chain(const uint4* cells, int r, int n, const float* x, size_t step) {
+    float v = 0.f;
+    for (int c = 0; c < n && v == v; ++c) {
+        const bf16* at = reinterpret_cast<const bf16*>(cells + (c >> 4) * DC_CELL + (r & 7) * 4 + (c >> 1 & 3)) + ((r >> 3) + 2 * (c >> 3 & 1)) * 2 + (c & 1);
+        float w = to_f32(at[0]);
+        if (fabsf(w) < INFINITY) w = (w + to_f32(at[256])) + to_f32(at[512]);
+        v = fmaf(w, __ldcg(x + c * step), v);
+    }
+    return v;
+}
+
+__device__ __noinline__ float4 dc_chains(float4 y, const uint4* cells, int r, int n, const float* x, size_t step) {
+#pragma unroll 1
+    for (int i = 0; i < 4; ++i) {
+        if (!(fabsf(y.x) < INFINITY)) y.x = dc_chain(cells, r + 8 * (i >> 1), n, x + (i & 1), step);
+        y = make_float4(y.y, y.z, y.w, y.x);
+    }
+    return y;
+}
+
+template <int NT>
+__global__ void __launch_bounds__(512, 1)
 delta_chunk_walk_kernel(const DeltaShape sh, const ChunkScratch cs, float* __restrict__ state, int write_state,
                         const int* __restrict__ positions, const int* __restrict__ q_start, const int* __restrict__ slots, int from) {
-    using M = DcWalkSmem<NC>;
-    constexpr int VS = M::VS;
     extern __shared__ __align__(16) unsigned char dc_raw[];
-    M& m = *reinterpret_cast<M*>(dc_raw);
+    DcWalkSmem<NT>& m = *reinterpret_cast<DcWalkSmem<NT>*>(dc_raw);
     ST_PDL_WAIT();
-    const int b = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * VS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int begin = q_start[b], n = q_start[b + 1] - begin, dim = sh.dim, vd = sh.vd;
+    const int b = blockIdx.z, h = blockIdx.y, col0 = blockIdx.x * 8 * NT, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, w8 = warp & 7;
+    const bool second = tid >= 256;                        // K^T and the state; the others W
+    const int begin = q_start[b], n = q_start[b + 1] - begin, dim = sh.dim, vd = sh.vd, blocks = dc_blocks(dim);
     if (n < from || positions[begin] < 0) return;
-    const int chunks = (n + HK_C - 1) / HK_C;
-    const size_t unit0 = (size_t)hk_place(begin, b, from) * sh.H + h;      // and one place, sh.H units, further per chunk
-    auto copy = [&](int c) {
-        const float* W = cs.W + (unit0 + (size_t)c * sh.H) * HK_C * dim;
-        const float* K = cs.K + (unit0 + (size_t)c * sh.H) * HK_C * dim;
-        for (int i = tid; i < HK_C * (HK_D / 4); i += 256) {
-            const int t = i / (HK_D / 4), e = (i % (HK_D / 4)) * 4;
-            if (e < dim) {
-                hk_cp16(m.W[c & 1] + t * HK_LD + e, W + t * dim + e);
-                hk_cp16(m.K[c & 1] + t * HK_LD + e, K + t * dim + e);
+    const int chunks = (n + HK_C - 1) / HK_C, g = lane >> 2, col = col0 + (lane & 3) * 2;
+    const size_t unit0 = (size_t)hk_place(begin, b, from) * sh.H + h, cells = dc_cells(dim);      // and sh.H units further per chunk
+    // a warp's four cells: of channels 16 w8 and all tokens, or of tokens 16 (w8 % 4) and one half or the other of the channels
+    const int tile = w8 & 3, upper = w8 >> 2;
+    const int cell0 = second ? w8 * 4 : tile * blocks + 4 * upper, n_cells = second ? (w8 < blocks ? 4 : 0) : min(max(blocks - 4 * upper, 0), 4);
+    const uint4* at = (second ? cs.K : cs.W) + unit0 * cells + (size_t)cell0 * DC_CELL;      // those of the chunk at hand
+    const size_t u_row = (size_t)sh.H * vd, on = sh.H * cells;
+    float* u = cs.U + ((size_t)begin * sh.H + h) * vd;     // the chunk's first row
+    float* before = cs.S + unit0 * dim * vd;               // the state before the chunk
+    float* st = state + ((size_t)slots[b] * sh.H + h) * dim * vd;
+    float s[NT][4];                                        // rows 16 w8 + g and + 8, columns col + 8 i and + 1
+    float p[2];                                            // and the rows' decays
+    float2 u0[2][NT];                                      // tokens 16 tile + g and + 8, the same columns
+    auto copy = [&](int c) {                               // asks for chunk c, in the place of chunk c - 2, had long ago
+        asm volatile("" ::: "memory");
+        if (c < chunks) {
+            const uint4* cell = (second ? cs.K : cs.W) + unit0 * cells + c * on + (size_t)cell0 * DC_CELL + lane;
+#pragma unroll 3
+            for (int i = 0; i < 3 * n_cells; ++i)
+                hk_cp16(reinterpret_cast<float*>(&m.cells[c & 1][warp][i][lane]), reinterpret_cast<const float*>(cell + i * 32));
+            if (second) {
+                const float* decay = cs.P + (unit0 + (size_t)c * sh.H) * dim;
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int r = 16 * w8 + 8 * x + g;
+                    dc_copy4(&m.decay[c & 1][x][tid & 255], decay + (r < dim ? r : 0), r < dim);
+                }
+            } else if (!upper) {
+                const float* row = cs.U + ((size_t)begin * sh.H + h) * vd;
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int i = 0; i < NT; ++i) {
+                        const int t = c * HK_C + 16 * tile + g + 8 * r;
+                        const bool in = t < n && col + 8 * i < vd;
+                        dc_copy8(&m.u0[c & 1][r][i][tid], row + (in ? t * u_row + col + 8 * i : 0), in);
+                    }
             }
         }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    auto take = [&](int c) {                               // and has it, in parts
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+        if (second) {
+#pragma unroll
+            for (int x = 0; x < 2; ++x) p[x] = m.decay[c & 1][x][tid & 255];
+        } else if (!upper) {
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int i = 0; i < NT; ++i) u0[r][i] = m.u0[c & 1][r][i][tid];
+        }
+    };
+    // the warp's cells times the right operand's blocks from x on
+    auto products = [&](int c, const uint2 (*x)[3][32], float (&y)[4]) {
+        const uint4* a = m.cells[c & 1][warp][0] + lane;
+        float acc[6][4] = {};
+#pragma unroll 1
+        for (int i = 0; i < n_cells; i += 2) {
+            const uint4 f0[3] = {a[0], a[32], a[64]}, f1[3] = {a[96], a[128], a[160]};
+            const uint2 v0[3] = {x[i][0][lane], x[i][1][lane], x[i][2][lane]}, v1[3] = {x[i + 1][0][lane], x[i + 1][1][lane], x[i + 1][2][lane]};
+            dc_products(acc, 0, f0, v0);
+            if (i + 1 < n_cells) dc_products(acc, 1, f1, v1);
+            a += 192;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y[i] = dc_sum(acc, i);
+    };
+    auto put_state = [&](float* dst) {
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                const int c = 16 * w8 + 8 * x + g;
+                if (c < dim && col + 8 * i < vd) *reinterpret_cast<float2*>(dst + (size_t)c * vd + col + 8 * i) = make_float2(s[i][2 * x], s[i][2 * x + 1]);
+            }
     };
     copy(0);
-    asm volatile("cp.async.commit_group;\n" ::);
-    // rows of S past dim stay zero, and so do the copied rows' places there
-    for (int i = tid; i < VS * 144; i += 256) m.S[i] = 0.f;
-    for (int i = tid; i < HK_C * HK_LD; i += 256)
-        if (i % HK_LD >= dim) m.W[0][i] = m.W[1][i] = m.K[0][i] = m.K[1][i] = 0.f;
-    __syncthreads();
-    // for S: a thread's rows 4 ig .., columns NC cg .., tokens of parity kp
-    const int kp = lane & 1, cg = (lane >> 1) & 3, ig = warp * 4 + (lane >> 3);
-    const bool live = ig * 4 < dim;
-    float s[4][NC];
-    float* st = state + ((size_t)slots[b] * sh.H + h) * dim * vd + col0;
+    if (second) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+        for (int x = 0; x < 2; ++x)
 #pragma unroll
-        for (int j = 0; j < NC; ++j) {
-            s[i][j] = live && col0 + cg * NC + j < vd ? __ldcg(st + (size_t)(ig * 4 + i) * vd + cg * NC + j) : 0.f;
-            if (kp == 0) m.S[(cg * NC + j) * 144 + ig * 4 + i] = s[i][j];
-        }
-    // for U: a thread's tokens tr + 16 i, columns NC cu .., dimensions 16 j + 4 kg .. ; of the finished sums it keeps token tr + 16 kg
-    const int tr = warp * 2 + (lane & 1), cu = (lane >> 1) & 3, kg = lane >> 3;
-    const int t_mine = tr + 16 * kg;
-    float u0[NC], p[4];
-    auto fetch = [&](int c) {
-        const size_t unit = unit0 + (size_t)c * sh.H;
-#pragma unroll
-        for (int j = 0; j < NC; ++j)
-            u0[j] = col0 + cu * NC + j < vd ? __ldcg(cs.U + (unit * HK_C + t_mine) * vd + col0 + cu * NC + j) : 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) p[i] = live ? __ldcg(cs.P + unit * dim + ig * 4 + i) : 0.f;
-    };
-    fetch(0);
-    for (int c = 0; c < chunks; ++c) {
-        const size_t unit = unit0 + (size_t)c * sh.H;
-        asm volatile("cp.async.wait_group 0;\n" ::);
-        __syncthreads();                                  // W, K of this chunk and S; everyone is done with the chunk before
-        if (c + 1 < chunks) copy(c + 1);
-        asm volatile("cp.async.commit_group;\n" ::);
-        if (kp == 0 && live) {                            // the state before the chunk, for the outputs
-            float* dst = cs.S + unit * dim * vd + col0 + cg * NC;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < NC; ++j)
-                    if (col0 + cg * NC + j < vd) dst[(size_t)(ig * 4 + i) * vd + j] = s[i][j];
-        }
-        float a[4][NC] = {};
-        {
-            const float* W = m.W[c & 1];
-#pragma unroll 2
-            for (int e = kg * 4; e < HK_D; e += 16) {
-                float4 w[4], x[NC];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) w[i] = load4(W + (tr + 16 * i) * HK_LD + e);
-#pragma unroll
-                for (int j = 0; j < NC; ++j) x[j] = load4(m.S + (cu * NC + j) * 144 + e);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < NC; ++j)
-                        a[i][j] += fmaf(w[i].x, x[j].x, fmaf(w[i].y, x[j].y, fmaf(w[i].z, x[j].z, w[i].w * x[j].w)));
+            for (int i = 0; i < NT; ++i) {
+                const int c = 16 * w8 + 8 * x + g;
+                const bool in = c < dim && col + 8 * i < vd;
+                const float2 v = in ? __ldcg(reinterpret_cast<const float2*>(st + (size_t)c * vd + col + 8 * i)) : make_float2(0.f, 0.f);
+                s[i][2 * x] = v.x;
+                s[i][2 * x + 1] = v.y;
             }
-        }
 #pragma unroll
-        for (int j = 0; j < NC; ++j) {
-            // four tokens' sums over the four lanes of K: a lane passes on those it does not keep
-            const bool up16 = lane & 16, up8 = lane & 8;
-            const float x0 = (up16 ? a[2][j] : a[0][j]) + __shfl_xor_sync(0xffffffffu, up16 ? a[0][j] : a[2][j], 16);
-            const float x1 = (up16 ? a[3][j] : a[1][j]) + __shfl_xor_sync(0xffffffffu, up16 ? a[1][j] : a[3][j], 16);
-            const float y = (up8 ? x1 : x0) + __shfl_xor_sync(0xffffffffu, up8 ? x0 : x1, 8);
-            const float u = u0[j] - y;
-            m.U[t_mine * VS + cu * NC + j] = u;
-            if (col0 + cu * NC + j < vd) cs.U[(unit * HK_C + t_mine) * vd + col0 + cu * NC + j] = u;
-        }
-        float pc[4];
+        for (int i = 0; i < NT; ++i) dc_put(m.S[i][w8], s[i], lane);
+        put_state(before);
+    } else {
+        copy(1);
+        take(0);
+    }
+    for (int c = 0; c < chunks; ++c) {
+        const bool more = c + 1 < chunks;
+        __syncthreads();                                   // S
+        if (second) {
+            copy(c + 1);
+            take(c);
+        } else {
+            float y[NT][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) pc[i] = p[i];
-        __syncthreads();
-        if (c + 1 < chunks) fetch(c + 1);
-        float d[4][NC] = {};
-        {
-            const float* K = m.K[c & 1] + ig * 4;
-#pragma unroll 4
-            for (int t = kp; t < HK_C; t += 2) {
-                const float4 k = load4(K + t * HK_LD);
-                float u[NC];
+            for (int j = 0; j < NT; ++j) products(c, &m.S[j][4 * upper], y[j]);
+            if (upper) {
 #pragma unroll
-                for (int j = 0; j < NC; ++j) u[j] = m.U[t * VS + cg * NC + j];
+                for (int j = 0; j < NT; ++j) m.half[tile][j][lane] = make_float4(y[j][0], y[j][1], y[j][2], y[j][3]);
+                asm volatile("bar.arrive %0, 64;\n" ::"r"(1 + tile) : "memory");
+            } else {
+                asm volatile("bar.sync %0, 64;\n" ::"r"(1 + tile) : "memory");
+                bool odd = false;
 #pragma unroll
-                for (int j = 0; j < NC; ++j) {
-                    d[0][j] = fmaf(k.x, u[j], d[0][j]);
-                    d[1][j] = fmaf(k.y, u[j], d[1][j]);
-                    d[2][j] = fmaf(k.z, u[j], d[2][j]);
-                    d[3][j] = fmaf(k.w, u[j], d[3][j]);
+                for (int j = 0; j < NT; ++j) {
+                    const float4 z = m.half[tile][j][lane];
+                    y[j][0] += z.x; y[j][1] += z.y; y[j][2] += z.z; y[j][3] += z.w;
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) odd |= !(fabsf(y[j][x]) < INFINITY);
+                }
+                if (odd)
+#pragma unroll
+                    for (int j = 0; j < NT; ++j)
+                        if (col + 8 * j < vd) {
+                            const float4 z = dc_chains(make_float4(y[j][0], y[j][1], y[j][2], y[j][3]), at, g, dim, before + col + 8 * j, vd);
+                            y[j][0] = z.x; y[j][1] = z.y; y[j][2] = z.z; y[j][3] = z.w;
+                        }
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < NT; ++j) {
+                    const float v[4] = {u0[0][j].x - y[j][0], u0[0][j].y - y[j][1], u0[1][j].x - y[j][2], u0[1][j].y - y[j][3]};
+                    dc_put(m.U[j][tile], v, lane);
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const int t = 16 * tile + g + 8 * r;
+                        if (c * HK_C + t < n && col + 8 * j < vd)
+                            *reinterpret_cast<float2*>(u + t * u_row + col + 8 * j) = make_float2(v[2 * r], v[2 * r + 1]);
+                    }
                 }
             }
         }
+        __syncthreads();                                   // U
+        if (second) {
+            float d[NT][4];
+            bool odd = false;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+            for (int i = 0; i < NT; ++i) {
+                products(c, &m.U[i][0], d[i]);
 #pragma unroll
-            for (int j = 0; j < NC; ++j) {
-                d[i][j] += __shfl_xor_sync(0xffffffffu, d[i][j], 1);
-                s[i][j] = fmaf(pc[i], s[i][j], d[i][j]);
+                for (int x = 0; x < 4; ++x) odd |= !(fabsf(d[i][x]) < INFINITY);
             }
-        if (kp == 0 && live)
+            if (odd)
 #pragma unroll
-            for (int j = 0; j < NC; ++j) store4(m.S + (cg * NC + j) * 144 + ig * 4, make_float4(s[0][j], s[1][j], s[2][j], s[3][j]));
+                for (int i = 0; i < NT; ++i)
+                    if (col + 8 * i < vd) {
+                        const float4 z = dc_chains(make_float4(d[i][0], d[i][1], d[i][2], d[i][3]), at, g, min(HK_C, n - c * HK_C), u + col + 8 * i, u_row);
+                        d[i][0] = z.x; d[i][1] = z.y; d[i][2] = z.z; d[i][3] = z.w;
+                    }
+            __syncwarp();
+            before += (size_t)sh.H * dim * vd;
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+#pragma unroll
+                for (int x = 0; x < 4; ++x) s[i][x] = fmaf(p[x >> 1], s[i][x], d[i][x]);
+                if (more) dc_put(m.S[i][w8], s[i], lane);
+            }
+            if (more) put_state(before);                   // the state before the next chunk, for the outputs as well
+        } else {
+            before += (size_t)sh.H * dim * vd;
+            if (more) {
+                copy(c + 2);
+                take(c + 1);
+            }
+        }
+        at += on;
+        u += HK_C * u_row;
     }
-    if (write_state && kp == 0 && live)
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-            for (int j = 0; j < NC; ++j)
-                if (col0 + cg * NC + j < vd) st[(size_t)(ig * 4 + i) * vd + cg * NC + j] = s[i][j];
+    if (write_state && second) put_state(st);
     ST_PDL_TRIGGER();
 }
 
@@ -414,7 +590,7 @@ delta_chunk_out_kernel(const DeltaShape sh, const ChunkScratch cs, float* __rest
     for (int i = tid; i < HK_C * (HK_D / 4); i += 256) {
         const int t = i / (HK_D / 4), e = (i % (HK_D / 4)) * 4;
         if (e < dim) hk_cp16(m.Q + t * HK_LD + e, cs.Q + (unit * HK_C + t) * dim + e);
-        if (e < vd) hk_cp16(m.V + t * HK_LD + e, cs.U + (unit * HK_C + t) * vd + e);
+        if (e < vd && t < n) hk_cp16(m.V + t * HK_LD + e, cs.U + ((size_t)(first + t) * sh.H + h) * vd + e);
     }
     for (int i = tid; i < HK_C * HK_C / 4; i += 256) {
         const int t = i / (HK_C / 4), e = (i % (HK_C / 4)) * 4;
@@ -442,7 +618,7 @@ delta_chunk_out_kernel(const DeltaShape sh, const ChunkScratch cs, float* __rest
 long long delta_chunks_floats(int n_tokens, int n_seqs, const DeltaShape& sh) {
     if (sh.dim % 4 || sh.vd % 4 || sh.dim > HK_D || sh.vd > HK_D || sh.H > 65535 || n_seqs > 65535) return 0;
     return hk_places(n_tokens, n_seqs) * sh.H *
-           ((long long)HK_C * (3 * sh.dim + sh.vd) + HK_C * HK_C + sh.dim + (long long)sh.dim * sh.vd);
+           (2 * 4 * dc_cells(sh.dim) + (long long)HK_C * sh.dim + HK_C * HK_C + sh.dim + (long long)sh.dim * sh.vd);
 }
 
 int delta_chunks_launch(const float* prep, const DeltaShape& sh, float* scratch, float* state, int write_state, float* o,
@@ -452,27 +628,25 @@ int delta_chunks_launch(const float* prep, const DeltaShape& sh, float* scratch,
     ChunkScratch cs;
     float* at = scratch;
     auto take = [&](long long per_unit) { float* p = at; at += units * per_unit; return p; };
-    cs.W = take((long long)HK_C * sh.dim);
-    cs.U = take((long long)HK_C * sh.vd);
+    cs.W = reinterpret_cast<uint4*>(take(4 * dc_cells(sh.dim)));
+    cs.K = reinterpret_cast<uint4*>(take(4 * dc_cells(sh.dim)));
+    cs.U = o;
     cs.Q = take((long long)HK_C * sh.dim);
-    cs.K = take((long long)HK_C * sh.dim);
     cs.A = take(HK_C * HK_C);
     cs.P = take(sh.dim);
     cs.S = take((long long)sh.dim * sh.vd);
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_prepare_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DcPrepareSmem));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DcWalkSmem<1>));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DcWalkSmem<2>));
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DcWalkSmem<4>));
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(DcOutSmem));
     if (e != cudaSuccess) return (int)e;
     int rc = st_launch_pdl("delta_chunks", delta_chunk_prepare_kernel, dim3((unsigned)places, sh.H), dim3(256), sizeof(DcPrepareSmem), s,
                            prep, sh, cs, positions, q_start, n_seqs, from);
     if (rc) return rc;
     if ((long long)n_seqs * sh.H * ((sh.vd + 7) / 8) <= st_sm_count())
-        rc = st_launch_pdl("delta_chunks", delta_chunk_walk_kernel<2>, dim3((sh.vd + 7) / 8, sh.H, n_seqs), dim3(256),
-                           sizeof(DcWalkSmem<2>), s, sh, cs, state, write_state, positions, q_start, slots, from);
+        rc = st_launch_pdl("delta_chunks", delta_chunk_walk_kernel<1>, dim3((sh.vd + 7) / 8, sh.H, n_seqs), dim3(512), sizeof(DcWalkSmem<1>), s, sh, cs, state, write_state, positions, q_start, slots, from);
     else
-        rc = st_launch_pdl("delta_chunks", delta_chunk_walk_kernel<4>, dim3((sh.vd + 15) / 16, sh.H, n_seqs), dim3(256),
-                           sizeof(DcWalkSmem<4>), s, sh, cs, state, write_state, positions, q_start, slots, from);
+        rc = st_launch_pdl("delta_chunks", delta_chunk_walk_kernel<2>, dim3((sh.vd + 15) / 16, sh.H, n_seqs), dim3(512), sizeof(DcWalkSmem<2>), s, sh, cs, state, write_state, positions, q_start, slots, from);
     if (rc) return rc;
     return st_launch_pdl("delta_chunks", delta_chunk_out_kernel, dim3((unsigned)places, sh.H), dim3(256), sizeof(DcOutSmem), s, sh, cs, o,
                          positions, q_start, n_seqs, from);

@@ -19,10 +19,10 @@
 // rest is float arithmetic, and every factor is a product of decays (at most 1), none a quotient.
 //
 // Measured on one B200, 2000 tokens of one request, 8 heads of 128 x 128: prepare 53 us, walk 57, out 26, with delta_prepare (20)
-// and delta_output (15) 169 us.  The walk on the float unit, 256 threads that copied W and K into shared memory, took 110; with
-// the cells' parts formed in the walk itself, 256 threads, 74.  Errors against 64 bits: outputs 2.17e-7 (walk on the
-// float unit 2.18e-7, token by token 2.33e-7), states 3.10e-7 (3.11e-7).  16 heads 178 us (281).  Portions of fewer than 256 tokens stay with the walk
-// token by token.
+// and delta_output (15) 169 us; 16 heads 178 (281 with the walk on the float unit).  The walk on the float unit, 256 threads that
+// copied W and K into shared memory, took 110; with the cells' parts formed in the walk itself, 256 threads, 74.  Errors
+// against 64 bits: outputs 2.17e-7 (walk on the float unit 2.18e-7, token by token 2.33e-7), states 3.10e-7 (3.11e-7).
+// Portions of fewer than 256 tokens stay with the walk token by token.
 #include "chunks.cuh"
 #include "delta_rule.cuh"
 #include "float_parts.cuh"

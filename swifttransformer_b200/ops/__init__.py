@@ -909,6 +909,7 @@ def diff_attention_tiles(q: torch.Tensor, pool: torch.Tensor, layer: int, out: t
 HGRN2_GATES_MIN_TOKENS = 64      # steps of more tokens prepare the recurrence's gates in a kernel of their own
 # Portions of about so many tokens and more run in chunks side by side.  us on one B200, walk / chunks, 16 heads of 128 x 128:
 # one request of 70 tokens 52 / 60, 96 67 / 60, 128 91 / 63; 4 heads 96 52 / 58, 128 67 / 61; 16 requests of 100 tokens 271 / 183.
+# (The chunks' times are those before their products moved to the tensor cores; the line stayed, so that no portion changes form.)
 HGRN2_CHUNK_MIN_TOKENS = 96
 
 def _hgrn2_chunks_from(n: int, n_seqs: int, nh: int, dim: int) -> int:
@@ -1584,6 +1585,7 @@ def gqa_attention_plain(q: torch.Tensor, pool: torch.Tensor, layer: int, out: to
 # Portions of so many tokens and more run in chunks side by side.  us on one B200, walk / chunks, 8 heads of 128 x 128: one
 # request of 200 tokens 81 / 92, 256 97 / 110, 300 116 / 95; two of 260 164 / 113, sixteen 637 / 493; 4 heads of 64 x 64: 256
 # 70 / 74, 300 79 / 74, sixteen of 260 174 / 173.
+# (The chunks' times are those before their walk moved to the tensor cores; the line stayed, so that no portion changes form.)
 DELTA_CHUNK_MIN_TOKENS = 256
 
 

@@ -61,11 +61,7 @@ __device__ __forceinline__ void hk_put(bf16* at, int plane, float4 v, const floa
     *reinterpret_cast<uint2*>(at + plane) = m;
     *reinterpret_cast<uint2*>(at + 2 * plane) = l;
 }
-template <int PLANES> __device__ __forceinline__ float hk_get(const bf16* at, int plane) {
-    float x = to_f32(at[0]);
-    if (PLANES == 3) x = (x + to_f32(at[plane])) + to_f32(at[2 * plane]);
-    return x;
-}
+__device__ __forceinline__ float hk_get(const bf16* at, int plane) { return (to_f32(at[0]) + to_f32(at[plane])) + to_f32(at[2 * plane]); }
 
 // ---- a chunk's sum of k~ v^T [dim][vd] and its product of gates [dim] ----------------------------------------
 // A thread forms k~ of two channels and sixteen tokens: products from its quarter's end backwards, then those of the quarters behind.
@@ -181,14 +177,17 @@ hgrn2_chunk_kv_kernel(const T* __restrict__ proj, const HgrnShape sh, float* __r
             odd |= !(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY);
             if (r < dim && col < vd) *reinterpret_cast<float2*>(dst + (size_t)r * vd + col) = v;
         }
-        if (odd)                                          // sums that are not finite: what a chain over the tokens gives
+        // Sums that are not finite: what a chain over the tokens gives.  It takes the values from the rows: the parts of an infinite
+        // one, or of a float beyond the largest bfloat16, do not add up to it.  (k~ is at most 1 where gates are.)
+        if (odd)
 #pragma unroll 1
             for (int x = 0; x < 64; ++x) {
                 const int r = m0 + 16 * (x >> 5) + 8 * (x >> 1 & 1) + g, col = n0 + 8 * (x >> 2 & 7) + t2 + (x & 1);
                 if (r >= dim || col >= vd || fabsf(dst[(size_t)r * vd + col]) < INFINITY) continue;
+                const T* value = proj + (size_t)first * sh.ld + sh.v_off + h * vd + col;
                 float v = 0.f;
 #pragma unroll 1
-                for (int t = 0; t < n; ++t) v = fmaf(hk_get<3>(K + t * HB_LD + r, PLANE), hk_get<PLANES>(V + t * HB_LD + col, PLANE), v);
+                for (int t = 0; t < n; ++t) v = fmaf(hk_get(K + t * HB_LD + r, PLANE), load1_cg(value + (size_t)t * sh.ld), v);
                 dst[(size_t)r * vd + col] = v;
             }
     }

@@ -29,16 +29,7 @@ struct GemmF32 {
     float* out;
     int n_rows, n_out, k_dim, act;
 };
-__device__ __noinline__ inline float gf_chain(const float* a, const float* w, int k_dim) {
-    float s = 0.f;
-    for (int k = 0; k < k_dim; ++k) s = fmaf(a[k], w[k], s);
-    return s;
-}
-// bias, activation and store of one output; a sum that is not finite gives way to the chain
-__device__ __forceinline__ void gf_store(const GemmF32& p, int row, int col, float v, float bias) {
-    if (!(fabsf(v) < INFINITY)) v = gf_chain(p.a + (size_t)row * p.k_dim, p.w + (size_t)col * p.k_dim, p.k_dim);
-    p.out[(size_t)row * p.n_out + col] = apply_act(p.bias ? v + bias : v, p.act);
-}
+__device__ __forceinline__ float gf_finish(const GemmF32& p, float v, float bias) { return apply_act(p.bias ? v + bias : v, p.act); }
 
 // gemm_f32_few.cu: for up to 8 rows, or in tiles of 16
 #define GF_FEW_ROWS 8

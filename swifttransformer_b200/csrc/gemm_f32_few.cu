@@ -25,6 +25,26 @@ struct GemmFew {
 // 16-byte piece c of row r of a stage: odd rows turned by four pieces, so that the rows of a read's quarter hit distinct banks
 __device__ __forceinline__ int gq_at(int r, int c) { return r * 64 + ((c ^ ((r & 1) << 2)) << 2); }
 
+// a chain over k, left as soon as it is no number (it stays none)
+__device__ __noinline__ float gq_chain(const float* a, const float* w, int k_dim) {
+    float s = 0.f;
+    int k = 0;
+    for (; k + 8 <= k_dim && s == s; k += 8) {
+        float x[8], y[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { x[j] = __ldg(a + k + j); y[j] = __ldg(w + k + j); }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s = fmaf(x[j], y[j], s);
+    }
+    for (; k < k_dim && s == s; ++k) s = fmaf(__ldg(a + k), __ldg(w + k), s);
+    return s;
+}
+// bias, activation and store of one output; a sum that is not finite gives way to the chain
+__device__ __forceinline__ void gq_store(const GemmF32& p, int row, int col, float v, float bias) {
+    if (!(fabsf(v) < INFINITY)) v = gq_chain(p.a + (size_t)row * p.k_dim, p.w + (size_t)col * p.k_dim, p.k_dim);
+    p.out[(size_t)row * p.n_out + col] = gf_finish(p, v, bias);
+}
+
 template <int NB>
 __global__ void __launch_bounds__(32 * GemmFew<NB>::WARPS, NB == 1 ? 2 : 1)
 gemm_f32_few_kernel(const GemmF32 p, int tiles, int row_tiles, int vec_a, int vec_w) {
@@ -138,7 +158,7 @@ gemm_f32_few_kernel(const GemmF32 p, int tiles, int row_tiles, int vec_a, int ve
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
                 const int row = n0 + 8 * b + (tid >> 4);
-                if (row < p.n_rows) gf_store(p, row, col, total[b], bias);
+                if (row < p.n_rows) gq_store(p, row, col, total[b], bias);
             }
         }
     }

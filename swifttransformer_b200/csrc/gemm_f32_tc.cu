@@ -80,14 +80,71 @@ gemm_f32_split_kernel(const float* __restrict__ a, uint4* __restrict__ parts, in
     parts[2 * n + i] = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// Outputs that came out infinite or not a number, again as chains of multiply-adds over k: all threads of a block walk through its tiles
+// once the pipeline has ended, where no warp waits for them under a limit, and multiply every tile that has such an output (128
+// x nt sums side by side, 32 k at a time through the pipeline's shared memory) until all of its sums of interest are no numbers, or
+// to the end.  us for 1000 x 2048 x 8192: 166 where all are finite, 1064 with one infinity among the operands, 3513 with one in every row.
+template <int NT>
+__device__ __noinline__ void gf_chains(const GemmF32Tc& p, float* smem) {
+    constexpr int NR = NT / 16, LD = 33;
+    const GemmF32& q = p.g;
+    float *W = smem, *A = smem + GF_BM * LD;                  // [128][33], [nt][33]
+    const int tid = threadIdx.x, cl = tid & 31, rl = tid >> 5;
+    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
+        const int m0 = tile / p.n_tiles * GF_BM, n0 = tile % p.n_tiles * p.nt;
+        // 512 threads: columns cl + 32 i, rows rl + 16 j; wanted: bit 4 j + i
+        auto out_at = [&](int i, int j) { return q.out + (size_t)(n0 + rl + 16 * j) * q.n_out + m0 + cl + 32 * i; };
+        uint32_t wanted = 0;
+#pragma unroll 1
+        for (int x = 0; x < 4 * NR; ++x) {
+            const int i = x & 3, j = x >> 2;
+            if (rl < 16 && 16 * j < p.nt && n0 + rl + 16 * j < q.n_rows && m0 + cl + 32 * i < q.n_out && !(fabsf(*out_at(i, j)) < INFINITY))
+                wanted |= 1u << x;
+        }
+        if (!__syncthreads_or(wanted != 0)) continue;
+        float s[NR][4] = {};
+#pragma unroll 1
+        for (int k0 = 0; k0 < q.k_dim; k0 += 32) {
+            bool open = false;
+#pragma unroll
+            for (int x = 0; x < 4 * NR; ++x) open |= (wanted >> x & 1) && s[x >> 2][x & 3] == s[x >> 2][x & 3];
+            if (!__syncthreads_or(open)) break;
+            for (int i = rl; i < GF_BM + p.nt; i += blockDim.x / 32) {
+                const bool is_w = i < GF_BM;
+                const int row = is_w ? m0 + i : n0 + i - GF_BM, k = k0 + cl;
+                smem[i * LD + cl] = row < (is_w ? q.n_out : q.n_rows) && k < q.k_dim ? __ldg((is_w ? q.w : q.a) + (size_t)row * q.k_dim + k) : 0.f;
+            }
+            __syncthreads();
+            if (rl < 16)
+#pragma unroll 4
+                for (int k = 0; k < 32; ++k) {
+                    float w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) w[i] = W[(cl + 32 * i) * LD + k];
+#pragma unroll
+                    for (int j = 0; j < NR; ++j) {
+                        if (16 * j >= p.nt) break;
+                        const float a = A[(rl + 16 * j) * LD + k];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) s[j][i] = fmaf(a, w[i], s[j][i]);
+                    }
+                }
+        }
+#pragma unroll
+        for (int x = 0; x < 4 * NR; ++x)
+            if (wanted >> x & 1) *out_at(x & 3, x >> 2) = gf_finish(q, s[x >> 2][x & 3], q.bias ? __ldg(q.bias + m0 + cl + 32 * (x & 3)) : 0.f);
+    }
+}
+
 template <int NT>
 __global__ void __launch_bounds__(GF_THREADS(NT), 1)
-gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map, const GemmF32Tc p, int* status) {
+gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap a_map,
+                   const __grid_constant__ GemmF32Tc p, int* status) {
     extern __shared__ unsigned char gf_raw[];
     // w landed / read; a group's operands in place and its sums' place free; its products complete
     __shared__ __align__(8) unsigned long long s_wfull[GF_MAX_STAGES], s_wfree[GF_MAX_STAGES], s_ready[GF_MAX_BUFS], s_done[GF_MAX_BUFS];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_dead, s_issued;
+    __shared__ int s_dead, s_issued, s_odd;
     constexpr int BUFS = NT <= 64 ? 4 : 2;                   // a power of two
     constexpr int W_COL = NT <= 64 ? 128 : 256;              // tensor memory: sums at 0 and W_COL / 2, parts of w from W_COL on, 96 each
     const GemmF32& q = p.g;
@@ -105,6 +162,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
         tc_mbar_init_fence();
         s_dead = 0;
         s_issued = 0;
+        s_odd = 0;
     }
     if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tc_smem(&s_tmem)), "r"(512) : "memory");
@@ -276,12 +334,14 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
             }
             if (ok && col < q.n_out) {
                 // The registers are stored by unrolled code, which has to be short: with every activation in it 20 us of a tile's
-                // 48 went into fetching instructions.  What is not short is done to the stored sums, one after the other.
+                // 48 went into fetching instructions.  What is not short is done to the stored sums, one after the other; those that
+                // are not finite stay as they are for gf_chains.
                 const float bias = q.bias ? __ldg(q.bias + col) : 0.f;
                 float* dst = q.out + (size_t)n0 * q.n_out + col;
-                bool later = q.act > 1;
+                bool odd = false;
 #pragma unroll
-                for (int j = 0; j < NT / 2; ++j) later |= !(fabsf(acc[j]) < INFINITY);
+                for (int j = 0; j < NT / 2; ++j) odd |= j < live && !(fabsf(acc[j]) < INFINITY);
+                const bool later = odd || q.act > 1;
 #pragma unroll
                 for (int j = 0; j < NT / 2; ++j)
                     if (j < live) {
@@ -290,9 +350,13 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
                         if (!later && q.act == 1) v = v > 0.f ? v : 0.f;
                         dst[(size_t)j * q.n_out] = v;
                     }
+                if (odd) s_odd = 1;
                 if (later)
 #pragma unroll 1
-                    for (int j = 0; j < live; ++j) gf_store(q, n0 + j, col, dst[(size_t)j * q.n_out], bias);
+                    for (int j = 0; j < live; ++j) {
+                        const float v = dst[(size_t)j * q.n_out];
+                        if (fabsf(v) < INFINITY) dst[(size_t)j * q.n_out] = gf_finish(q, v, bias);
+                    }
             }
             __syncwarp();
         }
@@ -307,6 +371,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
         for (int i = 0; i < 20000; ++i) __nanosleep(100);
     }
     __syncthreads();
+    if (s_odd && !s_dead) gf_chains<NT>(p, reinterpret_cast<float*>(gf_raw));
     if (warp == 9) {
         tc_fence_after_sync();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512) : "memory");

@@ -96,7 +96,7 @@ __device__ __forceinline__ bool tc_wait(uint32_t mbar, uint32_t parity) {
 // The same by a whole warp, with one answer for all its lanes, which also ends when the block has been marked dead, and marks it
 // when the limit is reached.  try_wait: the hardware holds the warp until the phase completes or a time of about a microsecond
 // is over, so that waiting warps take no issue slots from working ones.
-#define TC_TRY_LIMIT (1u << 17)       // tries: at least 0.1 s, whatever a try's time is
+#define TC_TRY_LIMIT (1u << 17)       // tries: at least 0.1 s, whatever a try's time is; no warp that others wait for may be busy for long
 __device__ __forceinline__ bool tc_wait_warp(uint32_t mbar, uint32_t parity, volatile int* dead) {
     bool ok = false;
     for (uint32_t i = 0; i < TC_TRY_LIMIT; ++i) {

@@ -58,3 +58,29 @@ def test_operands_that_are_not_finite(rows):
         scale = (np.abs(np.where(np.isfinite(an), an, 0)).astype(np.float64) @ np.abs(np.where(np.isfinite(wn), wn, 0)).T.astype(np.float64))
         assert np.all(np.abs(got[ok].astype(np.float64) - want[ok]) <= (k + 2) * 2.0 ** -23 * scale[ok] + 1e-30)
     assert ops.kernel_status(torch.device("cuda")) == 0
+
+
+@pytest.mark.parametrize("rows,k,outs", [(300, 520, 8200), (1000, 16384, 4096), (64, 768, 21000), (21, 2050, 40000)])
+@pytest.mark.parametrize("act", ["none", "relu", "gelu"])
+def test_rows_that_are_not_finite_in_tiles_one_after_the_other(rows, k, outs, act):
+    """Products whose outputs are for the most part not finite, several tiles a block: all of them are formed, no wait runs out, and the rows
+    beside them have the bits they have alone."""
+    from swifttransformer_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    a, w = torch.randn((rows, k), generator=gen, device="cuda"), torch.randn((outs, k), generator=gen, device="cuda")
+    bias = torch.randn(outs, generator=gen, device="cuda")
+    clean = ops.linear(a, w, bias, act)
+    bad = a.clone()
+    bad[::3, k - 7] = float("inf")                       # infinite outputs, their sign that of the weight
+    bad[1::3, 5] = float("nan")
+    got = ops.linear(bad, w, bias, act)
+    want = clean.clone()
+    want[::3] = torch.where(w[:, k - 7] > 0, float("inf"), float("-inf"))
+    want[1::3] = float("nan")
+    if act == "relu":                                    # (the kernels' is v > 0 ? v : 0)
+        want = torch.where(want > 0, want, 0.0)
+    elif act == "gelu":                                  # -inf times zero
+        want = torch.where(want == float("-inf"), float("nan"), want)
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.all((got == want) | want.isnan())
+    assert ops.kernel_status(a.device) == 0

@@ -355,7 +355,7 @@ __device__ __forceinline__ void dc_products(float (&acc)[6][4], int turn, const 
     mma_bf16(acc[5], &a[0].x, b[2].x, b[2].y);
 }
 __device__ __forceinline__ float dc_sum(const float (&acc)[6][4], int i) {
-    return (acc[0][i] + acc[1][i]) + ((acc[2][i] + acc[3][i]) + (acc[4][i] + acc[5][i]));
+    return ((acc[0][i] + acc[1][i]) + ((acc[2][i] + acc[3][i]) + (acc[4][i] + acc[5][i]))) * GF_DOWN2;
 }
 // Sums that are not finite, as chains over their n products give them: rows r and r + 8 of the cells from `cells` on, whose columns go
 // on by a cell every sixteen, with every `step`-th float from x on and from x + 1 on.  (What is no number stays none.)
@@ -364,7 +364,7 @@ __device__ __forceinline__ float dc_chain(const uint4* cells, int r, int n, cons
     for (int c = 0; c < n && v == v; ++c) {
         const bf16* at = reinterpret_cast<const bf16*>(cells + (c >> 4) * DC_CELL + (r & 7) * 4 + (c >> 1 & 3)) + ((r >> 3) + 2 * (c >> 3 & 1)) * 2 + (c & 1);
         float w = to_f32(at[0]);
-        if (fabsf(w) < INFINITY) w = (w + to_f32(at[256])) + to_f32(at[512]);
+        if (fabsf(w) < INFINITY) w = gf_join(w, to_f32(at[256]), to_f32(at[512]));
         v = fmaf(w, __ldcg(x + c * step), v);
     }
     return v;

@@ -1,8 +1,8 @@
 // The 32-bit matrix product on the tensor cores, out[n, m] = act( sum_k a[n,k] * w[m,k] + bias[m] ) with float operands and
 // w stored [out, in]: what its kernels (gemm_f32_tc.cu for many rows, gemm_f32_few.cu for few) share.
 //
-// A float is the sum of three bfloat16 numbers of eight bits each: x = h + m + l, h = bf16(x), m = bf16(x - h),
-// l = bf16(x - h - m), each difference exact.  Of the nine products of two such sums six are formed,
+// A float, times 2^16, is the sum of three bfloat16 numbers of eight bits each, h + m + l (float_parts.cuh); an output is the sum of their
+// products times 2^-32.  Of the nine products of two such sums six are formed,
 //   w_l a_h + w_h a_l + w_m a_m + w_m a_h + w_h a_m + w_h a_h,
 // each exact in the tensor cores' float accumulator; the three left out are at most 2^-25 of w a together.  The tensor
 // cores cut a sum off where a float addition rounds it (measured: 6e-8 of bias after four steps of 16 k, 1.2e-7 after eight), so a sum
@@ -12,9 +12,8 @@
 // same groups and add them in the same order (mma.sync and tcgen05.mma give the same bits for the same sixteen products; a test
 // holds the kernels to it).
 //
-// An output that comes out infinite or not a number (operands that are, sums that overflow, operands within 2^-8 of the largest
-// float) is computed again as a chain of fused multiply-adds over k, which is what such operands give in plain float.
-// Below 2^-110 in magnitude a number's last bits fall under bfloat16's smallest (2^-133).
+// A sum that comes out infinite or not a number (operands that are, operands from 2^112 on, outputs from 2^96 on) is formed again as
+// a chain of fused multiply-adds over k, which is what such operands give in plain float.
 //
 // Error against 64 bits, relative 2-norm, normal operands: k = 512 9.6e-8, 2048 1.3e-7, 8192 2.2e-7 (a chain of fused multiply-adds
 // over k: 4.0e-7, 8.1e-7, 1.6e-6).

@@ -39,9 +39,10 @@ __device__ __noinline__ float gq_chain(const float* a, const float* w, int k_dim
     for (; k < k_dim && s == s; ++k) s = fmaf(__ldg(a + k), __ldg(w + k), s);
     return s;
 }
-// bias, activation and store of one output; a sum that is not finite gives way to the chain
+// scale, bias, activation and store of one output; a sum that is not finite gives way to the chain
 __device__ __forceinline__ void gq_store(const GemmF32& p, int row, int col, float v, float bias) {
     if (!(fabsf(v) < INFINITY)) v = gq_chain(p.a + (size_t)row * p.k_dim, p.w + (size_t)col * p.k_dim, p.k_dim);
+    else v *= GF_DOWN2;
     p.out[(size_t)row * p.n_out + col] = gf_finish(p, v, bias);
 }
 

@@ -345,7 +345,7 @@ gemm_f32_tc_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
 #pragma unroll
                 for (int j = 0; j < NT / 2; ++j)
                     if (j < live) {
-                        float v = acc[j];
+                        float v = acc[j] * GF_DOWN2;
                         if (!later && q.bias) v += bias;
                         if (!later && q.act == 1) v = v > 0.f ? v : 0.f;
                         dst[(size_t)j * q.n_out] = v;

@@ -42,8 +42,8 @@ __device__ __forceinline__ void store2(bf16* p, float a, float b) { *reinterpret
 __device__ __forceinline__ float hk_gate(float z, float bias, float lo) { return lo + (1.f - lo) * hk_sigmoid(z + bias); }
 
 // ---- the products ------------------------------------------------------------------------------------------------
-// Matrices lie in shared memory as bfloat16 planes of their floats' parts (float_parts.cuh: 0 the highest), rows of HB_LD; values that are
-// bfloat16 have one plane.  A sum of products of two such matrices takes the small products first and is added to what
+// Matrices lie in shared memory as bfloat16 planes of their floats' parts (float_parts.cuh: 0 the highest, all times 2^16), rows of HB_LD;
+// values that are bfloat16 have one plane, as they are.  A sum of products of two such matrices takes the small products first and is added to what
 // it belongs to in float: see gemm_f32.cuh.
 #define HB_LD (HK_D + 8)                       // elements: rows 16 bytes apart modulo 128, so that ldmatrix meets no conflict
 
@@ -61,7 +61,7 @@ __device__ __forceinline__ void hk_put(bf16* at, int plane, float4 v, const floa
     *reinterpret_cast<uint2*>(at + plane) = m;
     *reinterpret_cast<uint2*>(at + 2 * plane) = l;
 }
-__device__ __forceinline__ float hk_get(const bf16* at, int plane) { return (to_f32(at[0]) + to_f32(at[plane])) + to_f32(at[2 * plane]); }
+__device__ __forceinline__ float hk_get(const bf16* at, int plane) { return gf_join(to_f32(at[0]), to_f32(at[plane]), to_f32(at[2 * plane])); }
 
 // ---- a chunk's sum of k~ v^T [dim][vd] and its product of gates [dim] ----------------------------------------
 // A thread forms k~ of two channels and sixteen tokens: products from its quarter's end backwards, then those of the quarters behind.
@@ -173,7 +173,8 @@ hgrn2_chunk_kv_kernel(const T* __restrict__ proj, const HgrnShape sh, float* __r
         for (int x = 0; x < 32; ++x) {
             const int mt = x >> 4, nt = x >> 1 & 7, half = x & 1;
             const int r = m0 + 16 * mt + 8 * half + g, col = n0 + 8 * nt + t2;
-            const float2 v = make_float2(acc[mt][nt][2 * half], acc[mt][nt][2 * half + 1]);
+            const float down = PLANES == 1 ? GF_DOWN : GF_DOWN2;
+            const float2 v = make_float2(acc[mt][nt][2 * half] * down, acc[mt][nt][2 * half + 1] * down);
             odd |= !(fabsf(v.x) < INFINITY && fabsf(v.y) < INFINITY);
             if (r < dim && col < vd) *reinterpret_cast<float2*>(dst + (size_t)r * vd + col) = v;
         }
@@ -452,7 +453,7 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
                     mma_bf16(a, qh, km[0], km[1]);
                     mma_bf16(a, qh, kh[0], kh[1]);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[i * (i - 1) / 2 + j][e] += a[e];
+                    for (int e = 0; e < 4; ++e) acc[i * (i - 1) / 2 + j][e] = fmaf(a[e], GF_DOWN2, acc[i * (i - 1) / 2 + j][e]);
                 }
             }
         }
@@ -591,7 +592,7 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
                 mma_bf16(c, xh, sm[2 * j], sm[2 * j + 1]);
                 mma_bf16(c, xh, sh_[2 * j], sh_[2 * j + 1]);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) acc[2 * nt + j][e] += c[e];
+                for (int e = 0; e < 4; ++e) acc[2 * nt + j][e] = fmaf(c[e], GF_DOWN2, acc[2 * nt + j][e]);
             }
         }
     }
@@ -612,7 +613,7 @@ hgrn2_chunk_out_kernel(const T* __restrict__ proj, const HgrnShape sh, const flo
                     mma_bf16(c, am, v[2 * j], v[2 * j + 1]);
                     mma_bf16(c, ah, v[2 * j], v[2 * j + 1]);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[2 * nt + j][e] += c[e];
+                    for (int e = 0; e < 4; ++e) acc[2 * nt + j][e] = fmaf(c[e], GF_DOWN, acc[2 * nt + j][e]);
                 }
             }
         }

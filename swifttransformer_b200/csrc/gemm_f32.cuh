@@ -30,6 +30,12 @@ struct GemmF32 {
 };
 __device__ __forceinline__ float gf_finish(const GemmF32& p, float v, float bias) { return apply_act(p.bias ? v + bias : v, p.act); }
 
+// gemm_f32_few.cu: chains of multiply-adds, for k below GF_SHORT.  The tensor cores cut a sum off, so a product of one k is off by 4.6e-8 of
+// itself where a float multiplication is by 2.6e-8; k = 2 4.6e-8 (chain 3.0e-8), 4 4.7e-8 (4.0e-8), 8 4.8e-8 (5.3e-8; of positive numbers 4.8e-8 and
+// 4.6e-8), 16 4.7e-8 (7.4e-8).
+#define GF_SHORT 9
+int gf_short_launch(const GemmF32& p, cudaStream_t s);
+
 // gemm_f32_few.cu: for up to 8 rows, or in tiles of 16
 #define GF_FEW_ROWS 8
 #define GF_FEW_MOST 32       // more rows than this it is not asked to take

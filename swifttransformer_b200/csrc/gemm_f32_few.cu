@@ -180,3 +180,31 @@ static int gq_launch(const GemmF32& p, cudaStream_t s) {
     return st_launch_status();
 }
 int gf_few_launch(const GemmF32& p, cudaStream_t s) { return p.n_rows <= GF_FEW_ROWS ? gq_launch<1>(p, s) : gq_launch<2>(p, s); }
+
+// ---- k below GF_SHORT: a thread has a row of w and takes `rows` rows of a, one chain each.  Bound by the launch and, for many rows, by
+// the results' way to memory.
+__global__ void __launch_bounds__(256) gemm_f32_short_kernel(const GemmF32 p, int rows) {
+    const int col = blockIdx.x * 256 + threadIdx.x;
+    if (col >= p.n_out) return;
+    float w[GF_SHORT - 1];
+#pragma unroll
+    for (int k = 0; k < GF_SHORT - 1; ++k) w[k] = k < p.k_dim ? __ldg(p.w + (size_t)col * p.k_dim + k) : 0.f;
+    const float bias = p.bias ? __ldg(p.bias + col) : 0.f;
+    for (long long row0 = (long long)blockIdx.y * rows; row0 < p.n_rows; row0 += (long long)gridDim.y * rows)
+#pragma unroll 4
+        for (int row = (int)row0; row < (row0 + rows < p.n_rows ? row0 + rows : p.n_rows); ++row) {
+            const float* a = p.a + (size_t)row * p.k_dim;
+            float s = 0.f;
+#pragma unroll
+            for (int k = 0; k < GF_SHORT - 1; ++k)
+                if (k < p.k_dim) s = fmaf(__ldg(a + k), w[k], s);
+            p.out[(size_t)row * p.n_out + col] = gf_finish(p, s, bias);
+        }
+}
+int gf_short_launch(const GemmF32& p, cudaStream_t s) {
+    const long long across = (p.n_out + 255LL) / 256;
+    const int rows = across * p.n_rows > 8 * st_sm_count() ? 8 : 1;
+    const long long down = (p.n_rows + rows - 1LL) / rows;
+    gemm_f32_short_kernel<<<dim3((unsigned)across, (unsigned)(down < 65535 ? down : 65535)), 256, 0, s>>>(p, rows);
+    return st_launch_status();
+}

@@ -388,13 +388,14 @@ static int gf_launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const G
 
 // a [n_rows, k_dim], w [n_out, k_dim], out [n_rows, n_out], float and contiguous, of any alignment.  nt: rows of a per tile (a
 // multiple of 16 up to 128; for any number of rows), 0: chosen here.  scratch: 6 n_rows (k_dim rounded up to 64) bytes, 16-byte
-// aligned, and status: both may be null for at most GF_FEW_ROWS rows.
+// aligned, and status: both may be null for at most GF_FEW_ROWS rows and for k below GF_SHORT.
 ST_EXPORT int st_gemm_f32(const float* a, const float* w, const float* bias, float* out, int n_rows, int n_out, int k_dim, int act,
                           int nt, void* scratch, int* status, void* stream) {
     if (n_rows <= 0 || n_out <= 0) return 0;
     if (k_dim <= 0) return ST_ERR_BAD_SIZE;
     const GemmF32 g = {a, w, bias, out, n_rows, n_out, k_dim, act};
     cudaStream_t s = (cudaStream_t)stream;
+    if (nt == 0 && k_dim < GF_SHORT) return gf_short_launch(g, s);
     if (nt == 0 && n_rows <= GF_FEW_ROWS) return gf_few_launch(g, s);
     if (!status || !scratch || !aligned16(scratch) || nt < 0 || nt > 128 || nt % 16) return ST_ERR_BAD_ARG;
     const int sms = st_sm_count();

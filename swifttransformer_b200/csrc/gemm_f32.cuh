@@ -36,7 +36,6 @@ __device__ __forceinline__ float gf_finish(const GemmF32& p, float v, float bias
 #define GF_SHORT 9
 int gf_short_launch(const GemmF32& p, cudaStream_t s);
 
-// gemm_f32_few.cu: for up to 8 rows, or in tiles of 16
-#define GF_FEW_ROWS 8
-#define GF_FEW_MOST 32       // more rows than this it is not asked to take
-int gf_few_launch(const GemmF32& p, cudaStream_t s);
+// the same file: in tiles of 8 or 16 rows (0: what takes less), and about what it takes, in units of 10 ns
+int gf_few_launch(const GemmF32& p, int rows, cudaStream_t s);
+long long gf_few_cost(const GemmF32& p);

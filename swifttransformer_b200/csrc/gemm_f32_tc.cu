@@ -15,10 +15,10 @@
 // of the tensor cores for any nt.  w is split by each block that uses it, for w is the larger operand and read from memory once.
 //
 // Bound by the tensor cores (24 products of 12 nt clocks a group; nt 128: 1670 clocks a group measured, 1536 of them products) and the
-// power limit for prompts, by the chain split - products - sum of a group for few rows.  us on one B200 with 6 us of an empty launch
-// between events, inputs not in cache, in brackets the float multiply-adds that served before: 1000 x 2048 x 8192 148 (770),
-// 1000 x 8192 x 2048 150 (928), 2000 x 4096 x 4096 288 (1521), 300 x 5504 x 2048 69 (240), 100 x 2048 x 8192 36 (127),
-// 64 x 8192 x 2048 77 (96), 33 x 2048 x 2048 28 (29), 64 x 768 x 2304 17.2 (16.4).
+// power limit for prompts, by the chain split - products - sum of a group for few rows.  us on one B200, recorded calls over weights that
+// are not in cache, in brackets the float multiply-adds that served before: 1000 x 2048 x 8192 149 (766; 176 in a run of other work, whose
+// power holds the clock down), 1000 x 8192 x 2048 151 (923), 1000 x 4096 x 4096 148 (773), 128 x 2048 x 8192 32 (123), 64 x 8192 x 2048 74 (92),
+// 33 x 2048 x 2048 22.5 (25.5), 64 x 768 x 2304 12.1 (12.1).
 //
 // Waits are bounded: one that expires marks the block dead, `status` gets 5, and the block waits (again with a limit) for its
 // copies under way, frees its tensor memory and leaves.
@@ -386,35 +386,49 @@ static int gf_launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const G
     return st_launch_pdl("gemm_f32", kernel, dim3((unsigned)grid), dim3(GF_THREADS(NT)), GF_SMEM, s, w_map, a_map, p, status);
 }
 
-// a [n_rows, k_dim], w [n_out, k_dim], out [n_rows, n_out], float and contiguous, of any alignment.  nt: rows of a per tile (a
-// multiple of 16 up to 128; for any number of rows), 0: chosen here.  scratch: 6 n_rows (k_dim rounded up to 64) bytes, 16-byte
-// aligned, and status: both may be null for at most GF_FEW_ROWS rows and for k below GF_SHORT.
+// Rows of a per tile, 0: gemm_f32_few.cu, by what they were measured to take (units of 10 ns, on one B200, recorded calls): a tile's group
+// 46 + nt / 3 up to 64 rows, 50 + nt / 2 above (two sets of splitting warps and two buffers then), a round of tiles 200 beside that and
+// the splitting kernel and the launch 450; twelve times as much for the groups but two where rows of w are not whole pieces of 16 bytes
+// (40 x 770 x 2304 87 us, 40 x 130 x 512 10).  us, this kernel / gemm_f32_few.cu: 16 x 768 x 3072 12.1 / 8.4, 16 x 2048 x 6144 23.5 / 27.6,
+// 24 x 4096 x 4096 40.2 / 52.8, 24 x 8192 x 2048 73 / 55, 1 x 768 x 50272 35 / 41, 64 x 64 x 64 5.7 / 3.5.
+static int gf_plan(const GemmF32& g) {
+    const long long sms = st_sm_count(), m_tiles = ((long long)g.n_out + GF_BM - 1) / GF_BM, n_groups = ((long long)g.k_dim + GF_BK - 1) / GF_BK;
+    const int rows16 = g.n_rows >= 128 ? 128 : (g.n_rows + 15) / 16 * 16;
+    long long best = gf_few_cost(g);
+    int nt = 0;
+    for (int t = 16; t <= rows16; t += 16) {
+        const long long tiles = m_tiles * (((long long)g.n_rows + t - 1) / t);
+        const long long groups = g.k_dim % 4 == 0 || n_groups <= 2 ? n_groups : 12 * (n_groups - 2);
+        const long long cost = 450 + (tiles + sms - 1) / sms * (groups * (t <= 64 ? 46 + t / 3 : 50 + t / 2) + 200);
+        if (cost < best) { best = cost; nt = t; }
+    }
+    return nt;
+}
+
+// Bytes of scratch st_gemm_f32 takes on the current device.
+ST_EXPORT long long st_gemm_f32_scratch(int n_rows, int n_out, int k_dim) {
+    const GemmF32 g = {nullptr, nullptr, nullptr, nullptr, n_rows, n_out, k_dim, 0};
+    if (n_rows <= 0 || n_out <= 0 || k_dim < GF_SHORT || gf_plan(g) == 0) return 0;
+    return 6LL * n_rows * (((long long)k_dim + GF_BK - 1) / GF_BK * GF_BK);
+}
+
+// a [n_rows, k_dim], w [n_out, k_dim], out [n_rows, n_out], float and contiguous, of any alignment.  scratch: 16-byte aligned, with status;
+// both may be null where st_gemm_f32_scratch is 0.  form, for tests: rows of a per tile of this kernel (a multiple of 16 up to 128; scratch
+// 6 n_rows (k_dim rounded up to 64) bytes then), -8 and -16: gemm_f32_few.cu in such tiles, 0: chosen here.
 ST_EXPORT int st_gemm_f32(const float* a, const float* w, const float* bias, float* out, int n_rows, int n_out, int k_dim, int act,
-                          int nt, void* scratch, int* status, void* stream) {
+                          int form, void* scratch, int* status, void* stream) {
     if (n_rows <= 0 || n_out <= 0) return 0;
     if (k_dim <= 0) return ST_ERR_BAD_SIZE;
     const GemmF32 g = {a, w, bias, out, n_rows, n_out, k_dim, act};
     cudaStream_t s = (cudaStream_t)stream;
-    if (nt == 0 && k_dim < GF_SHORT) return gf_short_launch(g, s);
-    if (nt == 0 && n_rows <= GF_FEW_ROWS) return gf_few_launch(g, s);
+    if (form == 0 && k_dim < GF_SHORT) return gf_short_launch(g, s);
+    if (form == -8 || form == -16) return gf_few_launch(g, -form, s);
+    const int nt = form == 0 ? gf_plan(g) : form;
+    if (nt == 0) return gf_few_launch(g, 0, s);
     if (!status || !scratch || !aligned16(scratch) || nt < 0 || nt > 128 || nt % 16) return ST_ERR_BAD_ARG;
     const int sms = st_sm_count();
     const long long m_tiles = ((long long)n_out + GF_BM - 1) / GF_BM, n_groups = ((long long)k_dim + GF_BK - 1) / GF_BK;
     const long long k_pad = n_groups * GF_BK;
-    if (nt == 0) {
-        // Rows per tile, and up to 32 rows which kernel, by what they were measured to take (in units of 10 ns, on one B200 with 6 us
-        // of an empty launch between events): a tile's group 52 + nt / 3 up to 64 rows, 50 + nt / 2 above (two sets of
-        // splitting warps and two buffers then), a round of tiles 200 beside that; in gemm_f32_few.cu a round of tiles 24 per group.
-        const int rows16 = n_rows >= 128 ? 128 : (n_rows + 15) / 16 * 16;
-        long long best = -1;
-        for (int t = 16; t <= rows16; t += 16) {
-            const long long tiles = m_tiles * (((long long)n_rows + t - 1) / t);
-            const long long cost = 900 + (tiles + sms - 1) / sms * (n_groups * (t <= 64 ? 46 + t / 3 : 50 + t / 2) + 200);
-            if (best < 0 || cost < best) { best = cost; nt = t; }
-        }
-        const long long few = ((long long)n_out + 15) / 16 * ((n_rows + 15) / 16);
-        if (n_rows <= GF_FEW_MOST && 700 + (few + sms - 1) / sms * n_groups * 24 < best) return gf_few_launch(g, s);
-    }
     GemmF32Tc p;
     p.g = g;
     p.vec_w = k_dim % 4 == 0 && aligned16(w);

@@ -13,6 +13,7 @@ so is a missing or unbuildable library.
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional, Sequence
 
 import torch
@@ -44,6 +45,7 @@ def lib() -> ctypes.CDLL:
         _LIB.st_attention_decode_scratch_floats.restype = ctypes.c_longlong
         _LIB.st_latent_attention_mma_scratch.restype = ctypes.c_longlong
         _LIB.st_hgrn2_chunks_scratch.restype = ctypes.c_longlong
+        _LIB.st_gemm_f32_scratch.restype = ctypes.c_longlong
         _LIB.st_delta_rule_scratch_floats.restype = ctypes.c_longlong
         _LIB.st_delta_rule_chunk_floats.restype = ctypes.c_longlong
         _LIB.st_uniform_host.restype = ctypes.c_float
@@ -454,6 +456,11 @@ def qkv_linear_to_cache(h: torch.Tensor, w: torch.Tensor, bias: Optional[torch.T
                                     _stream()), "qkv_linear_to_cache")
 
 
+@functools.lru_cache(maxsize=4096)
+def _gemm_f32_scratch(n: int, m: int, k: int, device: int) -> int:
+    return int(lib().st_gemm_f32_scratch(n, m, k))
+
+
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none",
                out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """The plain product for either storage type (fixed summation order).  float32: on the tensor cores, each operand as
@@ -467,11 +474,11 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = 
     out = a.new_empty((n, m), dtype=out_dtype)
     if a.dtype == torch.float32:
         assert out_dtype == torch.float32 and w.dtype == torch.float32
-        scratch = status = None
-        if n > 8:                            # beyond that the kernel may take a's parts, [3][n][k rounded up to 64], from memory
-            scratch = a.new_empty(6 * n * ((k + 63) // 64 * 64), dtype=torch.uint8)
-            status = _tc_status_word(a.device)
-        _check(lib().st_gemm_f32(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], 0, _p(scratch), _p(status),
+        pa, scratch, status = _p(a), None, None
+        need = _gemm_f32_scratch(n, m, k, a.device.index)
+        if need:                             # a's parts, [3][n][k rounded up to 64], go by way of memory
+            scratch, status = a.new_empty(need, dtype=torch.uint8), _tc_status_word(a.device)
+        _check(lib().st_gemm_f32(pa, _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], 0, _p(scratch), _p(status),
                                  _stream()), "gemm_plain")
         return out
     _check(lib().st_gemm_plain(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act],

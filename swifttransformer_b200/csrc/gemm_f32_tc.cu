@@ -405,18 +405,24 @@ static int gf_plan(const GemmF32& g) {
     return nt;
 }
 
-// Bytes of scratch st_gemm_f32 takes on the current device.
-ST_EXPORT long long st_gemm_f32_scratch(int n_rows, int n_out, int k_dim) {
+static long long gf_row_bytes(int k_dim) { return 6 * (((long long)k_dim + GF_BK - 1) / GF_BK * GF_BK); }
+
+// Bytes of scratch with which st_gemm_f32 takes all rows at once on the current device, or, where that is more than `most`, as many rows as
+// that holds in whole tiles of 128 at a time, at least one tile.
+ST_EXPORT long long st_gemm_f32_scratch(int n_rows, int n_out, int k_dim, long long most) {
     const GemmF32 g = {nullptr, nullptr, nullptr, nullptr, n_rows, n_out, k_dim, 0};
     if (n_rows <= 0 || n_out <= 0 || k_dim < GF_SHORT || gf_plan(g) == 0) return 0;
-    return 6LL * n_rows * (((long long)k_dim + GF_BK - 1) / GF_BK * GF_BK);
+    const long long per_row = gf_row_bytes(k_dim), tiles = most / (per_row * 128), rows = 128 * (tiles > 1 ? tiles : 1);
+    return per_row * (rows < n_rows ? rows : n_rows);
 }
 
+static int gf_run(const GemmF32& g, int nt, void* scratch, int* status, cudaStream_t s);
+
 // a [n_rows, k_dim], w [n_out, k_dim], out [n_rows, n_out], float and contiguous, of any alignment.  scratch: 16-byte aligned, with status;
-// both may be null where st_gemm_f32_scratch is 0.  form, for tests: rows of a per tile of this kernel (a multiple of 16 up to 128; scratch
-// 6 n_rows (k_dim rounded up to 64) bytes then), -8 and -16: gemm_f32_few.cu in such tiles, 0: chosen here.
+// both may be null where st_gemm_f32_scratch is 0; with fewer bytes than all rows take the rows go in parts.  form, for tests: rows of a per
+// tile of this kernel (a multiple of 16 up to 128), -8 and -16: gemm_f32_few.cu in such tiles, 0: chosen here.
 ST_EXPORT int st_gemm_f32(const float* a, const float* w, const float* bias, float* out, int n_rows, int n_out, int k_dim, int act,
-                          int form, void* scratch, int* status, void* stream) {
+                          int form, void* scratch, long long scratch_bytes, int* status, void* stream) {
     if (n_rows <= 0 || n_out <= 0) return 0;
     if (k_dim <= 0) return ST_ERR_BAD_SIZE;
     const GemmF32 g = {a, w, bias, out, n_rows, n_out, k_dim, act};
@@ -426,7 +432,24 @@ ST_EXPORT int st_gemm_f32(const float* a, const float* w, const float* bias, flo
     const int nt = form == 0 ? gf_plan(g) : form;
     if (nt == 0) return gf_few_launch(g, 0, s);
     if (!status || !scratch || !aligned16(scratch) || nt < 0 || nt > 128 || nt % 16) return ST_ERR_BAD_ARG;
-    const int sms = st_sm_count();
+    long long rows = scratch_bytes / gf_row_bytes(k_dim);
+    if (rows >= n_rows) return gf_run(g, nt, scratch, status, s);
+    if (rows >= nt) rows = rows / nt * nt;
+    if (rows < 1) return ST_ERR_BAD_ARG;
+    for (long long r0 = 0; r0 < n_rows; r0 += rows) {                // (a part's splitting kernel starts when the part before is done)
+        GemmF32 part = g;
+        part.a += r0 * k_dim;
+        part.out += r0 * n_out;
+        part.n_rows = (int)(n_rows - r0 < rows ? n_rows - r0 : rows);
+        const int rc = gf_run(part, nt, scratch, status, s);
+        if (rc) return rc;
+    }
+    return 0;
+}
+
+static int gf_run(const GemmF32& g, int nt, void* scratch, int* status, cudaStream_t s) {
+    const int sms = st_sm_count(), n_rows = g.n_rows, n_out = g.n_out, k_dim = g.k_dim;
+    const float *a = g.a, *w = g.w;
     const long long m_tiles = ((long long)n_out + GF_BM - 1) / GF_BM, n_groups = ((long long)k_dim + GF_BK - 1) / GF_BK;
     const long long k_pad = n_groups * GF_BK;
     GemmF32Tc p;

@@ -456,9 +456,13 @@ def qkv_linear_to_cache(h: torch.Tensor, w: torch.Tensor, bias: Optional[torch.T
                                     _stream()), "qkv_linear_to_cache")
 
 
+# Bytes a float32 product's row parts may take at a time (5461 rows of k = 8192); more rows go in parts.
+GEMM_F32_SCRATCH = 256 << 20
+
+
 @functools.lru_cache(maxsize=4096)
-def _gemm_f32_scratch(n: int, m: int, k: int, device: int) -> int:
-    return int(lib().st_gemm_f32_scratch(n, m, k))
+def _gemm_f32_scratch(n: int, m: int, k: int, most: int, device: int) -> int:
+    return int(lib().st_gemm_f32_scratch(n, m, k, ctypes.c_longlong(most)))
 
 
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none",
@@ -475,11 +479,11 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = 
     if a.dtype == torch.float32:
         assert out_dtype == torch.float32 and w.dtype == torch.float32
         pa, scratch, status = _p(a), None, None
-        need = _gemm_f32_scratch(n, m, k, a.device.index)
+        need = _gemm_f32_scratch(n, m, k, GEMM_F32_SCRATCH, a.device.index)
         if need:                             # a's parts, [3][n][k rounded up to 64], go by way of memory
             scratch, status = a.new_empty(need, dtype=torch.uint8), _tc_status_word(a.device)
-        _check(lib().st_gemm_f32(pa, _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], 0, _p(scratch), _p(status),
-                                 _stream()), "gemm_plain")
+        _check(lib().st_gemm_f32(pa, _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], 0, _p(scratch), ctypes.c_longlong(need),
+                                 _p(status), _stream()), "gemm_plain")
         return out
     _check(lib().st_gemm_plain(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act],
                                int(out_dtype == torch.float32), _stream()), "gemm_plain")

@@ -25,7 +25,30 @@ def test_forms(rows, k, outs, skip):
     p = lambda t: ctypes.c_void_p(t.data_ptr())
     for form in [-8, -16] + list(range(16, 129, 16)):
         out = torch.full((rows + 1, outs), 77.0, device="cuda")
-        assert ops.lib().st_gemm_f32(p(a), p(w), p(bias), p(out), rows, outs, k, ops.ACT_CODES["relu"], form, p(scratch), p(status),
-                                     ops._stream()) == 0
+        assert ops.lib().st_gemm_f32(p(a), p(w), p(bias), p(out), rows, outs, k, ops.ACT_CODES["relu"], form, p(scratch),
+                                     ctypes.c_longlong(scratch.numel()), p(status), ops._stream()) == 0
         assert torch.equal(out[:rows], chosen) and torch.all(out[rows] == 77.0), form
+    assert int(status) == 0
+
+
+@pytest.mark.parametrize("rows,k,outs", [(700, 520, 2000), (257, 1032, 640), (129, 64, 20000), (20, 2048, 8192)])
+def test_rows_in_parts(rows, k, outs, monkeypatch):
+    """Scratch for some of the rows at a time: the same bits, and no more scratch than is allowed (a tile of 128 rows at least)."""
+    from swifttransformer_b200 import ops
+    gen = torch.Generator(device="cuda").manual_seed(rows)
+    a, w, bias = (torch.randn(s, generator=gen, device="cuda") for s in ((rows, k), (outs, k), (outs,)))
+    whole = ops.linear(a, w, bias, "gelu")
+    per_row = 6 * ((k + 63) // 64 * 64)
+    for most in (0, 300 * per_row, 10 ** 9):
+        monkeypatch.setattr(ops, "GEMM_F32_SCRATCH", most)
+        need = ops._gemm_f32_scratch(rows, outs, k, most, a.device.index)
+        assert need == per_row * min(rows, max(most // (128 * per_row), 1) * 128)
+        assert torch.equal(ops.linear(a, w, bias, "gelu"), whole)
+    scratch, status = torch.empty(5 * per_row, dtype=torch.uint8, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, p = torch.empty_like(whole), lambda t: ctypes.c_void_p(t.data_ptr())
+    for size, taken in ((5 * per_row, True), (per_row - 1, False)):  # (five rows at a time; not one)
+        out.zero_()
+        got = ops.lib().st_gemm_f32(p(a), p(w), p(bias), p(out), rows, outs, k, ops.ACT_CODES["gelu"], 16, p(scratch), ctypes.c_longlong(size),
+                                    p(status), ops._stream())
+        assert (got == 0) == taken and torch.equal(out, whole if taken else torch.zeros_like(whole))
     assert int(status) == 0

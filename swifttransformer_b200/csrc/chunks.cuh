@@ -31,22 +31,20 @@ __device__ __forceinline__ bool hk_find(const int* q_start, const int* positions
     return chunk >= 0 && n > 0 && end - begin >= from && positions[begin] >= 0;      // (padding stands at position -1)
 }
 
-// 1 / d and z / d for d >= 1 to the last bit or next to it: the hardware's reciprocal (of at most 1e38: beyond, the quotient is next to
-// nothing either way) and a step of residual correction.  The compiler's own division tests every operand for its slow
-// form, and so a thread's divisions run one after the other, some 360 clocks each: 32 of them were most of a chunk's time.
+// 1 / d and z / d for d >= 1 (infinity among them), to the last bit or next to it: the hardware's reciprocal and one step of Newton's iteration
+// for it, r + r (1 - d r); the quotient q = z r with its residual, q + r (z - q d) (P. W. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990)).  A thread's quotients so run side by side; as divisions they ran one
+// after the other, some 360 clocks each: 32 of them were most of a chunk's time.
 __device__ __forceinline__ float hk_inverse(float d) {
     float r;
-    d = fminf(d, 1e38f);                                  // (a number that is none comes out as 1e-38 and makes the result none below)
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-    return fmaf(r, fmaf(-d, r, 1.f), r);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d * 0.0625f));
+    r *= 0.0625f;                                         // (from 2^126 on not normal, zero for an infinite d)
+    return fmaf(r, fmaf(-fminf(d, 3.4028234e38f), r, 1.f), r);
 }
-__device__ __forceinline__ float hk_sigmoid(float z) {
-    const float e = expf(-z), r = hk_inverse(1.f + e);
-    return z != z ? z : r;
-}
+__device__ __forceinline__ float hk_sigmoid(float z) { return hk_inverse(1.f + expf(-z)); }
 __device__ __forceinline__ float hk_silu(float z) {
-    const float d = fminf(1.f + expf(-z), 1e38f), r = hk_inverse(d), q = z * r, rest = fmaf(-q, d, z);
-    return rest < 0.f || rest > 0.f ? fmaf(rest, r, q) : q;          // (an infinite z has no residual)
+    const float d = 1.f + expf(-z), r = hk_inverse(d), q = z * r, rest = fmaf(-q, d, z);
+    return rest < 0.f || rest > 0.f ? fmaf(rest, r, q) : q;          // (an infinite z or d has no residual)
 }
 // 1 / sqrt(x): the hardware's and a Newton step
 __device__ __forceinline__ float hk_rsqrt(float x) {

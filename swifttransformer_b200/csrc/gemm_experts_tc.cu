@@ -55,9 +55,9 @@ __device__ __forceinline__ void ge_ld8(uint32_t taddr, float* v) {
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                  : "r"(taddr) : "memory");
 }
-// v / (1 + exp(-v)) of eight numbers side by side: the quotient by the fast division and one step of residual correction, which
-// gives the divided number's bits wherever the residual is a number; the compiler's own division tests every operand
-// for its slow form and so ran the eight one after the other, 360 clocks each
+// v / (1 + exp(-v)) of eight numbers side by side: the quotient by the fast division and one step of residual correction
+// (chunks.cuh names the method), which gives the divided number's bits wherever the residual is a number.  As divisions they ran one after
+// the other: 360 clocks each
 __device__ __forceinline__ void ge_silu8(float* v) {
 #pragma unroll
     for (int j = 0; j < 8; ++j) {

@@ -4,19 +4,18 @@
 // A float, times 2^16, is the sum of three bfloat16 numbers of eight bits each, h + m + l (float_parts.cuh); an output is the sum of their
 // products times 2^-32.  Of the nine products of two such sums six are formed,
 //   w_l a_h + w_h a_l + w_m a_m + w_m a_h + w_h a_m + w_h a_h,
-// each exact in the tensor cores' float accumulator; the three left out are at most 2^-25 of w a together.  The tensor
-// cores cut a sum off where a float addition rounds it (measured: 6e-8 of bias after four steps of 16 k, 1.2e-7 after eight), so a sum
-// stays there for one group of 64 k only, the small products first: its 24 steps end with the four of w_h a_h.  The
-// groups' sums are added up in float registers in ascending order, each addition rounded to nearest.  An output so
-// depends on its own row of a and of w alone, and its bits are the same for every number of rows, tile and kernel: all form the
-// same groups and add them in the same order (mma.sync and tcgen05.mma give the same bits for the same sixteen products; a test
-// holds the kernels to it).
+// each exact in the tensor cores' float accumulator; the three left out are at most 2^-24 of w a together (on average 2^-28).  The
+// tensor cores cut a sum off where a float addition rounds it (measured: 6e-8 of bias after four steps of 16 k, 1.2e-7 after eight), so a
+// sum stays there for one group of 64 k only, the small products first: its 24 steps end with the four of w_h a_h.  The groups' sums are
+// added up in float registers in ascending order, each addition rounded to nearest.  An output so depends on its own row of a and of w
+// alone, and its bits are the same for every number of rows, tile and kernel: all form the same groups and add them in the same order
+// (mma.sync and tcgen05.mma give the same bits for the same sixteen products; a test holds the kernels to it).
 //
 // A sum that comes out infinite or not a number (operands that are, operands from 2^112 on, outputs from 2^96 on) is formed again as
 // a chain of fused multiply-adds over k, which is what such operands give in plain float.
 //
-// Error against 64 bits, relative 2-norm, normal operands: k = 512 9.6e-8, 2048 1.3e-7, 8192 2.2e-7 (a chain of fused multiply-adds
-// over k: 4.0e-7, 8.1e-7, 1.6e-6).
+// Error against 64 bits, relative 2-norm, normal operands of any size from 2^-135 on: k = 16 4.7e-8, 64 7.7e-8, 512 9.6e-8, 2048 1.3e-7,
+// 8192 2.2e-7 (a chain of fused multiply-adds over k: 7.4e-8, 1.4e-7, 4.0e-7, 8.1e-7, 1.6e-6).
 #pragma once
 #include "common.cuh"
 #include "float_parts.cuh"

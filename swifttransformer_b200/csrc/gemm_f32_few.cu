@@ -7,8 +7,8 @@
 // bit.  The groups' sums meet in shared memory (two rounds of them, so that one is added up while the next is written), where the
 // last four warps, which have the fewest groups, add them up in ascending order.
 //
-// Bound by instructions (1 x 2048 x 50272: 65 % of the issue slots, DRAM 48 %), most of them cutting w and a into parts; so the copies'
-// addresses go on by constant steps, and rows of a that are not there are not copied.  us on one B200, recorded calls over weights that are not in cache, in brackets addresses worked out copy by copy and every row
+// Bound by instructions (1 x 2048 x 50272 before what follows: 65 % of the issue slots in use, DRAM 48 %), most of them cutting w and a
+// into parts; so the copies' addresses go on by constant steps, and rows of a that are not there are not copied.  us on one B200, recorded calls over weights that are not in cache, in brackets addresses worked out copy by copy and every row
 // copied, then float multiply-adds: 1 x 2048 x 8192 19.3 (21.2; 17.7), 1 x 4096 x 4096 18.8 (20.5; 19.7), 8 x 4096 x 4096 20.1 (20.5; 24.9),
 // 16 x 768 x 3072 8.4 (11.0; 9.0), 16 x 2048 x 2048 10.5 (11.2; 13.7), 1 x 64 x 64 3.2 (3.3; 2.3).
 #include "gemm_f32.cuh"

@@ -16,7 +16,7 @@
 //
 // The products run on the tensor cores, every float as the sum of three bfloat16 numbers (float_parts.cuh, gemm_f32.cuh).
 //
-// Measured on one B200, 2000 tokens of one request, 16 heads of 128 x 128: bfloat16 rows 116 us (kv 28, scan 12, out 70 alone) where
+// Measured on one B200, 2000 tokens of one request, 16 heads of 128 x 128: bfloat16 rows 112 us (kv 28, scan 12, out 70 alone) where
 // products on the float unit, divisions one after the other and 35 and 93 KB of code took 158 (kv 42, out 106) and the walk
 // (hgrn2_wide) 1030; float rows 142 (160).  333 tokens of 8 heads, 128 x 64: 44 (59); 150 of 16 heads 48 (63).  kv and out are bound
 // by their instructions, three or four warps a scheduler (two blocks of 256 threads per SM), the scan by its two trips to the

@@ -223,7 +223,7 @@ _addmm_activation = getattr(torch, "_addmm_activation", None)    # the library p
 
 def linear(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none",
            out_dtype: Optional[torch.dtype] = None, bias_bf16: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """act(a @ w.T + bias); w is [out, in].  float32: ``gemm_plain`` (true 32-bit).
+    """act(a @ w.T + bias); w is [out, in].  float32: ``gemm_plain`` (operands taken to their last bit, float sums).
     bfloat16, few rows: the weight-streaming kernel.  bfloat16, more rows: the library product with float
     accumulation; bias and ReLU ride in its epilogue when ``bias_bf16`` (a lossless bfloat16 copy of
     ``bias``, see lossless_bf16) is given, else the bias/activation kernel follows."""
@@ -468,8 +468,8 @@ def _gemm_f32_scratch(n: int, m: int, k: int, most: int, device: int) -> int:
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none",
                out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """The plain product for either storage type (fixed summation order).  float32: on the tensor cores, each operand as
-    the sum of three bfloat16 numbers, at least as close to 64 bits as a chain of float multiply-adds.  bfloat16: a
-    chain of float multiply-adds."""
+    the sum of three bfloat16 numbers, at least as close to 64 bits as a chain of float multiply-adds; such a chain up to 8 k, and
+    where a sum is not finite.  bfloat16: a chain of float multiply-adds."""
     out_dtype = out_dtype or a.dtype
     a = a.contiguous()
     assert w.is_contiguous()
@@ -1168,8 +1168,10 @@ def latent_attention(q_lat: torch.Tensor, pool: torch.Tensor, layer: int, out: t
         kernel = "mma" if latent_attention_mma_applies(q_lat, kr, rot) else "plain"
         if n_splits is None and q_start is not None and latent_attention_tc_applies(q_lat, pool, layer, kr, rot, page_size):
             # Prompt portions: where the mma.sync kernel would not cut the key ranges and the tcgen05 kernel's blocks (128 rows by
-            # 256 value columns) fill half of the SMs.  16 heads, 512 + 64, us (mma.sync): 2 x 1000 tokens 183 (268), 300 tokens
-            # (76 blocks) 41 (54), 450 tokens behind 1200 (114) 128 (192); 450 behind 1200 with 8 heads (58) 131 (119).
+            # 256 value columns) fill half of the SMs.  16 heads, 512 + 64, us with the launch between events (mma.sync): 2 x 1000 tokens
+            # 93 (222), 300 tokens (76 blocks) 26 (48), 450 tokens behind 1200 (114) 58 (187).  The line was drawn with a tcgen05 kernel
+            # half as fast, which lost 450 tokens behind 1200 with 8 heads (58 blocks); it wins that now, 56 (110), and what else was
+            # measured below the line: 150 tokens (38 blocks) 23 (30), 100 behind 1000 (26) 44 (46).
             n = q_lat.shape[0]
             if (out.data_ptr() % 16 == 0 and 2 * int(lib().st_latent_attention_tc_blocks(n, nh, kr)) >= sm_count(q_lat.device)
                     and int(lib().st_latent_attention_mma_splits(n, n_seqs, nh, window)) == 1):

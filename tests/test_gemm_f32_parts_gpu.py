@@ -17,7 +17,7 @@ def test_a_row_has_the_same_bits_in_every_batch(k, outs):
     whole = ops.linear(a, w)
     exact = a.double() @ w.double().T
     # Each of the six products of a group of 64 k is cut off at 2^-23 of the running sum at most 4 times, of which only the last
-    # four steps' sums are as large as the group's; then one rounding per group and the parts left out (2^-25): far
+    # four steps' sums are as large as the group's; then one rounding per group and the parts left out (2^-24): far
     # within k / 64 + 8 times 2^-23 of |a| |w|
     bound = (k / 64 + 8) * 2.0 ** -23 * (a.abs().double() @ w.abs().double().T)
     assert torch.all((whole.double() - exact).abs() <= bound)

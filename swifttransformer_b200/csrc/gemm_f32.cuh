@@ -35,6 +35,6 @@ __device__ __forceinline__ float gf_finish(const GemmF32& p, float v, float bias
 #define GF_SHORT 9
 int gf_short_launch(const GemmF32& p, cudaStream_t s);
 
-// the same file: in tiles of 8 or 16 rows (0: what takes less), and about what it takes, in units of 10 ns
+// the same file: in tiles of 8 or 16 rows, and about what it takes, in units of 10 ns, with the form (-8, -16) that takes less
 int gf_few_launch(const GemmF32& p, int rows, cudaStream_t s);
-long long gf_few_cost(const GemmF32& p);
+long long gf_few_cost(const GemmF32& p, int& form);

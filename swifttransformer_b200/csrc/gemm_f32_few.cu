@@ -213,12 +213,12 @@ static long long gq_cost(const GemmF32& p, int rows) {
     const long long cost = tiles * (15 * per_tile + 30) / sms, least = 18 * n_groups;
     return 250 + slow * (cost < least ? least : cost);
 }
-long long gf_few_cost(const GemmF32& p) {
+long long gf_few_cost(const GemmF32& p, int& form) {
     const long long c8 = gq_cost(p, 8), c16 = gq_cost(p, 16);
-    return p.n_rows <= 8 || c8 < c16 ? c8 : c16;
+    form = p.n_rows <= 8 || c8 < c16 ? -8 : -16;
+    return form == -8 ? c8 : c16;
 }
 int gf_few_launch(const GemmF32& p, int rows, cudaStream_t s) {
-    if (rows == 0) rows = p.n_rows <= 8 || gq_cost(p, 8) < gq_cost(p, 16) ? 8 : 16;
     return rows == 8 ? gq_launch<1>(p, s) : gq_launch<2>(p, s);
 }
 

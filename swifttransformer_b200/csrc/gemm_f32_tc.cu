@@ -387,32 +387,38 @@ static int gf_launch(const CUtensorMap& w_map, const CUtensorMap& a_map, const G
     return st_launch_pdl("gemm_f32", kernel, dim3((unsigned)grid), dim3(GF_THREADS(NT)), GF_SMEM, s, w_map, a_map, p, status);
 }
 
-// Rows of a per tile, 0: gemm_f32_few.cu, by what they were measured to take (units of 10 ns, on one B200, recorded calls): a tile's group
+// The form (see st_gemm_f32) by what they were measured to take (units of 10 ns, on one B200, recorded calls): a tile's group
 // 46 + nt / 3 up to 64 rows, 50 + nt / 2 above (two sets of splitting warps and two buffers then), a round of tiles 200 beside that and
 // the splitting kernel and the launch 450; twelve times as much for the groups but two where rows of w are not whole pieces of 16 bytes
 // (40 x 770 x 2304 87 us, 40 x 130 x 512 10).  us, this kernel / gemm_f32_few.cu: 16 x 768 x 3072 12.1 / 8.4, 16 x 2048 x 6144 23.5 / 27.6,
 // 24 x 4096 x 4096 40.2 / 52.8, 24 x 8192 x 2048 73 / 55, 1 x 768 x 50272 35 / 41, 64 x 64 x 64 5.7 / 3.5.
+#define GF_FORM_SHORT 1
 static int gf_plan(const GemmF32& g) {
+    if (g.k_dim < GF_SHORT) return GF_FORM_SHORT;
     const long long sms = st_sm_count(), m_tiles = ((long long)g.n_out + GF_BM - 1) / GF_BM, n_groups = ((long long)g.k_dim + GF_BK - 1) / GF_BK;
     const int rows16 = g.n_rows >= 128 ? 128 : (g.n_rows + 15) / 16 * 16;
-    long long best = gf_few_cost(g);
-    int nt = 0;
+    int form;
+    long long best = gf_few_cost(g, form);
     for (int t = 16; t <= rows16; t += 16) {
         const long long tiles = m_tiles * (((long long)g.n_rows + t - 1) / t);
         const long long groups = g.k_dim % 4 == 0 || n_groups <= 2 ? n_groups : 12 * (n_groups - 2);
         const long long cost = 450 + (tiles + sms - 1) / sms * (groups * (t <= 64 ? 46 + t / 3 : 50 + t / 2) + 200);
-        if (cost < best) { best = cost; nt = t; }
+        if (cost < best) { best = cost; form = t; }
     }
-    return nt;
+    return form;
 }
 
 static long long gf_row_bytes(int k_dim) { return 6 * (((long long)k_dim + GF_BK - 1) / GF_BK * GF_BK); }
 
 // Bytes of scratch with which st_gemm_f32 takes all rows at once on the current device, or, where that is more than `most`, as many rows as
-// that holds in whole tiles of 128 at a time, at least one tile.
-ST_EXPORT long long st_gemm_f32_scratch(int n_rows, int n_out, int k_dim, long long most) {
+// that holds in whole tiles of 128 at a time, at least one tile.  form: the one st_gemm_f32 chooses, so that a caller who keeps it by
+// size saves each call the choice.
+ST_EXPORT long long st_gemm_f32_scratch(int n_rows, int n_out, int k_dim, long long most, int* form) {
     const GemmF32 g = {nullptr, nullptr, nullptr, nullptr, n_rows, n_out, k_dim, 0};
-    if (n_rows <= 0 || n_out <= 0 || k_dim < GF_SHORT || gf_plan(g) == 0) return 0;
+    *form = 0;
+    if (n_rows <= 0 || n_out <= 0 || k_dim <= 0) return 0;
+    *form = gf_plan(g);
+    if (*form < 16) return 0;
     const long long per_row = gf_row_bytes(k_dim), tiles = most / (per_row * 128), rows = 128 * (tiles > 1 ? tiles : 1);
     return per_row * (rows < n_rows ? rows : n_rows);
 }
@@ -420,19 +426,18 @@ ST_EXPORT long long st_gemm_f32_scratch(int n_rows, int n_out, int k_dim, long l
 static int gf_run(const GemmF32& g, int nt, void* scratch, int* status, cudaStream_t s);
 
 // a [n_rows, k_dim], w [n_out, k_dim], out [n_rows, n_out], float and contiguous, of any alignment.  scratch: 16-byte aligned, with status;
-// both may be null where st_gemm_f32_scratch is 0; with fewer bytes than all rows take the rows go in parts.  form, for tests: rows of a per
-// tile of this kernel (a multiple of 16 up to 128), -8 and -16: gemm_f32_few.cu in such tiles, 0: chosen here.
+// both may be null where st_gemm_f32_scratch is 0; with fewer bytes than all rows take the rows go in parts.  form: rows of a per tile of
+// this kernel (a multiple of 16 up to 128), -8 and -16: gemm_f32_few.cu in such tiles, 1: chains (k below GF_SHORT), 0: chosen here.
 ST_EXPORT int st_gemm_f32(const float* a, const float* w, const float* bias, float* out, int n_rows, int n_out, int k_dim, int act,
                           int form, void* scratch, long long scratch_bytes, int* status, void* stream) {
     if (n_rows <= 0 || n_out <= 0) return 0;
     if (k_dim <= 0) return ST_ERR_BAD_SIZE;
     const GemmF32 g = {a, w, bias, out, n_rows, n_out, k_dim, act};
     cudaStream_t s = (cudaStream_t)stream;
-    if (form == 0 && k_dim < GF_SHORT) return gf_short_launch(g, s);
-    if (form == -8 || form == -16) return gf_few_launch(g, -form, s);
     const int nt = form == 0 ? gf_plan(g) : form;
-    if (nt == 0) return gf_few_launch(g, 0, s);
-    if (!status || !scratch || !aligned16(scratch) || nt < 0 || nt > 128 || nt % 16) return ST_ERR_BAD_ARG;
+    if (nt == GF_FORM_SHORT) return k_dim < GF_SHORT ? gf_short_launch(g, s) : ST_ERR_BAD_ARG;
+    if (nt == -8 || nt == -16) return gf_few_launch(g, -nt, s);
+    if (!status || !scratch || !aligned16(scratch) || nt < 16 || nt > 128 || nt % 16) return ST_ERR_BAD_ARG;
     long long rows = scratch_bytes / gf_row_bytes(k_dim);
     if (rows >= n_rows) return gf_run(g, nt, scratch, status, s);
     if (rows >= nt) rows = rows / nt * nt;

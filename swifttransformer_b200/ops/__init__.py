@@ -458,11 +458,15 @@ def qkv_linear_to_cache(h: torch.Tensor, w: torch.Tensor, bias: Optional[torch.T
 
 # Bytes a float32 product's row parts may take at a time (5461 rows of k = 8192); more rows go in parts.
 GEMM_F32_SCRATCH = 256 << 20
+_NO_SCRATCH = ctypes.c_longlong(0)
 
 
 @functools.lru_cache(maxsize=4096)
-def _gemm_f32_scratch(n: int, m: int, k: int, most: int, device: int) -> int:
-    return int(lib().st_gemm_f32_scratch(n, m, k, ctypes.c_longlong(most)))
+def _gemm_f32_plan(n: int, m: int, k: int, most: int, device: int):
+    """(form, bytes of scratch) of a float32 product of these sizes on a device."""
+    form = ctypes.c_int(0)
+    need = int(lib().st_gemm_f32_scratch(n, m, k, ctypes.c_longlong(most), ctypes.byref(form)))
+    return form.value, need
 
 
 def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None, act: str = "none",
@@ -478,12 +482,15 @@ def gemm_plain(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = 
     out = a.new_empty((n, m), dtype=out_dtype)
     if a.dtype == torch.float32:
         assert out_dtype == torch.float32 and w.dtype == torch.float32
-        pa, scratch, status = _p(a), None, None
-        need = _gemm_f32_scratch(n, m, k, GEMM_F32_SCRATCH, a.device.index)
-        if need:                             # a's parts, [3][n][k rounded up to 64], go by way of memory
-            scratch, status = a.new_empty(need, dtype=torch.uint8), _tc_status_word(a.device)
-        _check(lib().st_gemm_f32(pa, _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], 0, _p(scratch), ctypes.c_longlong(need),
-                                 _p(status), _stream()), "gemm_plain")
+        pa, at, status, size = _p(a), None, None, _NO_SCRATCH
+        if n <= 8 and m <= 8192 and k > 8:
+            form = -8                        # what the plan gives (but for k of a few and of 20 thousand), without asking: half a microsecond
+        else:
+            form, need = _gemm_f32_plan(n, m, k, GEMM_F32_SCRATCH, a.get_device())
+            if need:                         # a's parts, [3][n][k rounded up to 64], go by way of memory
+                scratch = a.new_empty(need, dtype=torch.uint8)
+                at, status, size = _p(scratch), _p(_tc_status_word(a.device)), ctypes.c_longlong(need)
+        _check(lib().st_gemm_f32(pa, _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act], form, at, size, status, _stream()), "gemm_plain")
         return out
     _check(lib().st_gemm_plain(_p(a), _p(w), _p(bias), _p(out), n, m, k, ACT_CODES[act],
                                int(out_dtype == torch.float32), _stream()), "gemm_plain")

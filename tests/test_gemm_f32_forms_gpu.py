@@ -23,7 +23,7 @@ def test_forms(rows, k, outs, skip):
     scratch = torch.empty(6 * rows * ((k + 63) // 64 * 64), dtype=torch.uint8, device="cuda")
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     p = lambda t: ctypes.c_void_p(t.data_ptr())
-    for form in [-8, -16] + list(range(16, 129, 16)):
+    for form in [0, -8, -16] + list(range(16, 129, 16)):
         out = torch.full((rows + 1, outs), 77.0, device="cuda")
         assert ops.lib().st_gemm_f32(p(a), p(w), p(bias), p(out), rows, outs, k, ops.ACT_CODES["relu"], form, p(scratch),
                                      ctypes.c_longlong(scratch.numel()), p(status), ops._stream()) == 0
@@ -41,8 +41,8 @@ def test_rows_in_parts(rows, k, outs, monkeypatch):
     per_row = 6 * ((k + 63) // 64 * 64)
     for most in (0, 300 * per_row, 10 ** 9):
         monkeypatch.setattr(ops, "GEMM_F32_SCRATCH", most)
-        need = ops._gemm_f32_scratch(rows, outs, k, most, a.device.index)
-        assert need == per_row * min(rows, max(most // (128 * per_row), 1) * 128)
+        form, need = ops._gemm_f32_plan(rows, outs, k, most, a.device.index)
+        assert form >= 16 and need == per_row * min(rows, max(most // (128 * per_row), 1) * 128)
         assert torch.equal(ops.linear(a, w, bias, "gelu"), whole)
     scratch, status = torch.empty(5 * per_row, dtype=torch.uint8, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
     out, p = torch.empty_like(whole), lambda t: ctypes.c_void_p(t.data_ptr())
